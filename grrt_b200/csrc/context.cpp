@@ -193,6 +193,8 @@ bool GRRTContext::ensure_device() {
     DevScene& S = dev;
     S.M = mass;
     S.a = spin_a;
+    S.a2 = spin_a * spin_a;
+    S.m2 = 2.0 * mass;
     S.r_stop = r_horizon + 0.01;
     S.r_escape = 1000.0;
     S.tol = tolerance;

@@ -30,6 +30,11 @@ constexpr double e1 = 71.0 / 57600.0, e3 = -71.0 / 16695.0, e4 = 71.0 / 1920.0,
 
 template <typename T>
 GRRT_HD Vec5<T> axpy(const Vec5<T>& y, T h, const Vec5<T>& k) {
+#ifdef GRRT_RHS_PINNED
+    if constexpr (sizeof(T) == sizeof(double))
+        return Vec5<T>{__fma_rn(h, k.r, y.r), __fma_rn(h, k.th, y.th), __fma_rn(h, k.ph, y.ph),
+                       __fma_rn(h, k.pr, y.pr), __fma_rn(h, k.pth, y.pth)};
+#endif
     return Vec5<T>{y.r + h * k.r, y.th + h * k.th, y.ph + h * k.ph, y.pr + h * k.pr, y.pth + h * k.pth};
 }
 
@@ -41,10 +46,126 @@ GRRT_HD Vec5<T> rk4_step(T M, T a, T pt, T pph, const Vec5<T>& y, T h) {
     const Vec5<T> k3 = kerr_rhs<T>(M, a, pt, pph, axpy(y, h * T(0.5), k2));
     const Vec5<T> k4 = kerr_rhs<T>(M, a, pt, pph, axpy(y, h, k3));
     const T w = h / T(6);
+#ifdef GRRT_RHS_PINNED
+    if constexpr (sizeof(T) == sizeof(double)) {
+        // the roundings the compiler picks where k1 comes from a call
+#define GRRT_RK4F(f) \
+    __fma_rn(__dadd_rn(__fma_rn(2.0, k3.f, __fma_rn(2.0, k2.f, k1.f)), k4.f), w, y.f)
+        return Vec5<T>{GRRT_RK4F(r), GRRT_RK4F(th), GRRT_RK4F(ph), GRRT_RK4F(pr), GRRT_RK4F(pth)};
+#undef GRRT_RK4F
+    }
+#endif
 #define GRRT_RK4C(f) y.f + (k1.f + T(2) * k2.f + T(2) * k3.f + k4.f) * w
     return Vec5<T>{GRRT_RK4C(r), GRRT_RK4C(th), GRRT_RK4C(ph), GRRT_RK4C(pr), GRRT_RK4C(pth)};
 #undef GRRT_RK4C
 }
+
+#if defined(__CUDACC__) && !defined(GRRT_RHS_GENERIC)
+struct DpConst {
+    double a21, a31, a32, a41, a42, a43, a51, a52, a53, a54, a61, a62, a63, a64, a65;
+    double b1, b3, b4, b5, b6, e1, e3, e4, e5, e6, e7, floor;
+};
+static __constant__ DpConst kDp = {dp::a21, dp::a31, dp::a32, dp::a41, dp::a42, dp::a43, dp::a51, dp::a52, dp::a53,
+                                   dp::a54, dp::a61, dp::a62, dp::a63, dp::a64, dp::a65, dp::b1, dp::b3, dp::b4,
+                                   dp::b5, dp::b6, dp::e1, dp::e3, dp::e4, dp::e5, dp::e6, dp::e7, 1e-10};
+
+// n / d, correctly rounded: the quotient from the reciprocal, corrected by its
+// exact residual (Markstein, as recip_f64) where both and the result are far
+// from the range's ends, the division operator elsewhere.
+__device__ __forceinline__ double div_f64(double n, double d) {
+    const int hn = __double2hiint(n) & 0x7fffffff, hd = __double2hiint(d) & 0x7fffffff;
+    // 2^-450 <= |n|, |d| < 2^450
+    if (static_cast<unsigned>(hn - 0x23d00000) >= 0x38400000u || static_cast<unsigned>(hd - 0x23d00000) >= 0x38400000u)
+        return n / d;
+    const double r = recip_f64(d), q = __dmul_rn(n, r);
+    return __fma_rn(__fma_rn(-d, q, n), r, q);
+}
+
+// One DP45 attempt on the device (dp45_attempt_k1 below), roundings written out
+// as the compiler fuses the generic form's sums: the first product of each.
+// What a stage no longer needs is folded into the sums of the later stages as
+// soon as it is known (the terms enter in the tableau's order), so fewer
+// registers live through the right-hand sides; phi does not feed the right-hand
+// side, so its stage states are not formed.
+struct ErrQuotient {
+    double num, den;  // error norm = num / den
+};
+
+template <typename F>
+__device__ __forceinline__ ErrQuotient dp45_attempt_f64(const F& f, const Vec5<double>& y, double h, const Vec5<double>& k1,
+                                                   Vec5<double>& y5, Vec5<double>& k7) {
+    const DpConst& C = kDp;
+    auto two = [](double c1, double x1, double c2, double x2) { return __fma_rn(c1, x1, __dmul_rn(c2, x2)); };
+#define GRRT_F4(s) f(s(r), s(th), s(pr), s(pth))
+#define GRRT_V4(s) {s(r), s(th), 0.0, s(pr), s(pth)}
+#define GRRT_V5(s) {s(r), s(th), s(ph), s(pr), s(pth)}
+#define GRRT_S2(f) __fma_rn(h, __dmul_rn(C.a21, k1.f), y.f)
+    const Vec5<double> k2 = GRRT_F4(GRRT_S2);
+#define GRRT_S3(f) __fma_rn(h, two(C.a31, k1.f, C.a32, k2.f), y.f)
+    const Vec5<double> k3 = GRRT_F4(GRRT_S3);
+#define GRRT_S4(f) __fma_rn(h, __fma_rn(C.a43, k3.f, two(C.a41, k1.f, C.a42, k2.f)), y.f)
+    const Vec5<double> k4 = GRRT_F4(GRRT_S4);
+#define GRRT_Q6(f) __fma_rn(C.a64, k4.f, __fma_rn(C.a63, k3.f, two(C.a61, k1.f, C.a62, k2.f)))
+    const Vec5<double> q6 GRRT_V4(GRRT_Q6);
+#define GRRT_QB(f) __fma_rn(C.b4, k4.f, two(C.b1, k1.f, C.b3, k3.f))
+    Vec5<double> qb GRRT_V5(GRRT_QB);
+#define GRRT_QE(f) __fma_rn(C.e4, k4.f, two(C.e1, k1.f, C.e3, k3.f))
+    Vec5<double> qe GRRT_V5(GRRT_QE);
+#define GRRT_S5(f) \
+    __fma_rn(h, __fma_rn(C.a54, k4.f, __fma_rn(C.a53, k3.f, two(C.a51, k1.f, C.a52, k2.f))), y.f)
+    const Vec5<double> k5 = GRRT_F4(GRRT_S5);
+#define GRRT_QB5(f) __fma_rn(C.b5, k5.f, qb.f)
+    qb = GRRT_V5(GRRT_QB5);
+#define GRRT_QE5(f) __fma_rn(C.e5, k5.f, qe.f)
+    qe = GRRT_V5(GRRT_QE5);
+#define GRRT_S6(f) __fma_rn(h, __fma_rn(C.a65, k5.f, q6.f), y.f)
+    const Vec5<double> k6 = GRRT_F4(GRRT_S6);
+#define GRRT_Y5(f) __fma_rn(h, __fma_rn(C.b6, k6.f, qb.f), y.f)
+    y5 = GRRT_V5(GRRT_Y5);
+#define GRRT_QE6(f) __fma_rn(C.e6, k6.f, qe.f)
+    qe = GRRT_V5(GRRT_QE6);
+    k7 = f(y5.r, y5.th, y5.pr, y5.pth);
+#undef GRRT_F4
+#undef GRRT_V4
+#undef GRRT_V5
+#undef GRRT_S2
+#undef GRRT_S3
+#undef GRRT_S4
+#undef GRRT_S5
+#undef GRRT_S6
+#undef GRRT_Q6
+#undef GRRT_QB
+#undef GRRT_QE
+#undef GRRT_QB5
+#undef GRRT_QE5
+#undef GRRT_QE6
+#undef GRRT_Y5
+    // the norm of dp45_attempt_k1, the largest quotient picked by a tree: with
+    // every term finite the order of the comparisons does not matter
+#define GRRT_N(f) fabs(__dmul_rn(h, __fma_rn(C.e7, k7.f, qe.f)))
+#define GRRT_D(f) __dadd_rn(fabs(y5.f), C.floor)
+    const ErrQuotient q[5] = {{GRRT_N(r), GRRT_D(r)},
+                              {GRRT_N(th), GRRT_D(th)},
+                              {GRRT_N(ph), GRRT_D(ph)},
+                              {GRRT_N(pr), GRRT_D(pr)},
+                              {GRRT_N(pth), GRRT_D(pth)}};
+#undef GRRT_N
+#undef GRRT_D
+    auto larger = [](const ErrQuotient& u, const ErrQuotient& v) {
+        const bool gt = __dmul_rn(u.num, v.den) < __dmul_rn(v.num, u.den);
+        return ErrQuotient{gt ? v.num : u.num, gt ? v.den : u.den};
+    };
+    int top = 0;
+#pragma unroll
+    for (int i = 0; i < 5; ++i) top = max(top, max(__double2hiint(q[i].num), __double2hiint(q[i].den)));
+    if (top >= 0x7ff00000) {  // an infinity or a NaN: the terms in order, a NaN skipped
+        ErrQuotient m{0.0, 1.0};
+        for (int i = 0; i < 5; ++i) m = larger(m, q[i]);
+        return m;
+    }
+    return larger(larger(larger(q[0], q[1]), larger(q[2], q[3])), q[4]);
+}
+#endif
 
 // One DP45 attempt with k1 = f(y) given by the caller: returns the error
 // norm, the 5th-order state in y5 and k7 = f(y5). The reference evaluates
@@ -58,6 +179,15 @@ GRRT_HD Vec5<T> rk4_step(T M, T a, T pt, T pph, const Vec5<T>& y, T h) {
 template <typename T>
 GRRT_HD T dp45_attempt_k1(T M, T a, T pt, T pph, const Vec5<T>& y, T h, const Vec5<T>& k1, Vec5<T>& y5,
                           Vec5<T>& k7_out) {
+#ifdef GRRT_RHS_PINNED
+    if constexpr (sizeof(T) == sizeof(double)) {
+        auto f = [&](double r, double th, double pr, double pth) {
+            return kerr_rhs<double>(M, a, pt, pph, Vec5<double>{r, th, 0.0, pr, pth});
+        };
+        const ErrQuotient q = dp45_attempt_f64(f, y, h, k1, y5, k7_out);
+        return div_f64(q.num, q.den);
+    }
+#endif
     using namespace dp;
 #define GRRT_S2(f) y.f + h * (T(a21) * k1.f)
     const Vec5<T> k2 = kerr_rhs<T>(M, a, pt, pph, Vec5<T>{GRRT_S2(r), GRRT_S2(th), GRRT_S2(ph), GRRT_S2(pr), GRRT_S2(pth)});
@@ -232,6 +362,14 @@ GRRT_HD double step_factor_pow(double x) {
 #endif
 }
 
+GRRT_HD double step_quotient(double tol, double err) {
+#ifdef GRRT_RHS_PINNED
+    return div_f64(tol, err);
+#else
+    return tol / err;
+#endif
+}
+
 // retry = number of rejected attempts so far in this outer step (0..20). The
 // 21st attempt (retry == 20) is taken unconditionally with next = dl, as the
 // reference's "exhausted retries" path.
@@ -247,14 +385,14 @@ GRRT_HD StepDecision pi_control(double err, double tol, double dl, int retry,
         return d;
     }
     if (err <= tol) {
-        double f = (err > 1e-30) ? safety * step_factor_pow(tol / err) : grow_max;
+        double f = (err > 1e-30) ? safety * step_factor_pow(step_quotient(tol, err)) : grow_max;
         f = (f < 1.0) ? 1.0 : (grow_max < f) ? grow_max : f;
         const double nx = dl * f;
         d.accept = true;
         d.next = (cap < nx) ? cap : nx;
         return d;
     }
-    double f = safety * step_factor_pow(tol / err);
+    double f = safety * step_factor_pow(step_quotient(tol, err));
     f = (f < shrink_max) ? shrink_max : (1.0 < f) ? 1.0 : f;
     const double ndl = dl * f;
     if (ndl < dl_min) {
@@ -266,6 +404,49 @@ GRRT_HD StepDecision pi_control(double err, double tol, double dl, int retry,
     d.next = ndl;
     return d;
 }
+
+#if defined(__CUDACC__) && !defined(GRRT_RHS_GENERIC)
+// pi_control of the error norm q.num / q.den, with the same decision and the
+// same step to the bit but without its two divisions in sequence: the factor
+// needs (tol / err) rounded to single precision only, so tol * den * (1 / num),
+// a few ulp off, rounds alike unless it lies that close to a rounding boundary,
+// and err <= tol is the same as that quotient >= 1 unless it is as close to 1.
+// Those cases (1 in 10^7), numbers near the range's ends and tolerances
+// where the 1e-30 rule could matter take pi_control. Positive doubles are
+// compared as integers, off the FP64 pipe.
+__device__ __forceinline__ StepDecision pi_control_q(const ErrQuotient& q, double tol, double dl, int retry,
+                                                     double r5) {
+    constexpr double safety = 0.9, grow_max = 5.0, shrink_max = 0.2, dl_min = 1e-6;
+    double y;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(q.num));
+    const double e = __fma_rn(-q.num, y, 1.0);
+    y = __fma_rn(y, __fma_rn(e, e, e), y);
+    const double ratio = __dmul_rn(__dmul_rn(tol, q.den), y);  // tol / err
+    const long long rb = __double_as_longlong(ratio);
+    // 2^-450 <= num, den < 2^450 (a negative or NaN num fails as well)
+    const bool in_range = static_cast<unsigned>(__double2hiint(q.num) - 0x23d00000) < 0x38400000u &&
+                          static_cast<unsigned>(__double2hiint(q.den) - 0x23d00000) < 0x38400000u;
+    const bool near_half = ((static_cast<unsigned>(rb) - 0x10000000u + 16u) & 0x1fffffffu) <= 32u;
+    const bool near_one = static_cast<unsigned long long>(rb - 0x3ff0000000000000ll + 64) <= 128ull;
+    if (!in_range || near_half || near_one || !(tol >= 1e-20 && tol <= 1e20))
+        return pi_control(div_f64(q.num, q.den), tol, dl, retry, r5);
+    auto less = [](double a, double b) { return __double_as_longlong(a) < __double_as_longlong(b); };
+    const bool ok = rb >= 0x3ff0000000000000ll;
+    double f = __dmul_rn(safety, static_cast<double>(__powf(static_cast<float>(ratio), 0.2f)));
+    const double lo = ok ? 1.0 : shrink_max, hi = ok ? grow_max : 1.0;
+    f = less(f, lo) ? lo : less(hi, f) ? hi : f;
+    const double ar = fabs(r5);
+    const double cap = __dmul_rn(5.0, less(ar, 1.0) ? 1.0 : ar);
+    const double nx = __dmul_rn(dl, f);
+    const bool tiny = !ok && less(nx, dl_min);
+    StepDecision d;
+    d.accept = ok || tiny || retry >= 20;
+    d.next = tiny ? dl_min : nx;
+    if ((ok || tiny) && less(cap, d.next)) d.next = cap;
+    if (retry >= 20) d.next = dl;
+    return d;
+}
+#endif
 
 // The FP32 pass's controller: pi_control with (tol/err)^0.2 formed from a
 // single-precision quotient (the FP32 error norm carries no more digits).

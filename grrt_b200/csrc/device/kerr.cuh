@@ -120,11 +120,147 @@ GRRT_HD float recip(float x) {
 #endif
 }
 
+#if defined(__CUDA_ARCH__) && !defined(GRRT_RHS_GENERIC)
+#define GRRT_RHS_PINNED 1
+#endif
+
+#if defined(__CUDACC__) && !defined(GRRT_RHS_GENERIC)
+// FP64 constants of the right-hand side and of the Dormand-Prince attempt, as
+// constant-bank operands: a 64-bit literal costs the instructions that build it
+// at every use.
+struct RhsConst {
+    double dp1, dp2, dp3, fopi, shift;
+    double s0, s1, s2, s3, s4, s5, c0, c1, c2, c3, c4, c5;
+};
+static __constant__ RhsConst kRhs = {
+    7.85398125648498535156e-1, 3.77489470793079817668e-8, 2.69515142907905952645e-15, 1.27323954473516268615,
+    6755399441055744.0,  // 1.5 * 2^52
+    -1.66666666666666324348e-01, 8.33333333332248946124e-03, -1.98412698298579493134e-04,
+    2.75573137070700676789e-06, -2.50507602534068634195e-08, 1.58969099521155010221e-10,
+    4.16666666666666019037e-02, -1.38888888888741095749e-03, 2.48015872894767294178e-05,
+    -2.75573143513906633035e-07, 2.08757232129817482790e-09, -1.13596475577881948265e-11};
+
+// fast_sincos and the right-hand side's pole clamp (|sin| >= 1e-10) with the
+// same bits in fewer instructions and a shorter chain. The octant comes from
+// one add to 1.5 * 2^52 rounded down (its low word then holds floor(|x| 4/pi)
+// + 1) instead of two conversions. The signs go into the polynomials' factors
+// and the clamp into the sine's argument (sin x = x that close to 0), beside
+// the chain through z.
+__device__ __forceinline__ void sincos_clamped_f64(double x, double& s, double& c) {
+    auto flip = [](double v, unsigned sign) {
+        return __hiloint2double(__double2hiint(v) ^ static_cast<int>(sign), __double2loint(v));
+    };
+    const double xa = fabs(x);
+    const double t = __dmul_rn(xa, kRhs.fopi);
+    const double u = __dadd_rd(t, kRhs.shift + 1.0);
+    int oct = __double2loint(u) & ~1;
+    double y = __dadd_rn(__hiloint2double(__double2hiint(u), oct), -kRhs.shift);
+    // past the int range (floor(t) + 1 >= 2^31) fast_sincos has -2^31, octant 0
+    if (__double_as_longlong(u) >= 0x4338000080000000ll) {
+        y = -2147483648.0;
+        oct = 0;
+    }
+    const double ax = __fma_rn(-y, kRhs.dp3, __fma_rn(-y, kRhs.dp2, __fma_rn(-y, kRhs.dp1, xa)));
+    const double z = __dmul_rn(ax, ax);
+    double ps = __fma_rn(kRhs.s5, z, kRhs.s4), pc = __fma_rn(kRhs.c5, z, kRhs.c4);
+    ps = __fma_rn(ps, z, kRhs.s3);
+    pc = __fma_rn(pc, z, kRhs.c3);
+    ps = __fma_rn(ps, z, kRhs.s2);
+    pc = __fma_rn(pc, z, kRhs.c2);
+    ps = __fma_rn(ps, z, kRhs.s1);
+    pc = __fma_rn(pc, z, kRhs.c1);
+    ps = __fma_rn(ps, z, kRhs.s0);
+    pc = __fma_rn(pc, z, kRhs.c0);
+    const bool swap = (oct & 2) != 0;
+    // sin: negative for x < 0 and in octants 4-7; cos: in octants 2-5
+    const unsigned ss = (static_cast<unsigned>(__double2hiint(x)) ^ (static_cast<unsigned>(oct) << 29)) & 0x80000000u;
+    const unsigned cs = (static_cast<unsigned>(oct + 2) << 29) & 0x80000000u;
+    const bool pole = !swap && (__double_as_longlong(ax) & 0x7fffffffffffffffll) < __double_as_longlong(1e-10);
+    const double ar = flip(pole ? copysign(1e-10, ax) : ax, swap ? cs : ss);
+    const unsigned rs = swap ? ss : cs;
+    const double sr = __fma_rn(__dmul_rn(ar, z), ps, ar);
+    const double cr = __fma_rn(flip(__dmul_rn(z, z), rs), pc, flip(__fma_rn(-0.5, z, 1.0), rs));
+    s = swap ? cr : sr;
+    c = swap ? sr : cr;
+}
+
+// 1/x, correctly rounded, without the branch of the division operator (which
+// splits the right-hand side into blocks the scheduler cannot interleave): of
+// |x|, the hardware approximation, one cubic and one quadratic Newton step with
+// the residuals exact in fused multiply-adds (P. Markstein, IBM J. Res. Dev.
+// 34, 1990). The cubic step rounds up, so that the last one starts from above
+// and also rounds an all-ones significand, its one exception, correctly.
+// x = inf gives 0; a zero or subnormal x or result is not handled (NaN or 0).
+__device__ __forceinline__ double recip_f64(double x) {
+    const int hi = __double2hiint(x);
+    const double xa = __hiloint2double(min(hi & 0x7fffffff, 0x7fe00000), __double2loint(x));
+    double y;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(xa));
+    double e = __fma_rn(-xa, y, 1.0);
+    y = __fma_ru(y, __fma_rn(e, e, e), y);
+    e = __fma_rn(-xa, y, 1.0);
+    y = __fma_rn(y, e, y);
+    return __hiloint2double(__double2hiint(y) ^ (hi & static_cast<int>(0x80000000u)), __double2loint(y));
+}
+
+// The FP64 right-hand side on the device, every rounding written out, so that
+// each inlined or called copy in each kernel returns the same bits (left to
+// the compiler, each copy's multiplies and adds are fused in its own way). It
+// is the generic body below with these products fused into their sums: the
+// first of Sigma, Delta, Q and H, a * p_phi of P and a * p_t of dG; the exact
+// factors of two are cancelled (2 H, dF / 2, dG / 2). One basic block.
+struct KerrHole {
+    double M, a;
+    double a2, m2;  // a^2, 2 M
+};
+
+__device__ __forceinline__ Vec5<double> kerr_rhs_f64(const KerrHole& K, double pt, double pph, double r, double th,
+                                                     double pr, double pth) {
+    const double a = K.a, a2 = K.a2;
+    double s, c;
+    sincos_clamped_f64(th, s, c);
+    const double r2 = __dmul_rn(r, r);
+    const double Sigma = __fma_rn(__dmul_rn(a2, c), c, r2);
+    const double Delta = __dadd_rn(__fma_rn(-K.m2, r, r2), a2);
+    const double SD = __dmul_rn(Sigma, Delta);
+    const double inv = recip_f64(__dmul_rn(SD, s));
+    const double iS = __dmul_rn(__dmul_rn(Delta, s), inv);  // 1/Sigma
+    const double iD = __dmul_rn(__dmul_rn(Sigma, s), inv);  // 1/Delta
+    const double is = __dmul_rn(SD, inv);                   // 1/sin(theta)
+    const double P = __fma_rn(a, pph, __dmul_rn(__dadd_rn(r2, a2), pt));
+    const double pis = __dmul_rn(pph, is);
+    const double Q = __fma_rn(__dmul_rn(a, s), pt, pis);
+    const double PiD = __dmul_rn(P, iD);
+    const double Dp = __dmul_rn(Delta, pr);
+    double X = __fma_rn(Dp, pr, -__dmul_rn(P, PiD));
+    X = __fma_rn(Q, Q, __fma_rn(pth, pth, X));
+    const double H2 = __dmul_rn(X, iS);  // 2 H, 0 on the light cone
+    // dx/dlambda = dH/dp
+    Vec5<double> d;
+    d.r = __dmul_rn(Dp, iS);
+    d.th = __dmul_rn(pth, iS);
+    d.ph = __dmul_rn(__fma_rn(Q, is, -__dmul_rn(a, PiD)), iS);
+    // half of dF/dr at fixed momenta and of dG/dtheta
+    const double pp = __fma_rn(pr, pr, __dmul_rn(PiD, PiD));
+    const double hF = __fma_rn(__dadd_rn(r, -K.M), pp, -__dmul_rn(__dmul_rn(r, 2.0 * pt), PiD));
+    const double hG = __dmul_rn(__dmul_rn(Q, c), __fma_rn(a, pt, -__dmul_rn(pis, is)));
+    // dp/dlambda = -dH/dx, with dSigma/dr = 2r and dSigma/dtheta = -2 a^2 sin cos
+    d.pr = __fma_rn(__dmul_rn(H2, r), iS, -__dmul_rn(hF, iS));
+    const double E = __dmul_rn(__dmul_rn(__dmul_rn(H2, a2), s), c);
+    d.pth = -__fma_rn(hG, iS, __dmul_rn(E, iS));
+    return d;
+}
+#endif
+
 // Returns dx/dlambda and dp/dlambda for (r, theta, phi, p_r, p_theta) given the
 // constants p_t, p_phi.
 template <typename T>
 GRRT_HD Vec5<T> kerr_rhs_body(T M, T a, T pt, T pph, const Vec5<T>& y) {
     using std::fabs;
+#ifdef GRRT_RHS_PINNED
+    if constexpr (sizeof(T) == sizeof(double)) 
+        return kerr_rhs_f64(KerrHole{M, a, a * a, 2.0 * M}, pt, pph, y.r, y.th, y.pr, y.pth);
+#endif
     const T r = y.r, pr = y.pr, pth = y.pth;
     T s, c;
     rhs_sincos(y.th, s, c);

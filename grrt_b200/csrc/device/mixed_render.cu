@@ -19,11 +19,11 @@
 // cameras at once (one sample space, items in order), so each phase is one
 // launch for the whole batch and every sample gets the arithmetic of its own
 // camera's single render.
-// One shared body of the FP64 right-hand side instead of seven inlined copies
-// per attempt: less code to fetch (Kerr a=0.998, 1024x1024, 4 spp: 46.4 ->
-// 43.4 ms for the FP64 form on B200). The FP64 form and the mixed form's
-// re-trace must use the same setting, so that their arithmetic is identical.
-#define GRRT_RHS_CALL_F64 1
+// The FP64 trace inlines the right-hand side into its attempt: with the
+// roundings written out (kerr.cuh) every copy has the same bits, and without
+// the calls an attempt is 1,060 instructions instead of 1,600 (Kerr a=0.998,
+// 1024x1024, 4 spp on B200: FP64 form 31.7 -> 24.0 ms, the mixed form's
+// re-trace 6.7 -> 5.3 ms; one lone ray 2.53 -> 1.71 us an attempt).
 #include <cuda_runtime.h>
 
 #include <cstdint>
@@ -170,7 +170,7 @@ mixed_speculate_kernel(const __grid_constant__ DevScene S0, const DevTile tile, 
                                   : (mb.spec_list ? *mb.spec_count
                                                   : static_cast<unsigned>(tile.w) * tile.h * (S0.grid * S0.grid));
     float Mf = static_cast<float>(S0.M), af = static_cast<float>(S0.a);
-    unsigned long long n_att = 0, n_acc = 0, n_rays = 0;
+    unsigned n_att = 0, n_acc = 0, n_rays = 0;
     // warp-uniform: prepared slots [ring_head, ring_n) and the queue state
     int ring_head = 0, ring_n = 0;
     bool drained = false;
@@ -389,6 +389,9 @@ struct WarpStage {
     double th[32], ph[32], c[3][32];          // escape direction and colour so far
     unsigned pq[32], pfate[32];
     const DevScene* psp[32];
+    // the lane's own sample: what it touches rarely, out of the registers
+    double col[3][32];    // colour so far
+    unsigned lq[32], ncross[32];
 };
 
 // Writes the parked escapes' colours (colour + star brightness, the order of
@@ -417,9 +420,12 @@ __device__ __forceinline__ void flush_star_lookups(WarpStage& W, int n, const De
 // form traces every sample of the tile (kList = false, work item = sample),
 // the mixed form's re-trace the listed ones (kList = true, work item = entry
 // of mb.retrace_list). Each loop iteration is one DP45 attempt for every lane
-// with a live ray. The per-sample work around it (camera ray, first
+// with a live ray; what follows an attempt is one vote unless a sample ended.
+// The per-sample work around it (camera ray, first
 // right-hand side, star lookup) runs for 32 samples at a time with the whole
-// warp (WarpStage), not lane by lane as rays end. counter: the work counter
+// warp (WarpStage), not lane by lane as rays end. Bound by the FP64 pipe (75%
+// active) and, with few samples, by the chain of one attempt; four blocks of
+// 128 registers: three 28.6 ms, five with 96 registers 24.6 ms (four: 24.5). counter: the work counter
 // (zeroed by the launcher), total: the item count for kList = false.
 template <bool kList, bool kBatch>
 __global__ void __launch_bounds__(kMixThreads, 4)
@@ -432,97 +438,105 @@ fp64_trace_kernel(const __grid_constant__ DevScene S0, const DevTile tile, const
     const DevScene* sp = nullptr;
 #define S (kBatch ? *sp : S0)
     const unsigned total = kList ? *mb.retrace_count : total_items;
-    unsigned long long n_att = 0, n_acc = 0, n_rays = 0;
+    unsigned n_att = 0, n_acc = 0, n_rays = 0;  // this lane's share
     // warp-uniform: prepared slots [ring_head, ring_n), parked lookups, queue state
     int ring_head = 0, ring_n = 0, pend_n = 0;
     bool drained = false;
-    unsigned q = 0;
     bool live = false;
-    Vec5<double> y, k1;  // k1 = f(y)
+    Vec5<double> y, k1;
     double pt = 0, pph = 0, dl = 0;
-    int retry = 0, step = 0, ncross = 0;
-    double c0 = 0, c1 = 0, c2 = 0;
+    int retry = 0, step = 0, term = -1;
+    unsigned need = kMask;  // warp-uniform: the lanes without a ray
     while (true) {
-        const unsigned need = __ballot_sync(kMask, !live);
-        // ---- the warp prepares its next 32 starts (every lane one) ----
-        if (need && ring_head == ring_n && !drained) {
-            unsigned base = 0;
-            if (lane == 0) base = atomicAdd(counter, 32u);
-            base = __shfl_sync(kMask, base, 0);
-            ring_head = 0;
-            ring_n = base < total ? static_cast<int>(min(32u, total - base)) : 0;
-            if (ring_n < 32) drained = true;
-            if (lane < ring_n) {
-                const unsigned w = base + lane;
-                const unsigned qq = kList ? mb.retrace_list[w] : w;
-                const DevScene* ssp = nullptr;
-                Vec5<double> ys;
-                double pts, pphs;
-                start_ray<kBatch>(S0, tile, B, qq, ssp, ys, pts, pphs);
-                const DevScene& Ss = kBatch ? *ssp : S0;
-                const Vec5<double> f = kerr_rhs<double>(Ss.M, Ss.a, pts, pphs, ys);
-                W.q[lane] = qq;
-                if (kBatch) W.sp[lane] = ssp;
-                W.pr[lane] = ys.pr;
-                W.pth[lane] = ys.pth;
-                W.pt[lane] = pts;
-                W.pph[lane] = pphs;
-                W.k[0][lane] = f.r;
-                W.k[1][lane] = f.th;
-                W.k[2][lane] = f.ph;
-                W.k[3][lane] = f.pr;
-                W.k[4][lane] = f.pth;
+        if (need) {
+            if (ring_head < ring_n || !drained) {
+                // ---- the warp prepares its next 32 starts (every lane one) ----
+                if (ring_head == ring_n && !drained) {
+                    unsigned base = 0;
+                    if (lane == 0) base = atomicAdd(counter, 32u);
+                    base = __shfl_sync(kMask, base, 0);
+                    ring_head = 0;
+                    ring_n = base < total ? static_cast<int>(min(32u, total - base)) : 0;
+                    if (ring_n < 32) drained = true;
+                    if (lane < ring_n) {
+                        const unsigned w = base + lane;
+                        const unsigned qq = kList ? mb.retrace_list[w] : w;
+                        const DevScene* ssp = nullptr;
+                        Vec5<double> ys;
+                        double pts, pphs;
+                        start_ray<kBatch>(S0, tile, B, qq, ssp, ys, pts, pphs);
+                        const DevScene& Ss = kBatch ? *ssp : S0;
+                        const Vec5<double> f = kerr_rhs<double>(Ss.M, Ss.a, pts, pphs, ys);
+                        W.q[lane] = qq;
+                        if (kBatch) W.sp[lane] = ssp;
+                        W.pr[lane] = ys.pr;
+                        W.pth[lane] = ys.pth;
+                        W.pt[lane] = pts;
+                        W.pph[lane] = pphs;
+                        W.k[0][lane] = f.r;
+                        W.k[1][lane] = f.th;
+                        W.k[2][lane] = f.ph;
+                        W.k[3][lane] = f.pr;
+                        W.k[4][lane] = f.pth;
+                    }
+                    __syncwarp();
+                }
+                // ---- lanes without a ray take the prepared starts in order ----
+                if (ring_head < ring_n) {
+                    const int avail = ring_n - ring_head;
+                    const int rank = __popc(need & lt_mask);
+                    if (!live && rank < avail) {
+                        const int slot = ring_head + rank;
+                        W.lq[lane] = W.q[slot];
+                        if (kBatch) sp = W.sp[slot];
+                        y = Vec5<double>{S.cam_pos[1], S.cam_pos[2], S.cam_pos[3], W.pr[slot], W.pth[slot]};
+                        pt = W.pt[slot];
+                        pph = W.pph[slot];
+                        k1 = Vec5<double>{W.k[0][slot], W.k[1][slot], W.k[2][slot], W.k[3][slot], W.k[4][slot]};
+                        dl = S.dl0;
+                        retry = 0;
+                        step = 0;
+                        term = start_test(S, 0, y.r);
+                        W.ncross[lane] = 0;
+                        W.col[0][lane] = W.col[1][lane] = W.col[2][lane] = 0.0;
+                        live = true;
+                        ++n_rays;
+                    }
+                    ring_head += min(__popc(need), avail);
+                    __syncwarp();
+                }
+                need = __ballot_sync(kMask, !live);
             }
-            __syncwarp();
+            if (need == kMask) break;  // no lane holds a ray and the queue is drained
         }
-        // ---- lanes without a ray take the prepared starts in order ----
-        if (need && ring_head < ring_n) {
-            const int avail = ring_n - ring_head;
-            const int rank = __popc(need & lt_mask);
-            if (!live && rank < avail) {
-                const int slot = ring_head + rank;
-                q = W.q[slot];
-                if (kBatch) sp = W.sp[slot];
-                y = Vec5<double>{S.cam_pos[1], S.cam_pos[2], S.cam_pos[3], W.pr[slot], W.pth[slot]};
-                pt = W.pt[slot];
-                pph = W.pph[slot];
-                k1 = Vec5<double>{W.k[0][slot], W.k[1][slot], W.k[2][slot], W.k[3][slot], W.k[4][slot]};
-                dl = S.dl0;
-                retry = 0;
-                step = 0;
-                ncross = 0;
-                c0 = c1 = c2 = 0.0;
-                live = true;
-                ++n_rays;
-            }
-            ring_head += min(__popc(need), avail);
-            __syncwarp();
-        }
-        // No lane holds a ray: the queue is drained (a lane without a ray
-        // would have taken a prepared start, and a refill found none).
-        if (!__any_sync(kMask, live)) break;
-        int term = -1;
-        if (live && retry == 0) term = start_test(S, step, y.r);
         if (live && term < 0) {
             Vec5<double> y5, k7;
-            const double err = dp45_attempt_k1<double>(S.M, S.a, pt, pph, y, dl, k1, y5, k7);
+            auto rhs = [&](double r, double th, double pr, double pth) {
+                return kerr_rhs_f64(KerrHole{S.M, S.a, S.a2, S.m2}, pt, pph, r, th, pr, pth);
+            };
+            const ErrQuotient err = dp45_attempt_f64(rhs, y, dl, k1, y5, k7);
             ++n_att;
-            const StepDecision d = pi_control(err, S.tol, dl, retry, y5.r);
+            const StepDecision d = pi_control_q(err, S.tol, dl, retry, y5.r);
             if (d.accept) {
                 ++n_acc;
                 if (S.disk_on) {
-                    const double d_prev = y.th - kHalfPi;
-                    const double d_new = y5.th - kHalfPi;
-                    if (d_prev * d_new < 0.0 && fabs(d_prev - d_new) > 1e-12) {
-                        const double frac = -d_prev / (d_new - d_prev);
-                        const double rc = y.r + frac * (y5.r - y.r);
-                        if (rc >= S.r_in && rc <= S.r_out) {
-                            double e0, e1, e2;
-                            disk_emission(S, rc, pt, pph, e0, e1, e2);
-                            c0 += e0;
-                            c1 += e1;
-                            c2 += e2;
-                            ++ncross;
+                    // sides of the equator by integer comparison: only a step
+                    // that changes side can pass the test below
+                    const long long hp = __double_as_longlong(kHalfPi);
+                    if ((__double_as_longlong(y.th) <= hp) != (__double_as_longlong(y5.th) < hp)) {
+                        const double d_prev = y.th - kHalfPi;
+                        const double d_new = y5.th - kHalfPi;
+                        if (d_prev * d_new < 0.0 && fabs(d_prev - d_new) > 1e-12) {
+                            const double frac = -d_prev / (d_new - d_prev);
+                            const double rc = y.r + frac * (y5.r - y.r);
+                            if (rc >= S.r_in && rc <= S.r_out) {
+                                double e0, e1, e2;
+                                disk_emission(S, rc, pt, pph, e0, e1, e2);
+                                W.col[0][lane] += e0;
+                                W.col[1][lane] += e1;
+                                W.col[2][lane] += e2;
+                                ++W.ncross[lane];
+                            }
                         }
                     }
                 }
@@ -552,9 +566,11 @@ fp64_trace_kernel(const __grid_constant__ DevScene S0, const DevTile tile, const
         }
         // ---- finished samples: park escapes under a star sky, write the rest ----
         const bool fin = live && term >= 0;
+        const unsigned fmask = __ballot_sync(kMask, fin);
+        if (!fmask) continue;
+        need |= fmask;
         const bool star = fin && term == kTermEscaped && S.stars_on;
-        const unsigned nc = (ncross > 0x3fffffff) ? 0x3fffffffu : static_cast<unsigned>(ncross);
-        const unsigned fate = static_cast<unsigned>(term) | (nc << 2);
+        auto fate = [&] { return static_cast<unsigned>(term) | (min(W.ncross[lane], 0x3fffffffu) << 2); };
         const unsigned smask = __ballot_sync(kMask, star);
         if (smask) {
             const int ns = __popc(smask);
@@ -566,11 +582,10 @@ fp64_trace_kernel(const __grid_constant__ DevScene S0, const DevTile tile, const
                 const int slot = pend_n + __popc(smask & lt_mask);
                 W.th[slot] = y.th;
                 W.ph[slot] = y.ph;
-                W.c[0][slot] = c0;
-                W.c[1][slot] = c1;
-                W.c[2][slot] = c2;
-                W.pq[slot] = q;
-                W.pfate[slot] = fate;
+#pragma unroll
+                for (int k = 0; k < 3; ++k) W.c[k][slot] = W.col[k][lane];
+                W.pq[slot] = W.lq[lane];
+                W.pfate[slot] = fate();
                 if (kBatch) W.psp[slot] = sp;
             }
             pend_n += ns;
@@ -579,10 +594,10 @@ fp64_trace_kernel(const __grid_constant__ DevScene S0, const DevTile tile, const
         if (fin) {
             live = false;
             if (!star) {
-                mb.sample_rgb[3 * static_cast<size_t>(q) + 0] = c0;
-                mb.sample_rgb[3 * static_cast<size_t>(q) + 1] = c1;
-                mb.sample_rgb[3 * static_cast<size_t>(q) + 2] = c2;
-                mb.sample_fate[q] = fate;
+                const size_t q = W.lq[lane];
+#pragma unroll
+                for (int k = 0; k < 3; ++k) mb.sample_rgb[3 * q + k] = W.col[k][lane];
+                mb.sample_fate[q] = fate();
             }
         }
     }

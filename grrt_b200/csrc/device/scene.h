@@ -46,6 +46,7 @@ struct DevVolume {
 struct DevScene {
     // spacetime and integrator
     double M = 1, a = 0;
+    double a2 = 0, m2 = 2;  // a^2 and 2 M, operands of the right-hand side
     double r_stop = 0;      // horizon radius + 0.01 (termination)
     double r_escape = 1000; // escape radius
     double tol = 1e-8;

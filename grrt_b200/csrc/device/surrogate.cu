@@ -2,6 +2,7 @@
 // integrator, the MLP's non-GEMM training kernels (the GEMMs are
 // umma_gemm.cu, inference is mlp_fused.cu), and the surrogate render's
 // prepare / shade passes.
+#define GRRT_RHS_GENERIC 1
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
