@@ -245,6 +245,8 @@ bool GRRTContext::ensure_device() {
         V.a = vol->a;
         V.r_min = vol->r_min;
         V.r_outer = vol->r_outer;
+        V.span = V.r_outer - V.r_min;
+        V.inv_span = 1.0 / V.span;
         V.r_isco = vol->r_isco;
         V.r_horizon = vol->r_horizon;
         V.taper_width = vol->taper_width;

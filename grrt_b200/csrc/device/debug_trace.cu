@@ -7,7 +7,7 @@
 // and an END record (termination, colour, attempts).
 //
 // The steps are the render kernels' own: dp45_attempt_k1 with the kept k1,
-// pi_control, vol_clamp, vol_enters and vol_march_rgb_step, so the record
+// pi_control, vol_clamp, vol_enters and vol_march_rgb, so the record
 // list describes the ray those kernels trace for the same sample. Like the
 // reference's debug trace, the END colour is the disk's (and the volume's)
 // emission only; the sky is not added. One thread does the work: the trace is
@@ -95,7 +95,7 @@ __global__ void __launch_bounds__(32) debug_trace_kernel(const __grid_constant__
             k1 = kerr_rhs<double>(S.M, S.a, pt, pph, y);
             k1_ok = true;
         }
-        if (vol && vol_clamp(S, k1, y, dlambda)) ++cnt.clamp;
+        if (vol && vol_near_radius(V, y.r) && vol_clamp(k1, y.r, vol_geo(V, y.r, y.th), dlambda)) ++cnt.clamp;
         const Vec5<double> prev = y;
         double dl = dlambda;
         Vec5<double> y5, k7;
@@ -117,15 +117,17 @@ __global__ void __launch_bounds__(32) debug_trace_kernel(const __grid_constant__
             const bool opaque = (Tt[0] < 1e-6 && Tt[1] < 1e-6 && Tt[2] < 1e-6);
             const int event = opaque ? kDebugNone : vol_event(V, prev, y);
             out.put(kDebugStep, step, event, 0, y.r, y.th, z, dlambda, v_scale_height(V, y.r), v_zmax(V, y.r), y.ph);
-            if (!opaque && vol_enters(V, prev, y)) {
+            const VolGeo gp = vol_geo(V, prev.r, prev.th);
+            if (!opaque && vol_may_enter(V, prev.r, y.r) && vol_enters(V, prev, gp, y, vol_geo(V, y.r, y.th))) {
                 out.put(kDebugMarchEntry, step, 0, 0, prev.r, prev.r * cos(prev.th));
                 Vec5<double> ms = prev;
                 bool been_inside = false;
-                double ds = vol_march_start(V, ms, been_inside);
+                double ds = vol_march_start(V, ms.r, gp, been_inside);
                 int mcount = 0;
                 bool end = false;
                 while (!end) {
-                    end = vol_march_rgb_step(S, pt, pph, ms, ds, been_inside, J, Tt, cnt);
+                    ms = rk4_step<double>(S.M, S.a, pt, pph, ms, ds);
+                    end = vol_march_rgb(S, pt, pph, ms, vol_geo(V, ms.r, ms.th), ds, been_inside, J, Tt, cnt);
                     ++mcount;
                     if (!end && mcount >= 4096) end = true;
                 }

@@ -38,28 +38,6 @@ GRRT_HD Vec5<T> axpy(const Vec5<T>& y, T h, const Vec5<T>& k) {
     return Vec5<T>{y.r + h * k.r, y.th + h * k.th, y.ph + h * k.ph, y.pr + h * k.pr, y.pth + h * k.pth};
 }
 
-// Classic RK4 step (include/grrt/geodesic/rk4.h:34-52).
-template <typename T>
-GRRT_HD Vec5<T> rk4_step(T M, T a, T pt, T pph, const Vec5<T>& y, T h) {
-    const Vec5<T> k1 = kerr_rhs<T>(M, a, pt, pph, y);
-    const Vec5<T> k2 = kerr_rhs<T>(M, a, pt, pph, axpy(y, h * T(0.5), k1));
-    const Vec5<T> k3 = kerr_rhs<T>(M, a, pt, pph, axpy(y, h * T(0.5), k2));
-    const Vec5<T> k4 = kerr_rhs<T>(M, a, pt, pph, axpy(y, h, k3));
-    const T w = h / T(6);
-#ifdef GRRT_RHS_PINNED
-    if constexpr (sizeof(T) == sizeof(double)) {
-        // the roundings the compiler picks where k1 comes from a call
-#define GRRT_RK4F(f) \
-    __fma_rn(__dadd_rn(__fma_rn(2.0, k3.f, __fma_rn(2.0, k2.f, k1.f)), k4.f), w, y.f)
-        return Vec5<T>{GRRT_RK4F(r), GRRT_RK4F(th), GRRT_RK4F(ph), GRRT_RK4F(pr), GRRT_RK4F(pth)};
-#undef GRRT_RK4F
-    }
-#endif
-#define GRRT_RK4C(f) y.f + (k1.f + T(2) * k2.f + T(2) * k3.f + k4.f) * w
-    return Vec5<T>{GRRT_RK4C(r), GRRT_RK4C(th), GRRT_RK4C(ph), GRRT_RK4C(pr), GRRT_RK4C(pth)};
-#undef GRRT_RK4C
-}
-
 #if defined(__CUDACC__) && !defined(GRRT_RHS_GENERIC)
 struct DpConst {
     double a21, a31, a32, a41, a42, a43, a51, a52, a53, a54, a61, a62, a63, a64, a65;
@@ -91,46 +69,39 @@ struct ErrQuotient {
     double num, den;  // error norm = num / den
 };
 
-template <typename F>
-__device__ __forceinline__ ErrQuotient dp45_attempt_f64(const F& f, const Vec5<double>& y, double h, const Vec5<double>& k1,
-                                                   Vec5<double>& y5, Vec5<double>& k7) {
-    const DpConst& C = kDp;
-    auto two = [](double c1, double x1, double c2, double x2) { return __fma_rn(c1, x1, __dmul_rn(c2, x2)); };
-#define GRRT_F4(s) f(s(r), s(th), s(pr), s(pth))
 #define GRRT_V4(s) {s(r), s(th), 0.0, s(pr), s(pth)}
 #define GRRT_V5(s) {s(r), s(th), s(ph), s(pr), s(pth)}
-#define GRRT_S2(f) __fma_rn(h, __dmul_rn(C.a21, k1.f), y.f)
-    const Vec5<double> k2 = GRRT_F4(GRRT_S2);
-#define GRRT_S3(f) __fma_rn(h, two(C.a31, k1.f, C.a32, k2.f), y.f)
-    const Vec5<double> k3 = GRRT_F4(GRRT_S3);
-#define GRRT_S4(f) __fma_rn(h, __fma_rn(C.a43, k3.f, two(C.a41, k1.f, C.a42, k2.f)), y.f)
-    const Vec5<double> k4 = GRRT_F4(GRRT_S4);
-#define GRRT_Q6(f) __fma_rn(C.a64, k4.f, __fma_rn(C.a63, k3.f, two(C.a61, k1.f, C.a62, k2.f)))
+__device__ __forceinline__ double sum2_f64(double c1, double x1, double c2, double x2) {
+    return __fma_rn(c1, x1, __dmul_rn(c2, x2));
+}
+
+// The attempt from its fourth stage on.
+template <typename F>
+__device__ __forceinline__ ErrQuotient dp45_tail_f64(const F& f, const Vec5<double>& y, double h,
+                                                     const Vec5<double>& k1, const Vec5<double>& k2,
+                                                     const Vec5<double>& k3, const Vec5<double>& k4, Vec5<double>& y5,
+                                                     Vec5<double>& k7) {
+    const DpConst& C = kDp;
+#define GRRT_Q6(f) __fma_rn(C.a64, k4.f, __fma_rn(C.a63, k3.f, sum2_f64(C.a61, k1.f, C.a62, k2.f)))
     const Vec5<double> q6 GRRT_V4(GRRT_Q6);
-#define GRRT_QB(f) __fma_rn(C.b4, k4.f, two(C.b1, k1.f, C.b3, k3.f))
+#define GRRT_QB(f) __fma_rn(C.b4, k4.f, sum2_f64(C.b1, k1.f, C.b3, k3.f))
     Vec5<double> qb GRRT_V5(GRRT_QB);
-#define GRRT_QE(f) __fma_rn(C.e4, k4.f, two(C.e1, k1.f, C.e3, k3.f))
+#define GRRT_QE(f) __fma_rn(C.e4, k4.f, sum2_f64(C.e1, k1.f, C.e3, k3.f))
     Vec5<double> qe GRRT_V5(GRRT_QE);
 #define GRRT_S5(f) \
-    __fma_rn(h, __fma_rn(C.a54, k4.f, __fma_rn(C.a53, k3.f, two(C.a51, k1.f, C.a52, k2.f))), y.f)
-    const Vec5<double> k5 = GRRT_F4(GRRT_S5);
+    __fma_rn(h, __fma_rn(C.a54, k4.f, __fma_rn(C.a53, k3.f, sum2_f64(C.a51, k1.f, C.a52, k2.f))), y.f)
+    const Vec5<double> k5 = f(Vec5<double> GRRT_V4(GRRT_S5));
 #define GRRT_QB5(f) __fma_rn(C.b5, k5.f, qb.f)
     qb = GRRT_V5(GRRT_QB5);
 #define GRRT_QE5(f) __fma_rn(C.e5, k5.f, qe.f)
     qe = GRRT_V5(GRRT_QE5);
 #define GRRT_S6(f) __fma_rn(h, __fma_rn(C.a65, k5.f, q6.f), y.f)
-    const Vec5<double> k6 = GRRT_F4(GRRT_S6);
+    const Vec5<double> k6 = f(Vec5<double> GRRT_V4(GRRT_S6));
 #define GRRT_Y5(f) __fma_rn(h, __fma_rn(C.b6, k6.f, qb.f), y.f)
     y5 = GRRT_V5(GRRT_Y5);
 #define GRRT_QE6(f) __fma_rn(C.e6, k6.f, qe.f)
     qe = GRRT_V5(GRRT_QE6);
-    k7 = f(y5.r, y5.th, y5.pr, y5.pth);
-#undef GRRT_F4
-#undef GRRT_V4
-#undef GRRT_V5
-#undef GRRT_S2
-#undef GRRT_S3
-#undef GRRT_S4
+    k7 = f(y5);
 #undef GRRT_S5
 #undef GRRT_S6
 #undef GRRT_Q6
@@ -165,7 +136,73 @@ __device__ __forceinline__ ErrQuotient dp45_attempt_f64(const F& f, const Vec5<d
     }
     return larger(larger(larger(q[0], q[1]), larger(q[2], q[3])), q[4]);
 }
+
+// f: the right-hand side of a state (its phi unused).
+template <typename F>
+__device__ __forceinline__ ErrQuotient dp45_attempt_f64(const F& f, const Vec5<double>& y, double h,
+                                                        const Vec5<double>& k1, Vec5<double>& y5, Vec5<double>& k7) {
+    const DpConst& C = kDp;
+#define GRRT_S2(f) __fma_rn(h, __dmul_rn(C.a21, k1.f), y.f)
+    const Vec5<double> k2 = f(Vec5<double> GRRT_V4(GRRT_S2));
+#define GRRT_S3(f) __fma_rn(h, sum2_f64(C.a31, k1.f, C.a32, k2.f), y.f)
+    const Vec5<double> k3 = f(Vec5<double> GRRT_V4(GRRT_S3));
+#define GRRT_S4(f) __fma_rn(h, __fma_rn(C.a43, k3.f, sum2_f64(C.a41, k1.f, C.a42, k2.f)), y.f)
+    const Vec5<double> k4 = f(Vec5<double> GRRT_V4(GRRT_S4));
+#undef GRRT_S2
+#undef GRRT_S3
+#undef GRRT_S4
+    return dp45_tail_f64(f, y, h, k1, k2, k3, k4, y5, k7);
+}
+
+// Stages 2 to 4 of an attempt, or of a classic RK4 step (rk4_step: its stage
+// coefficients 1/2, 1/2, 1 in the same sums, where a zero coefficient leaves
+// the bits), so that lanes of both kinds evaluate these right-hand sides
+// together.
+template <typename F>
+__device__ __forceinline__ void shared_stages_f64(const F& f, bool rk4, const Vec5<double>& y, double h,
+                                                  const Vec5<double>& k1, Vec5<double>& k2, Vec5<double>& k3,
+                                                  Vec5<double>& k4) {
+    const double c21 = rk4 ? 0.5 : kDp.a21, c31 = rk4 ? 0.0 : kDp.a31, c32 = rk4 ? 0.5 : kDp.a32;
+    const double c41 = rk4 ? 0.0 : kDp.a41, c42 = rk4 ? 0.0 : kDp.a42, c43 = rk4 ? 1.0 : kDp.a43;
+#define GRRT_S2(f) __fma_rn(h, __dmul_rn(c21, k1.f), y.f)
+    k2 = f(Vec5<double> GRRT_V4(GRRT_S2));
+#define GRRT_S3(f) __fma_rn(h, sum2_f64(c31, k1.f, c32, k2.f), y.f)
+    k3 = f(Vec5<double> GRRT_V4(GRRT_S3));
+#define GRRT_S4(f) __fma_rn(h, __fma_rn(c43, k3.f, sum2_f64(c41, k1.f, c42, k2.f)), y.f)
+    k4 = f(Vec5<double> GRRT_V4(GRRT_S4));
+#undef GRRT_S2
+#undef GRRT_S3
+#undef GRRT_S4
+}
+
+// The end state of an RK4 step of length h from its four right-hand sides.
+__device__ __forceinline__ Vec5<double> rk4_end_f64(const Vec5<double>& y, double h, const Vec5<double>& k1,
+                                                    const Vec5<double>& k2, const Vec5<double>& k3,
+                                                    const Vec5<double>& k4) {
+    const double w = div_f64(h, 6.0);
+#define GRRT_R4(f) __fma_rn(__dadd_rn(__fma_rn(2.0, k3.f, __fma_rn(2.0, k2.f, k1.f)), k4.f), w, y.f)
+    return Vec5<double> GRRT_V5(GRRT_R4);
+#undef GRRT_R4
+}
+#undef GRRT_V4
+#undef GRRT_V5
 #endif
+
+// Classic RK4 step (include/grrt/geodesic/rk4.h:34-52).
+template <typename T>
+GRRT_HD Vec5<T> rk4_step(T M, T a, T pt, T pph, const Vec5<T>& y, T h) {
+    const Vec5<T> k1 = kerr_rhs<T>(M, a, pt, pph, y);
+    const Vec5<T> k2 = kerr_rhs<T>(M, a, pt, pph, axpy(y, h * T(0.5), k1));
+    const Vec5<T> k3 = kerr_rhs<T>(M, a, pt, pph, axpy(y, h * T(0.5), k2));
+    const Vec5<T> k4 = kerr_rhs<T>(M, a, pt, pph, axpy(y, h, k3));
+#ifdef GRRT_RHS_PINNED
+    if constexpr (sizeof(T) == sizeof(double)) return rk4_end_f64(y, h, k1, k2, k3, k4);
+#endif
+    const T w = h / T(6);
+#define GRRT_RK4C(f) y.f + (k1.f + T(2) * k2.f + T(2) * k3.f + k4.f) * w
+    return Vec5<T>{GRRT_RK4C(r), GRRT_RK4C(th), GRRT_RK4C(ph), GRRT_RK4C(pr), GRRT_RK4C(pth)};
+#undef GRRT_RK4C
+}
 
 // One DP45 attempt with k1 = f(y) given by the caller: returns the error
 // norm, the 5th-order state in y5 and k7 = f(y5). The reference evaluates
@@ -181,9 +218,7 @@ GRRT_HD T dp45_attempt_k1(T M, T a, T pt, T pph, const Vec5<T>& y, T h, const Ve
                           Vec5<T>& k7_out) {
 #ifdef GRRT_RHS_PINNED
     if constexpr (sizeof(T) == sizeof(double)) {
-        auto f = [&](double r, double th, double pr, double pth) {
-            return kerr_rhs<double>(M, a, pt, pph, Vec5<double>{r, th, 0.0, pr, pth});
-        };
+        auto f = [&](const Vec5<double>& s) { return kerr_rhs<double>(M, a, pt, pph, s); };
         const ErrQuotient q = dp45_attempt_f64(f, y, h, k1, y5, k7_out);
         return div_f64(q.num, q.den);
     }

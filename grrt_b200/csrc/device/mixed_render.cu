@@ -511,8 +511,8 @@ fp64_trace_kernel(const __grid_constant__ DevScene S0, const DevTile tile, const
         }
         if (live && term < 0) {
             Vec5<double> y5, k7;
-            auto rhs = [&](double r, double th, double pr, double pth) {
-                return kerr_rhs_f64(KerrHole{S.M, S.a, S.a2, S.m2}, pt, pph, r, th, pr, pth);
+            auto rhs = [&](const Vec5<double>& s) {
+                return kerr_rhs_f64(KerrHole{S.M, S.a, S.a2, S.m2}, pt, pph, s.r, s.th, s.pr, s.pth);
             };
             const ErrQuotient err = dp45_attempt_f64(rhs, y, dl, k1, y5, k7);
             ++n_att;

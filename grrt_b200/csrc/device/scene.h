@@ -28,6 +28,7 @@ struct DevVolume {
     double r_min = 0, r_outer = 0, r_isco = 0, r_horizon = 0, taper_width = 0;
     double E_isco = 0, L_isco = 0, rho_scale = 1, noise_scale = 1, turbulence = 0;
     double inv_taper_w2 = 0;
+    double span = 1, inv_span = 1;    // r_outer - r_min and 1 / span, for the radial tables' coordinate
     int octaves = 2, n_r = 500, n_z = 128;
     const double* H = nullptr;        // n_r
     const double* z_max = nullptr;    // n_r

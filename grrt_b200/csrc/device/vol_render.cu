@@ -8,14 +8,10 @@
 // Same persistent execution model as the thin-disk kernel: a lane owns one
 // pixel, one loop iteration advances each live ray by one DP45 attempt (outer
 // phase) or one RK4 march step (march phase); the three channels' transfer
-// state sits in registers. The list instantiation is the FP64 re-trace of the
-// mixed form (its speculation is in vol_spectral.cu).
-// One shared body of the FP64 right-hand side instead of inlined copies: the
-// launches end on a few long rays, where instruction fetch stalls (Kerr
-// a=0.9, 512x512 RGB: 49 -> 41 ms for the FP64 form on B200). The FP64 form
-// and the mixed form's re-trace are both in this file, so their arithmetic is
-// identical.
-#define GRRT_RHS_CALL_F64 1
+// state sits in registers. As in the spectral kernel, a step keeps what the
+// next one needs and both kinds of step share their stages 2 to 4 (Kerr a=0.9,
+// 512x512, mixed form on B200: 42 -> 31 ms). The list instantiation is the FP64
+// re-trace of the mixed form (its speculation is in vol_spectral.cu).
 #include <cuda_runtime.h>
 
 #include <cstdint>
@@ -59,128 +55,153 @@ vol_render_kernel(const __grid_constant__ DevScene S, const DevTile tile, float4
     int pix = -1, smp = 0;
     double acc[3] = {0.0, 0.0, 0.0};
     bool live = false, need_start = false, marching = false;
-    Vec5<double> y{}, prev{};
+    // the outer loop's state, or the march's (which starts from the state
+    // before the step that handed over)
+    Vec5<double> y{};
     Vec5<double> k1{};  // f(y) while k1_ok: the last accepted attempt's k7 or this step's first stage
     bool k1_ok = false;
-    double pt = 0.0, pph = 0.0, dl = 0.0, dlambda = 0.0;
+    VolGeo geo{};       // the geometry of y while geo_ok
+    bool geo_ok = false;
+    double pt = 0.0, pph = 0.0, dl = 0.0, dlambda = 0.0;  // dl: trial step, or the march's step
     int retry = 0, step = 0, entries = 0;
     // transfer state (RGB in registers)
     double J[3] = {0.0, 0.0, 0.0}, Tt[3] = {1.0, 1.0, 1.0};
-    // march state
-    Vec5<double> ms{};
-    double ds = 0.0;
     int mcount = 0;
     bool been_inside = false;
     bool cancelled = false;
     unsigned iter = 0;
+    bool refill = true;  // warp-uniform: some lane has no ray
 
     while (true) {
-        // ---- refill ----
-        const bool want = (pix == -1);
-        const unsigned want_mask = __ballot_sync(kFullMask, want);
-        if (want_mask) {
-            unsigned base = 0;
-            const int leader = __ffs(want_mask) - 1;
-            if (lane == leader) base = atomicAdd(queue, static_cast<unsigned>(__popc(want_mask)));
-            base = __shfl_sync(kFullMask, base, leader);
-            if (want) {
-                const unsigned q = base + __popc(want_mask & lt_mask);
-                if (q < total) {
-                    pix = static_cast<int>(kList ? list[q] : q);  // kList: the listed sample
-                    smp = 0;
-                    acc[0] = acc[1] = acc[2] = 0.0;
-                } else {
-                    pix = -2;
+        if (refill) {
+            // ---- refill ----
+            const bool want = (pix == -1);
+            const unsigned want_mask = __ballot_sync(kFullMask, want);
+            if (want_mask) {
+                unsigned base = 0;
+                const int leader = __ffs(want_mask) - 1;
+                if (lane == leader) base = atomicAdd(queue, static_cast<unsigned>(__popc(want_mask)));
+                base = __shfl_sync(kFullMask, base, leader);
+                if (want) {
+                    const unsigned q = base + __popc(want_mask & lt_mask);
+                    if (q < total) {
+                        pix = static_cast<int>(kList ? list[q] : q);  // kList: the listed sample
+                        smp = 0;
+                        acc[0] = acc[1] = acc[2] = 0.0;
+                    } else {
+                        pix = -2;
+                    }
                 }
             }
-        }
-        if (!live && pix >= 0) {
-            const int pixel = kList ? pix / grid2 : pix;
-            const int s = kList ? pix % grid2 : smp;
-            const int qx = pixel % tile.w, qy = pixel / tile.w;
-            const int i = tile.x0 + qx, j = tile.y0 + qy * tile.row_step;
-            const int sy = s / S.grid, sx = s % S.grid;
-            const double x = i + (sx + pixel_hash(i, j, s, 0)) * S.cell;
-            const double yy = j + (sy + pixel_hash(i, j, s, 1)) * S.cell;
-            double p[4];
-            camera_momentum(S, x, yy, p);
-            y = Vec5<double>{S.cam_pos[1], S.cam_pos[2], S.cam_pos[3], p[1], p[2]};
-            pt = p[0];
-            pph = p[3];
-            dlambda = S.dl0;
-            step = 0;
-            entries = 0;
-            marching = false;
-            J[0] = J[1] = J[2] = 0.0;
-            Tt[0] = Tt[1] = Tt[2] = 1.0;
-            k1_ok = false;
-            live = true;
-            need_start = true;
+            if (!live && pix >= 0) {
+                const int pixel = kList ? pix / grid2 : pix;
+                const int s = kList ? pix % grid2 : smp;
+                const int qx = pixel % tile.w, qy = pixel / tile.w;
+                const int i = tile.x0 + qx, j = tile.y0 + qy * tile.row_step;
+                const int sy = s / S.grid, sx = s % S.grid;
+                const double x = i + (sx + pixel_hash(i, j, s, 0)) * S.cell;
+                const double yy = j + (sy + pixel_hash(i, j, s, 1)) * S.cell;
+                double p[4];
+                camera_momentum(S, x, yy, p);
+                y = Vec5<double>{S.cam_pos[1], S.cam_pos[2], S.cam_pos[3], p[1], p[2]};
+                pt = p[0];
+                pph = p[3];
+                dlambda = S.dl0;
+                step = 0;
+                entries = 0;
+                marching = false;
+                J[0] = J[1] = J[2] = 0.0;
+                Tt[0] = Tt[1] = Tt[2] = 1.0;
+                k1_ok = false;
+                geo_ok = false;
+                live = true;
+                need_start = true;
+            }
+            if (!__any_sync(kFullMask, live || pix >= -1)) break;
+            refill = false;
         }
 
         int term = -1;
-        // ---- start of an outer step: termination tests, then the near-disk clamp ----
+        // ---- start of an outer step: termination tests ----
         if (live && need_start) {
             if (step >= S.max_steps) term = kTermMaxSteps;
             else if (y.r < S.r_stop) term = kTermHorizon;
             else if (y.r > S.r_escape) term = kTermEscaped;
-            if (term < 0) {
-                if (!k1_ok) {
-                    k1 = kerr_rhs<double>(S.M, S.a, pt, pph, y);
-                    k1_ok = true;
+        }
+        auto rhs = [&](const Vec5<double>& s) {
+            return kerr_rhs_f64(KerrHole{S.M, S.a, S.a2, S.m2}, pt, pph, s.r, s.th, s.pr, s.pth);
+        };
+        if (live && term < 0) {
+            // ---- first stage, where the last step did not leave it (a march's first step
+            //      takes the outer step's) ----
+            if (!k1_ok) {
+                k1 = rhs(y);
+                k1_ok = true;
+            }
+            // ---- near-disk clamp of a new outer step ----
+            if (need_start) {
+                if (vol_near_radius(V, y.r)) {
+                    if (!geo_ok) geo = vol_geo(V, y.r, y.th);
+                    geo_ok = true;
+                    if (vol_clamp(k1, y.r, geo, dlambda)) ++cnt.clamp;
                 }
-                if (vol_clamp(S, k1, y, dlambda)) ++cnt.clamp;
-                prev = y;
                 dl = dlambda;
                 retry = 0;
                 need_start = false;
             }
-        }
-
-        if (live && term < 0 && !marching) {
-            // ---- one DP45 attempt ----
-            Vec5<double> y5, k7;
-            const double err = dp45_attempt_k1<double>(S.M, S.a, pt, pph, y, dl, k1, y5, k7);
-            ++cnt.fp64;
-            ++cnt.attempts;
-            const StepDecision d = pi_control(err, S.tol, dl, retry, y5.r);
-            if (!d.accept) {
-                dl = d.next;
-                ++retry;
-            } else {
-                ++cnt.accepted;
-                y = y5;
-                k1 = k7;
-                dlambda = d.next;
-                ++step;  // the reference's loop counter advances on every outer iteration
-                // hand-over to the ray-march (src/geodesic_tracer.cpp:105-153)
-                const bool opaque = (Tt[0] < 1e-6 && Tt[1] < 1e-6 && Tt[2] < 1e-6);
-                if (!opaque && vol_enters(V, prev, y)) {
-                    // march from the pre-step state
-                    marching = true;
-                    ++entries;
-                    ms = prev;
-                    ds = vol_march_start(V, ms, been_inside);
-                    mcount = 0;
+            Vec5<double> k2, k3, k4;
+            shared_stages_f64(rhs, marching, y, dl, k1, k2, k3, k4);
+            if (!marching) {
+                // ---- the rest of the DP45 attempt ----
+                Vec5<double> y5, k7;
+                const ErrQuotient err = dp45_tail_f64(rhs, y, dl, k1, k2, k3, k4, y5, k7);
+                ++cnt.attempts;
+                const StepDecision d = pi_control_q(err, S.tol, dl, retry, y5.r);
+                if (!d.accept) {
+                    dl = d.next;
+                    ++retry;
+                } else {
+                    ++cnt.accepted;
+                    dlambda = d.next;
+                    ++step;  // the reference's loop counter advances on every outer iteration
+                    // hand-over to the ray-march (src/geodesic_tracer.cpp:105-153)
+                    const bool opaque = (Tt[0] < 1e-6 && Tt[1] < 1e-6 && Tt[2] < 1e-6);
+                    const bool may = vol_may_enter(V, y.r, y5.r);
+                    VolGeo g5{};
+                    if (may) g5 = vol_geo(V, y5.r, y5.th);
+                    if (!opaque && may && vol_enters(V, y, geo, y5, g5)) {
+                        marching = true;  // from the pre-step state
+                        ++entries;
+                        dl = vol_march_start(V, y.r, geo, been_inside);
+                        mcount = 0;
+                    } else {
+                        // the next outer step starts now, or when the march ends
+                        y = y5;
+                        k1 = k7;
+                        geo = g5;
+                        geo_ok = may;
+                        need_start = true;
+                    }
                 }
-                // the next outer step starts now, or when the march ends
-                if (!marching) need_start = true;
-            }
-        } else if (live && term < 0 && marching) {
-            // ---- one RK4 march step ----
-            bool end = vol_march_rgb_step(S, pt, pph, ms, ds, been_inside, J, Tt, cnt);
-            ++mcount;
-            if (!end && mcount >= 4096) end = true;
-            if (end) {
-                marching = false;
-                y = ms;  // the outer loop continues from the march's end state
+            } else {
+                // ---- the end of the RK4 march step ----
+                y = rk4_end_f64(y, dl, k1, k2, k3, k4);
+                geo = vol_geo(V, y.r, y.th);
                 k1_ok = false;
-                need_start = true;
+                const bool end = vol_march_rgb(S, pt, pph, y, geo, dl, been_inside, J, Tt, cnt);
+                ++mcount;
+                if (end || mcount >= 4096) {
+                    marching = false;  // the outer loop continues from the march's end state
+                    geo_ok = true;
+                    need_start = true;
+                }
             }
         }
 
-        // ---- finish a terminated sample ----
-        if (live && term >= 0) {
+        // ---- finish the terminated samples ----
+        const bool finish = live && term >= 0;
+        if (__any_sync(kFullMask, finish)) refill = true;
+        if (finish) {
             live = false;
             if (!kList) {
                 ++cnt.rays;
@@ -237,8 +258,8 @@ vol_render_kernel(const __grid_constant__ DevScene S, const DevTile tile, float4
                 break;
             }
         }
-        if (!__any_sync(kFullMask, live || pix >= -1)) break;
     }
+    cnt.fp64 = cnt.attempts;
     flush_vol(stats, cnt, cancelled);
 }
 

@@ -15,6 +15,14 @@
 // and sample finishes (reset of the ray's row, the J nu^3 sum and the
 // coalesced store of a pixel's spectrum) are served the same way.
 //
+// What bounds the launch is its longest rays: near the photon orbit a ray
+// alternates an outer step with a march of one step thousands of times, a
+// serial chain. So a step keeps what the next one needs (the first stage and
+// the geometry of its state), both kinds of step share the right-hand sides of
+// stages 2 to 4 (a warp holds both), and an iteration takes two votes unless a
+// sample ended (Kerr a=0.9, 512x512, 32 bins on B200: 62 -> 37 ms for the FP64
+// form; 101x75, 16 bins, mixed: 28 -> 14.4 ms).
+//
 // A ray's transfer state is a row of 4 x nb doubles per lane slot
 // [J | T | tau | pixel sum], so the warp's accesses to one row are
 // contiguous. Every bin sees the plain kernel's arithmetic in the same order,
@@ -26,11 +34,6 @@
 // so the FP64 form would give them zero intensity and the same termination.
 // The rest are listed and re-traced from the camera by the FP64 kernel; a
 // resolve pass sums each pixel's samples in order.
-// The volumetric kernels end on a few long rays, one warp per SM, where
-// instruction fetch stalls as much as arithmetic: one shared body of the FP64
-// right-hand side instead of twelve inlined copies (Kerr a=0.9, 512x512, 32
-// bins: 82 -> 74-79 ms for the FP64 form on B200).
-#define GRRT_RHS_CALL_F64 1
 #include <cuda_runtime.h>
 
 #include <cstdint>
@@ -96,91 +99,94 @@ vol_spectral_kernel(const __grid_constant__ DevScene S0, const DevTile tile, con
     VolCounters cnt;
     int pix = -1, smp = 0;  // kList: pix = the listed sample
     bool live = false, need_start = false, marching = false;
-    Vec5<double> y{}, prev{};
+    // the outer loop's state, or the march's (which starts from the state
+    // before the step that handed over)
+    Vec5<double> y{};
     Vec5<double> k1{};  // f(y) while k1_ok: the last accepted attempt's k7 or this step's first stage
     bool k1_ok = false;
-    double pt = 0.0, pph = 0.0, dl = 0.0, dlambda = 0.0;
-    int retry = 0, step = 0, entries = 0, n_thick = 0;
-    Vec5<double> ms{};
-    double ds = 0.0;
-    int mcount = 0;
+    VolGeo geo{};       // the geometry of y while geo_ok
+    bool geo_ok = false;
+    double pt = 0.0, pph = 0.0, dl = 0.0, dlambda = 0.0;  // dl: trial step, or the march's step
+    int retry = 0, step = 0, entries = 0, n_thick = 0, mcount = 0;
     bool been_inside = false, cancelled = false;
     unsigned iter = 0;
+    bool refill = true;  // warp-uniform: some lane has no ray
 
     while (true) {
-        // ---- refill ----
-        const bool want = (pix == -1);
-        const unsigned want_mask = __ballot_sync(kWarp, want);
-        bool fresh_pixel = false;
-        if (want_mask) {
-            unsigned base = 0;
-            const int leader = __ffs(want_mask) - 1;
-            if (lane == leader) base = atomicAdd(queue, static_cast<unsigned>(__popc(want_mask)));
-            base = __shfl_sync(kWarp, base, leader);
-            if (want) {
-                const unsigned k = base + __popc(want_mask & lt_mask);
-                if (k < total) {
-                    if (kBatch) {
-                        const DevBatchChunk ch = B.chunks[k / B.chunk_size];
-                        const int within = static_cast<int>(k % B.chunk_size);
-                        if (within < ch.count) {
-                            item = ch.item;
-                            const DevBatchItem& it = B.items[item];
-                            sp = B.scenes + it.scene;
-                            nb = it.nb;
-                            freqs = it.freqs;
-                            pix = ch.start + within;
+        if (refill) {
+            // ---- work items for the lanes without one ----
+            const bool want = (pix == -1);
+            const unsigned want_mask = __ballot_sync(kWarp, want);
+            bool fresh_pixel = false;
+            if (want_mask) {
+                unsigned base = 0;
+                const int leader = __ffs(want_mask) - 1;
+                if (lane == leader) base = atomicAdd(queue, static_cast<unsigned>(__popc(want_mask)));
+                base = __shfl_sync(kWarp, base, leader);
+                if (want) {
+                    const unsigned k = base + __popc(want_mask & lt_mask);
+                    if (k < total) {
+                        if (kBatch) {
+                            const DevBatchChunk ch = B.chunks[k / B.chunk_size];
+                            const int within = static_cast<int>(k % B.chunk_size);
+                            if (within < ch.count) {
+                                item = ch.item;
+                                const DevBatchItem& it = B.items[item];
+                                sp = B.scenes + it.scene;
+                                nb = it.nb;
+                                freqs = it.freqs;
+                                pix = ch.start + within;
+                                smp = 0;
+                                fresh_pixel = true;
+                            }  // else: padding slot of a short chunk, fetch again
+                        } else {
+                            // list: the listed samples (kList), or the pixel order;
+                            // taken in the spread order (vol_spread_order)
+                            const unsigned ks = vol_spread_order(k, total);
+                            pix = static_cast<int>(list ? list[ks] : ks);
                             smp = 0;
                             fresh_pixel = true;
-                        }  // else: padding slot of a short chunk, fetch again
+                        }
                     } else {
-                        // list: the listed samples (kList), or the pixel order;
-                        // taken in the spread order (vol_spread_order)
-                        const unsigned ks = vol_spread_order(k, total);
-                        pix = static_cast<int>(list ? list[ks] : ks);
-                        smp = 0;
-                        fresh_pixel = true;
+                        pix = -2;
                     }
-                } else {
-                    pix = -2;
                 }
             }
-        }
-        bool fresh_ray = false;
-        if (!live && pix >= 0) {
-            const int grid2 = S.grid * S.grid;
-            const int pixel = kList ? pix / grid2 : pix;
-            const int s = kList ? pix % grid2 : smp;
-            int i, j;
-            if (kBatch) {
-                const DevBatchItem& it = B.items[item];
-                i = it.x0 + pixel % it.w;
-                j = it.y0 + pixel / it.w;
-            } else {
-                const int qx = pixel % tile.w, qy = pixel / tile.w;
-                i = tile.x0 + qx;
-                j = tile.y0 + qy * tile.row_step;
+            bool fresh_ray = false;
+            if (!live && pix >= 0) {
+                const int grid2 = S.grid * S.grid;
+                const int pixel = kList ? pix / grid2 : pix;
+                const int s = kList ? pix % grid2 : smp;
+                int i, j;
+                if (kBatch) {
+                    const DevBatchItem& it = B.items[item];
+                    i = it.x0 + pixel % it.w;
+                    j = it.y0 + pixel / it.w;
+                } else {
+                    const int qx = pixel % tile.w, qy = pixel / tile.w;
+                    i = tile.x0 + qx;
+                    j = tile.y0 + qy * tile.row_step;
+                }
+                const int sy = s / S.grid, sx = s % S.grid;
+                const double x = i + (sx + pixel_hash(i, j, s, 0)) * S.cell;
+                const double yy = j + (sy + pixel_hash(i, j, s, 1)) * S.cell;
+                double p[4];
+                camera_momentum(S, x, yy, p);
+                y = Vec5<double>{S.cam_pos[1], S.cam_pos[2], S.cam_pos[3], p[1], p[2]};
+                pt = p[0];
+                pph = p[3];
+                dlambda = S.dl0;
+                step = 0;
+                entries = 0;
+                marching = false;
+                n_thick = 0;
+                k1_ok = false;
+                geo_ok = false;
+                live = true;
+                need_start = true;
+                fresh_ray = true;
             }
-            const int sy = s / S.grid, sx = s % S.grid;
-            const double x = i + (sx + pixel_hash(i, j, s, 0)) * S.cell;
-            const double yy = j + (sy + pixel_hash(i, j, s, 1)) * S.cell;
-            double p[4];
-            camera_momentum(S, x, yy, p);
-            y = Vec5<double>{S.cam_pos[1], S.cam_pos[2], S.cam_pos[3], p[1], p[2]};
-            pt = p[0];
-            pph = p[3];
-            dlambda = S.dl0;
-            step = 0;
-            entries = 0;
-            marching = false;
-            n_thick = 0;
-            k1_ok = false;
-            live = true;
-            need_start = true;
-            fresh_ray = true;
-        }
-        // ---- reset the new rays' rows (J = 0, T = 1, tau = 0; a new pixel's sum = 0) ----
-        {
+            // ---- reset the new rays' rows (J = 0, T = 1, tau = 0; a new pixel's sum = 0) ----
             const unsigned rm = __ballot_sync(kWarp, fresh_ray);
             const unsigned pm = __ballot_sync(kWarp, fresh_pixel);
             for (unsigned m = rm; m; m &= m - 1) {
@@ -195,102 +201,114 @@ vol_spectral_kernel(const __grid_constant__ DevScene S0, const DevTile tile, con
                     if (new_pixel) row[3 * seg + b] = 0.0;
                 }
             }
+            if (!__any_sync(kWarp, live || pix >= -1)) break;
+            refill = __any_sync(kWarp, pix == -1);
         }
 
+        // ---- start of an outer step: termination tests ----
         int term = -1;
-        // ---- start of an outer step: termination tests, then the near-disk clamp ----
         if (live && need_start) {
             if (step >= S.max_steps) term = kTermMaxSteps;
             else if (y.r < S.r_stop) term = kTermHorizon;
             else if (y.r > S.r_escape) term = kTermEscaped;
-            if (term < 0) {
-                if (!k1_ok) {
-                    k1 = kerr_rhs<double>(S.M, S.a, pt, pph, y);
-                    k1_ok = true;
-                }
-                if (vol_clamp(S, k1, y, dlambda)) ++cnt.clamp;
-                prev = y;
-                dl = dlambda;
-                retry = 0;
-                need_start = false;
-            }
         }
+        auto rhs = [&](const Vec5<double>& s) {
+            return kerr_rhs_f64(KerrHole{S.M, S.a, S.a2, S.m2}, pt, pph, s.r, s.th, s.pr, s.pth);
+        };
 
         // physics step inputs handed to the warp (bin-independent)
         bool phys = false;
         double ph_ag = 0.0, ph_rho = 0.0, ph_T = 0.0, ph_dsp = 0.0, ph_ke = 0.0, ph_fr = 0.0, ph_fT = 0.0;
-        double ph_r = 0.0, ph_H = 0.0, ph_kamed = 0.0;
+        double ph_kamed = 0.0;
         int ph_ir = 0, ph_iT = 0;
-        bool marched = false, mend = false;
-        Vec5<double> ns{};
-        if (live && term < 0 && !marching) {
-            // ---- one DP45 attempt ----
-            Vec5<double> y5, k7;
-            const double err = dp45_attempt_k1<double>(S.M, S.a, pt, pph, y, dl, k1, y5, k7);
-            ++cnt.fp64;
-            ++cnt.attempts;
-            const StepDecision d = pi_control(err, S.tol, dl, retry, y5.r);
-            if (!d.accept) {
-                dl = d.next;
-                ++retry;
-            } else {
-                ++cnt.accepted;
-                y = y5;
-                k1 = k7;
-                dlambda = d.next;
-                ++step;  // the reference's loop counter advances on every outer iteration
-                // hand-over to the ray-march (src/geodesic_tracer.cpp:105-153)
-                if (vol_enters(V, prev, y)) {
-                    marching = true;
-                    ++entries;
-                    ms = prev;  // march from the pre-step state
-                    ds = vol_march_start(V, ms, been_inside);
-                    mcount = 0;
-                }
-                if (!marching) need_start = true;
+        bool mend = false;
+        const bool marched = marching;  // this iteration's step is a march step
+        if (live && term < 0) {
+            // ---- first stage, where the last step did not leave it (a march's first step
+            //      takes the outer step's) ----
+            if (!k1_ok) {
+                k1 = rhs(y);
+                k1_ok = true;
             }
-        } else if (live && term < 0 && marching) {
-            // ---- one RK4 march step (geometry; the bins follow below) ----
-            marched = true;
-            ns = rk4_step<double>(S.M, S.a, pt, pph, ms, ds);
-            ++mcount;
-            ++cnt.march;
-            const double r = ns.r, theta = ns.th;
-            double st, ct;
-            sincos(theta, &st, &ct);
-            const double z = r * ct;
-            if (r < V.r_horizon || r > V.r_outer) {
-                mend = true;
-            } else if (n_thick == nb) {
-                mend = true;
+            // ---- near-disk clamp of a new outer step ----
+            if (need_start) {
+                if (vol_near_radius(V, y.r)) {
+                    if (!geo_ok) geo = vol_geo(V, y.r, y.th);
+                    geo_ok = true;
+                    if (vol_clamp(k1, y.r, geo, dlambda)) ++cnt.clamp;
+                }
+                dl = dlambda;
+                retry = 0;
+                need_start = false;
+            }
+            Vec5<double> k2, k3, k4;
+            shared_stages_f64(rhs, marching, y, dl, k1, k2, k3, k4);
+            if (!marching) {
+                // ---- the rest of the DP45 attempt ----
+                Vec5<double> y5, k7;
+                const ErrQuotient err = dp45_tail_f64(rhs, y, dl, k1, k2, k3, k4, y5, k7);
+                ++cnt.attempts;
+                const StepDecision d = pi_control_q(err, S.tol, dl, retry, y5.r);
+                if (!d.accept) {
+                    dl = d.next;
+                    ++retry;
+                } else {
+                    ++cnt.accepted;
+                    dlambda = d.next;
+                    ++step;  // the reference's loop counter advances on every outer iteration
+                    // hand-over to the ray-march (src/geodesic_tracer.cpp:105-153)
+                    const bool may = vol_may_enter(V, y.r, y5.r);
+                    VolGeo g5{};
+                    if (may) g5 = vol_geo(V, y5.r, y5.th);
+                    if (may && vol_enters(V, y, geo, y5, g5)) {
+                        marching = true;  // from the pre-step state
+                        ++entries;
+                        dl = vol_march_start(V, y.r, geo, been_inside);
+                        mcount = 0;
+                    } else {
+                        y = y5;
+                        k1 = k7;
+                        geo = g5;
+                        geo_ok = may;
+                        need_start = true;
+                    }
+                }
             } else {
-                const double H = v_scale_height(V, r);
-                if (!v_inside(V, r, z)) {
-                    const double zm = v_zmax(V, r);
-                    if (been_inside && fabs(z) > zm + 3.0 * H) {
+                // ---- the end of the RK4 march step (geometry; the bins follow below) ----
+                y = rk4_end_f64(y, dl, k1, k2, k3, k4);
+                geo = vol_geo(V, y.r, y.th);
+                k1_ok = false;
+                ++mcount;
+                ++cnt.march;
+                const double r = y.r;
+                if (r < V.r_horizon || r > V.r_outer) {
+                    mend = true;
+                } else if (n_thick == nb) {
+                    mend = true;
+                } else if (!geo_inside(V, r, geo)) {
+                    const double H = geo.H;
+                    if (been_inside && fabs(geo.z) > __fma_rn(3.0, H, geo.zm)) {
                         mend = true;
                     } else if (!been_inside) {
-                        ds = vmax(vmin(fabs(z) / 8.0, H * 2.0), H / 64.0);
+                        dl = vmax(vmin(fabs(geo.z) / 8.0, H * 2.0), H / 64.0);
                     } else {
-                        ds = vclamp(H / 4.0, H / 64.0, H);
+                        dl = vclamp(H / 4.0, H / 64.0, H);
                     }
                 } else {
                     been_inside = true;
-                    const double rho = v_density(V, V.perm, r, z, ns.ph);
-                    const double Tl = v_temperature(V, r, fabs(z));
+                    const double rho = v_density(V, V.perm, r, geo.z, y.ph);
+                    const double Tl = v_temperature(V, r, fabs(geo.z));
                     if (rho > 0.0 && Tl > 0.0) {
                         ++cnt.physics;
                         double g, pue;
-                        v_redshift(V, pt, ns.pr, pph, r, theta, g, pue);
-                        ph_dsp = fabs(pue) * fabs(ds);
+                        v_redshift(V, pt, y.pr, pph, r, y.th, g, pue);
+                        ph_dsp = fabs(pue) * fabs(dl);
                         log_locate(log10(rho), V.log_rho_min, V.log_rho_max, V.n_rho, ph_ir, ph_fr);
                         log_locate(log10(Tl), V.log_T_min, V.log_T_max, V.n_T, ph_iT, ph_fT);
                         ph_ke = v_kappa_es(V, ph_ir, ph_fr, ph_iT, ph_fT);
                         ph_ag = fabs(g);
                         ph_rho = rho;
                         ph_T = Tl;
-                        ph_r = r;
-                        ph_H = H;
                         phys = true;
                     }
                 }
@@ -351,57 +369,53 @@ vol_spectral_kernel(const __grid_constant__ DevScene S0, const DevTile tile, con
             }
         }
         if (phys) {
-            cnt.bins += static_cast<unsigned long long>(nb);
+            cnt.bins += static_cast<unsigned>(nb);
             const double at = (ph_kamed + ph_ke) * ph_rho;
-            const double ds_tau = (at > 0.0) ? 0.05 / at : ds * 2.0;
-            const double ds_geo = 0.1 * vmax(ph_r - V.r_horizon, 0.5);
-            ds = vclamp(vmin(ds_tau, ds_geo), ph_H / 64.0, ph_H);
+            const double ds_tau = (at > 0.0) ? 0.05 / at : dl * 2.0;
+            const double ds_geo = 0.1 * vmax(y.r - V.r_horizon, 0.5);
+            dl = vclamp(vmin(ds_tau, ds_geo), geo.H / 64.0, geo.H);
         }
-        if (marched) {
-            ms = ns;
-            if (!mend && mcount >= 4096) mend = true;
-            if (mend) {
-                marching = false;
-                y = ms;  // the outer loop continues from the march's end state
-                k1_ok = false;
-                need_start = true;
-            }
+        if (marched && (mend || mcount >= 4096)) {
+            marching = false;  // the outer loop continues from the march's end state
+            geo_ok = true;
+            need_start = true;
         }
 
-        // ---- finish a terminated sample ----
-        bool finish = false, pixel_done = false;
-        size_t out_elem = 0;  // first output element of the finished pixel (list: sample)
-        if (live && term >= 0) {
-            live = false;
-            finish = true;
-            ++cnt.rays;
-            if (term == kTermEscaped) ++cnt.escaped;
-            else if (term == kTermHorizon) ++cnt.horizon;
-            else ++cnt.maxsteps;
-            const int grid2 = S.grid * S.grid;
-            if (!kBatch && out_fate) {
-                const unsigned ne = (entries > 0x3fffffff) ? 0x3fffffffu : static_cast<unsigned>(entries);
-                const size_t q = kList ? static_cast<size_t>(pix) : static_cast<size_t>(pix) * grid2 + smp;
-                out_fate[q] = static_cast<unsigned>(term) | (ne << 2);
-            }
-            if (kList) {
-                out_elem = static_cast<size_t>(pix) * nb;
-                pixel_done = true;
-                pix = -1;
-            } else if (++smp == grid2) {
-                if (kBatch) {
-                    out_elem = B.items[item].spec_offset + static_cast<size_t>(pix) * nb;
-                } else {
-                    const int qx = pix % tile.w, qy = pix / tile.w;
-                    out_elem = (static_cast<size_t>(qy) * tile.out_pitch + qx) * nb;
+        // ---- finish the terminated samples ----
+        const bool finish = live && term >= 0;
+        const unsigned fm = __ballot_sync(kWarp, finish);
+        if (fm) {
+            bool pixel_done = false;
+            size_t out_elem = 0;  // first output element of the finished pixel (list: sample)
+            if (finish) {
+                live = false;
+                ++cnt.rays;
+                if (term == kTermEscaped) ++cnt.escaped;
+                else if (term == kTermHorizon) ++cnt.horizon;
+                else ++cnt.maxsteps;
+                const int grid2 = S.grid * S.grid;
+                if (!kBatch && out_fate) {
+                    const unsigned ne = (entries > 0x3fffffff) ? 0x3fffffffu : static_cast<unsigned>(entries);
+                    const size_t q = kList ? static_cast<size_t>(pix) : static_cast<size_t>(pix) * grid2 + smp;
+                    out_fate[q] = static_cast<unsigned>(term) | (ne << 2);
                 }
-                pixel_done = true;
-                pix = -1;
+                if (kList) {
+                    out_elem = static_cast<size_t>(pix) * nb;
+                    pixel_done = true;
+                    pix = -1;
+                } else if (++smp == grid2) {
+                    if (kBatch) {
+                        out_elem = B.items[item].spec_offset + static_cast<size_t>(pix) * nb;
+                    } else {
+                        const int qx = pix % tile.w, qy = pix / tile.w;
+                        out_elem = (static_cast<size_t>(qy) * tile.out_pitch + qx) * nb;
+                    }
+                    pixel_done = true;
+                    pix = -1;
+                }
             }
-        }
-        {
+            refill = true;
             // I nu^3 of the finished samples into the pixel sums; finished pixels stored
-            const unsigned fm = __ballot_sync(kWarp, finish);
             const unsigned dm = __ballot_sync(kWarp, pixel_done);
             // finished work items, for progress reports (the work counter
             // counts items taken; the long rays finish long after)
@@ -439,8 +453,8 @@ vol_spectral_kernel(const __grid_constant__ DevScene S0, const DevTile tile, con
                 break;
             }
         }
-        if (!__any_sync(kWarp, live || pix >= -1)) break;
     }
+    cnt.fp64 = cnt.attempts;
 #undef S
 #undef V
     flush_vol(stats, cnt, cancelled);

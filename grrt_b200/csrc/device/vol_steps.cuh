@@ -10,9 +10,10 @@
 
 namespace grrt_b200 {
 
-struct VolCounters {
-    unsigned long long attempts = 0, accepted = 0, rays = 0, horizon = 0, escaped = 0, maxsteps = 0;
-    unsigned long long clamp = 0, march = 0, physics = 0, bins = 0, fp64 = 0;
+struct VolCounters {  // one lane's counts: 32 bits hold hours of steps
+    unsigned attempts = 0, accepted = 0, rays = 0, horizon = 0, escaped = 0, maxsteps = 0;
+    unsigned clamp = 0, march = 0, physics = 0, fp64 = 0;
+    unsigned long long bins = 0;
 };
 
 // Order in which the spectral kernel takes its work items: within each full
@@ -65,60 +66,89 @@ __device__ __forceinline__ double add_intensity(double sum, double J, double f) 
     return __dadd_rn(sum, __dmul_rn(__dmul_rn(__dmul_rn(J, f), f), f));
 }
 
+// Where a state lies relative to the volume: the sine and cosine of its
+// colatitude, its height z, and the disk's scale height and photosphere height
+// at its radius. The clamp, the hand-over and the march's start need it of the
+// same two states of a step, so a trace keeps the one of its current state
+// instead of looking it up up to three times. The radial coordinate's quotient
+// is formed from the span's reciprocal and corrected by its exact residual (the
+// division's value), both tables share it, and the roundings are written out.
+struct VolGeo {
+    double st, ct, z, H, zm;
+};
+__device__ __forceinline__ VolGeo vol_geo(const DevVolume& V, double r, double th) {
+    VolGeo g;
+    sincos(th, &g.st, &g.ct);
+    g.z = __dmul_rn(r, g.ct);
+    if (r <= V.r_min || r >= V.r_outer) {
+        const int k = (r <= V.r_min) ? 0 : V.n_r - 1;
+        g.H = __ldg(V.H + k);
+        g.zm = __ldg(V.z_max + k);
+        return g;
+    }
+    const double num = __dadd_rn(r, -V.r_min);
+    const double q0 = __dmul_rn(num, V.inv_span);
+    const double q = __fma_rn(__fma_rn(-V.span, q0, num), V.inv_span, q0);
+    const double frac = __dmul_rn(q, static_cast<double>(V.n_r - 1));
+    const int idx = table_index(frac, 0, V.n_r - 2);
+    const double t = __dadd_rn(frac, -static_cast<double>(idx)), u = __dadd_rn(1.0, -t);
+    g.H = __fma_rn(__ldg(V.H + idx + 1), t, __dmul_rn(__ldg(V.H + idx), u));
+    g.zm = __fma_rn(__ldg(V.z_max + idx + 1), t, __dmul_rn(__ldg(V.z_max + idx), u));
+    return g;
+}
+
+// v_inside of a state whose geometry is known.
+__device__ __forceinline__ bool geo_inside(const DevVolume& V, double r, const VolGeo& g) {
+    return !(r <= V.r_horizon || r > V.r_outer) && fabs(g.z) < __fma_rn(1.5, g.H, g.zm);
+}
+
+// Radii whose outer steps the clamp and the hand-over look at.
+__device__ __forceinline__ bool vol_near_radius(const DevVolume& V, double r) {
+    return r >= V.r_horizon * 0.9 && r <= V.r_outer * 1.5;
+}
+
 // Near-disk clamp at the start of an outer step (src/geodesic_tracer.cpp:71-95):
-// for r in [0.9 r_h, 1.5 r_outer] and |z| < z_max + 6 H, dlambda is capped at
-// max(H / (4 |dz/dlambda|), H / 64). d = f(y), the right-hand side the step's
-// first DP45 stage uses too (the reference evaluates it here once more).
-// Returns whether the clamp applied (the clamp counter).
-__device__ __forceinline__ bool vol_clamp(const DevScene& S, const Vec5<double>& d, const Vec5<double>& y,
-                                          double& dlambda) {
-    const DevVolume& V = S.vol;
-    const double r = y.r;
-    if (!(r >= V.r_horizon * 0.9 && r <= V.r_outer * 1.5)) return false;
-    double st, ct;
-    sincos(y.th, &st, &ct);
-    const double z = r * ct;
-    const double H = v_scale_height(V, r);
-    const double zm = v_zmax(V, r);
-    if (!(fabs(z) < zm + 6.0 * H)) return false;
-    const double dz_dl = fabs(ct * d.r - r * st * d.th);
+// for r in [0.9 r_h, 1.5 r_outer] (vol_near_radius, the caller's test) and
+// |z| < z_max + 6 H, dlambda is capped at max(H / (4 |dz/dlambda|), H / 64).
+// d = f(y), the right-hand side the step's first DP45 stage uses too (the
+// reference evaluates it here once more); g = the geometry of y. Returns
+// whether the clamp applied (the clamp counter).
+__device__ __forceinline__ bool vol_clamp(const Vec5<double>& d, double r, const VolGeo& g, double& dlambda) {
+    if (!(fabs(g.z) < __fma_rn(6.0, g.H, g.zm))) return false;
+    const double dz_dl = fabs(__fma_rn(g.ct, d.r, -__dmul_rn(__dmul_rn(r, g.st), d.th)));
     if (dz_dl > 1e-20) {
-        const double dl_max = vmax(0.25 * H / dz_dl, H / 64.0);
+        const double dl_max = vmax(div_f64(0.25 * g.H, dz_dl), g.H * (1.0 / 64.0));
         dlambda = vmin(dlambda, dl_max);
     }
     return true;
 }
 
-// Hand-over after an accepted outer step prev -> y (src/geodesic_tracer.cpp:105-153):
-// the step crossed the equator, ends inside the volume, or either end is
-// within z_max + 2H of the plane over the disk's radii; and the step's radii
-// reach [r_h, r_outer] from a start inside [0.9 r_h, 1.5 r_outer]. The march
-// then starts from prev.
-__device__ __forceinline__ bool vol_enters(const DevVolume& V, const Vec5<double>& prev, const Vec5<double>& y) {
-    const double hp = kHalfPi;
-    const double d_prev = prev.th - hp, d_new = y.th - hp;
-    const double r_new = y.r, r_prev = prev.r;
-    const double z_new = r_new * cos(y.th);
-    const double z_prev = r_prev * cos(prev.th);
-    const bool crossed = (d_prev * d_new < 0.0) && fabs(d_prev - d_new) > 1e-12;
-    const bool inside_now = v_inside(V, r_new, z_new);
-    const double zm_new = v_zmax(V, r_new), H_new = v_scale_height(V, r_new);
-    const double H_prev = v_scale_height(V, r_prev);
-    const bool near = (fabs(z_new) < zm_new + 2.0 * H_new || fabs(z_prev) < v_zmax(V, r_prev) + 2.0 * H_prev) &&
-                      r_new >= V.r_horizon && r_new <= V.r_outer;
-    if (!(crossed || inside_now || near)) return false;
+// Whether an accepted outer step between these radii can hand over at all: its
+// radii reach [r_h, r_outer] from a start inside [0.9 r_h, 1.5 r_outer].
+__device__ __forceinline__ bool vol_may_enter(const DevVolume& V, double r_prev, double r_new) {
     const double r_lo = vmin(r_prev, r_new), r_hi = vmax(r_prev, r_new);
-    return r_hi >= V.r_horizon && r_lo <= V.r_outer && r_prev >= V.r_horizon * 0.9 && r_prev <= V.r_outer * 1.5;
+    return r_hi >= V.r_horizon && r_lo <= V.r_outer && vol_near_radius(V, r_prev);
 }
 
-// First march step length from the start state s: H/16 inside the volume,
-// else min(|z|/8, 2H).
-__device__ __forceinline__ double vol_march_start(const DevVolume& V, const Vec5<double>& s, bool& been_inside) {
-    const double r0 = s.r;
-    const double z0 = r0 * cos(s.th);
-    const double H0 = v_scale_height(V, r0);
-    been_inside = v_inside(V, r0, z0);
-    return been_inside ? H0 / 16.0 : vmin(fabs(z0) / 8.0, H0 * 2.0);
+// Hand-over after an accepted outer step prev -> y (src/geodesic_tracer.cpp:105-153)
+// that vol_may_enter: the step crossed the equator, ends inside the volume, or
+// either end is within z_max + 2H of the plane over the disk's radii. The march
+// then starts from prev. gp, g: the geometry of the two ends.
+__device__ __forceinline__ bool vol_enters(const DevVolume& V, const Vec5<double>& prev, const VolGeo& gp,
+                                           const Vec5<double>& y, const VolGeo& g) {
+    const double hp = kHalfPi;
+    const double d_prev = prev.th - hp, d_new = y.th - hp;
+    const bool crossed = (d_prev * d_new < 0.0) && fabs(d_prev - d_new) > 1e-12;
+    const bool near = (fabs(g.z) < __fma_rn(2.0, g.H, g.zm) || fabs(gp.z) < __fma_rn(2.0, gp.H, gp.zm)) &&
+                      y.r >= V.r_horizon && y.r <= V.r_outer;
+    return crossed || near || geo_inside(V, y.r, g);
+}
+
+// First march step length from the start state s of geometry g: H/16 inside
+// the volume, else min(|z|/8, 2H).
+__device__ __forceinline__ double vol_march_start(const DevVolume& V, double r, const VolGeo& g, bool& been_inside) {
+    been_inside = geo_inside(V, r, g);
+    return been_inside ? g.H / 16.0 : vmin(fabs(g.z) / 8.0, g.H * 2.0);
 }
 
 // Observer-frame RGB frequencies (450, 550, 650 nm) of the RGB transfer.
@@ -127,78 +157,62 @@ __device__ __forceinline__ double rgb_nu(int ch) {
     return ch == 0 ? c / 450e-7 : (ch == 1 ? c / 550e-7 : c / 650e-7);
 }
 
-// One RK4 step of the RGB ray-march (src/geodesic_tracer.cpp:183-337): ms
-// advances by ds; inside the volume the three channels' emission and
-// absorption update J and Tt and the next ds follows the optical depth and
-// the radius; outside it ds approaches the volume (never inside yet) or holds
-// at H/4 (after being inside). Returns whether the march ends here: outside
-// [r_h, r_outer], all channels opaque, or beyond z_max + 3H after being
-// inside. The 4096-step cap is the caller's.
-__device__ __forceinline__ bool vol_march_rgb_step(const DevScene& S, double pt, double pph, Vec5<double>& ms,
-                                                   double& ds, bool& been_inside, double* J, double* Tt,
-                                                   VolCounters& cnt) {
+// The RGB ray-march's work at a new state ns of geometry g, reached by a step
+// of length ds (src/geodesic_tracer.cpp:183-337): inside the volume the three
+// channels' emission and absorption update J and Tt and the next ds follows
+// the optical depth and the radius; outside it ds approaches the volume (never
+// inside yet) or holds at H/4 (after being inside). Returns whether the march
+// ends here: outside [r_h, r_outer], all channels opaque, or beyond z_max + 3H
+// after being inside. The 4096-step cap is the caller's.
+__device__ __forceinline__ bool vol_march_rgb(const DevScene& S, double pt, double pph, const Vec5<double>& ns,
+                                              const VolGeo& g, double& ds, bool& been_inside, double* J, double* Tt,
+                                              VolCounters& cnt) {
     const DevVolume& V = S.vol;
-    const Vec5<double> ns = rk4_step<double>(S.M, S.a, pt, pph, ms, ds);
     ++cnt.march;
     const double r = ns.r, theta = ns.th;
-    double st, ct;
-    sincos(theta, &st, &ct);
-    const double z = r * ct;
-    bool end = false;
-    if (r < V.r_horizon || r > V.r_outer) {
-        end = true;
-    } else if (Tt[0] < 1e-6 && Tt[1] < 1e-6 && Tt[2] < 1e-6) {
-        end = true;
-    } else {
-        const double H = v_scale_height(V, r);
-        if (!v_inside(V, r, z)) {
-            const double zm = v_zmax(V, r);
-            if (been_inside && fabs(z) > zm + 3.0 * H) {
-                end = true;
-            } else if (!been_inside) {
-                ds = vmax(vmin(fabs(z) / 8.0, H * 2.0), H / 64.0);
-            } else {
-                ds = vclamp(H / 4.0, H / 64.0, H);
-            }
-        } else {
-            been_inside = true;
-            const double rho = v_density(V, V.perm, r, z, ns.ph);
-            const double Tl = v_temperature(V, r, fabs(z));
-            if (rho > 0.0 && Tl > 0.0) {
-                ++cnt.physics;
-                double g, pue;
-                v_redshift(V, pt, ns.pr, pph, r, theta, g, pue);
-                const double dsp = fabs(pue) * fabs(ds);
-                int ir, iT;
-                double fr, fT;
-                log_locate(log10(rho), V.log_rho_min, V.log_rho_max, V.n_rho, ir, fr);
-                log_locate(log10(Tl), V.log_T_min, V.log_T_max, V.n_T, iT, fT);
-                const double ke = v_kappa_es(V, ir, fr, iT, fT);
-                const double ag = fabs(g);
-                double ka_med = 0.0;
-                for (int b = 0; b < 3; ++b) {
-                    const double nu = ag * rgb_nu(b);
-                    const double ka = v_kappa_abs(V, nu, ir, fr, iT, fT);
-                    if (b == 1) ka_med = ka;
-                    const double kt = ka + ke;
-                    const double eps = (kt > 0.0) ? ka / kt : 1.0;
-                    const double dtau = kt * rho * dsp;
-                    const double B = planck_nu(nu, Tl);
-                    const double Sv = eps * B / (nu * nu * nu);
-                    const double e = exp(-dtau);
-                    J[b] += Tt[b] * Sv * (1.0 - e);
-                    Tt[b] *= e;
-                }
-                cnt.bins += 3;
-                const double at = (ka_med + ke) * rho;
-                const double ds_tau = (at > 0.0) ? 0.05 / at : ds * 2.0;
-                const double ds_geo = 0.1 * vmax(r - V.r_horizon, 0.5);
-                ds = vclamp(vmin(ds_tau, ds_geo), H / 64.0, H);
-            }
-        }
+    const double z = g.z, H = g.H;
+    if (r < V.r_horizon || r > V.r_outer) return true;
+    if (Tt[0] < 1e-6 && Tt[1] < 1e-6 && Tt[2] < 1e-6) return true;
+    if (!geo_inside(V, r, g)) {
+        if (been_inside && fabs(z) > __fma_rn(3.0, H, g.zm)) return true;
+        ds = been_inside ? vclamp(H / 4.0, H / 64.0, H) : vmax(vmin(fabs(z) / 8.0, H * 2.0), H / 64.0);
+        return false;
     }
-    ms = ns;
-    return end;
+    been_inside = true;
+    const double rho = v_density(V, V.perm, r, z, ns.ph);
+    const double Tl = v_temperature(V, r, fabs(z));
+    if (rho > 0.0 && Tl > 0.0) {
+        ++cnt.physics;
+        double gs, pue;
+        v_redshift(V, pt, ns.pr, pph, r, theta, gs, pue);
+        const double dsp = fabs(pue) * fabs(ds);
+        int ir, iT;
+        double fr, fT;
+        log_locate(log10(rho), V.log_rho_min, V.log_rho_max, V.n_rho, ir, fr);
+        log_locate(log10(Tl), V.log_T_min, V.log_T_max, V.n_T, iT, fT);
+        const double ke = v_kappa_es(V, ir, fr, iT, fT);
+        const double ag = fabs(gs);
+        double ka_med = 0.0;
+        for (int b = 0; b < 3; ++b) {
+            const double nu = ag * rgb_nu(b);
+            const double ka = v_kappa_abs(V, nu, ir, fr, iT, fT);
+            if (b == 1) ka_med = ka;
+            const double kt = ka + ke;
+            const double eps = (kt > 0.0) ? ka / kt : 1.0;
+            const double dtau = kt * rho * dsp;
+            const double B = planck_nu(nu, Tl);
+            const double Sv = eps * B / (nu * nu * nu);
+            const double e = exp(-dtau);
+            J[b] += Tt[b] * Sv * (1.0 - e);
+            Tt[b] *= e;
+        }
+        cnt.bins += 3;
+        const double at = (ka_med + ke) * rho;
+        const double ds_tau = (at > 0.0) ? 0.05 / at : ds * 2.0;
+        const double ds_geo = 0.1 * vmax(r - V.r_horizon, 0.5);
+        ds = vclamp(vmin(ds_tau, ds_geo), H / 64.0, H);
+    }
+    return false;
 }
 
 }  // namespace grrt_b200
