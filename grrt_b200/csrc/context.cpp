@@ -173,10 +173,13 @@ bool GRRTContext::ensure_device() {
         o_cs = ab.add(stars.cell_start);
         o_ci = ab.add(stars.cell_items);
     }
-    size_t o_H = 0, o_zm = 0, o_rm = 0, o_rp = 0, o_tp = 0, o_perm = 0, o_lk = 0, o_kes = 0;
+    size_t o_H = 0, o_zm = 0, o_izm = 0, o_rm = 0, o_rp = 0, o_tp = 0, o_perm = 0, o_lk = 0, o_kes = 0;
     if (vol) {
         o_H = ab.add(vol->H);
         o_zm = ab.add(vol->z_max);
+        std::vector<double> inv_z_max(vol->z_max.size());
+        for (size_t i = 0; i < inv_z_max.size(); ++i) inv_z_max[i] = 1.0 / vol->z_max[i];
+        o_izm = ab.add(inv_z_max);
         o_rm = ab.add(vol->rho_mid);
         o_rp = ab.add(vol->rho_profile);
         o_tp = ab.add(vol->T_profile);
@@ -247,19 +250,23 @@ bool GRRTContext::ensure_device() {
         V.r_outer = vol->r_outer;
         V.span = V.r_outer - V.r_min;
         V.inv_span = 1.0 / V.span;
+        V.sqrt_M = std::sqrt(V.M);
         V.r_isco = vol->r_isco;
         V.r_horizon = vol->r_horizon;
-        V.taper_width = vol->taper_width;
+        V.taper_w2 = vol->taper_width * vol->taper_width;
+        V.inv_taper_w2 = 1.0 / V.taper_w2;
         V.E_isco = vol->E_isco;
         V.L_isco = vol->L_isco;
         V.rho_scale = vol->rho_scale;
         V.noise_scale = vol->noise_scale;
+        V.inv_noise = 1.0 / V.noise_scale;
         V.turbulence = vol->cfg.turbulence;
         V.octaves = vol->cfg.noise_octaves;
         V.n_r = vol->n_r;
         V.n_z = vol->n_z;
         V.H = reinterpret_cast<const double*>(at(o_H));
         V.z_max = reinterpret_cast<const double*>(at(o_zm));
+        V.inv_z_max = reinterpret_cast<const double*>(at(o_izm));
         V.rho_mid = reinterpret_cast<const double*>(at(o_rm));
         V.rho_prof = reinterpret_cast<const double*>(at(o_rp));
         V.T_prof = reinterpret_cast<const double*>(at(o_tp));
@@ -274,6 +281,12 @@ bool GRRTContext::ensure_device() {
         V.log_rho_max = op.log_rho_max;
         V.log_T_min = op.log_T_min;
         V.log_T_max = op.log_T_max;
+        V.len_nu = op.log_nu_max - op.log_nu_min;
+        V.len_rho = op.log_rho_max - op.log_rho_min;
+        V.len_T = op.log_T_max - op.log_T_min;
+        V.inv_len_nu = 1.0 / V.len_nu;
+        V.inv_len_rho = 1.0 / V.len_rho;
+        V.inv_len_T = 1.0 / V.len_T;
         V.ln_kabs = reinterpret_cast<const double*>(at(o_lk));
         V.kes = reinterpret_cast<const double*>(at(o_kes));
         V.ut_obs = 1.0 / std::sqrt(1.0 - 2.0 / observer_r);

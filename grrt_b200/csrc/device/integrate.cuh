@@ -47,16 +47,21 @@ static __constant__ DpConst kDp = {dp::a21, dp::a31, dp::a32, dp::a41, dp::a42, 
                                    dp::a54, dp::a61, dp::a62, dp::a63, dp::a64, dp::a65, dp::b1, dp::b3, dp::b4,
                                    dp::b5, dp::b6, dp::e1, dp::e3, dp::e4, dp::e5, dp::e6, dp::e7, 1e-10};
 
-// n / d, correctly rounded: the quotient from the reciprocal, corrected by its
-// exact residual (Markstein, as recip_f64) where both and the result are far
-// from the range's ends, the division operator elsewhere.
+// n / d, correctly rounded, from inv = the rounded 1 / d: the quotient
+// corrected by its exact residual (Markstein, as recip_f64). For numbers far
+// from the range's ends.
+__device__ __forceinline__ double div_by(double n, double d, double inv) {
+    const double q = __dmul_rn(n, inv);
+    return __fma_rn(__fma_rn(-d, q, n), inv, q);
+}
+
+// n / d, correctly rounded: by the reciprocal for 2^-450 <= |n|, |d| < 2^450
+// or n = 0, by the division operator elsewhere.
 __device__ __forceinline__ double div_f64(double n, double d) {
     const int hn = __double2hiint(n) & 0x7fffffff, hd = __double2hiint(d) & 0x7fffffff;
-    // 2^-450 <= |n|, |d| < 2^450
-    if (static_cast<unsigned>(hn - 0x23d00000) >= 0x38400000u || static_cast<unsigned>(hd - 0x23d00000) >= 0x38400000u)
-        return n / d;
-    const double r = recip_f64(d), q = __dmul_rn(n, r);
-    return __fma_rn(__fma_rn(-d, q, n), r, q);
+    const bool n_ok = static_cast<unsigned>(hn - 0x23d00000) < 0x38400000u || (hn | __double2loint(n)) == 0;
+    if (!n_ok || static_cast<unsigned>(hd - 0x23d00000) >= 0x38400000u) return n / d;
+    return div_by(n, d, recip_f64(d));
 }
 
 // One DP45 attempt on the device (dp45_attempt_k1 below), roundings written out

@@ -25,13 +25,17 @@ struct DevStars {
 
 struct DevVolume {
     double M = 1, a = 0;  // the disk's own mass and spin (raw create parameters)
-    double r_min = 0, r_outer = 0, r_isco = 0, r_horizon = 0, taper_width = 0;
+    double r_min = 0, r_outer = 0, r_isco = 0, r_horizon = 0;
     double E_isco = 0, L_isco = 0, rho_scale = 1, noise_scale = 1, turbulence = 0;
-    double inv_taper_w2 = 0;
-    double span = 1, inv_span = 1;    // r_outer - r_min and 1 / span, for the radial tables' coordinate
+    // divisors the kernels meet at every step, and their reciprocals (div_by):
+    // r_outer - r_min, the noise scale, the taper width squared, the tables' axis lengths
+    double span = 1, inv_span = 1, inv_noise = 1, taper_w2 = 1, inv_taper_w2 = 1;
+    double len_nu = 1, inv_len_nu = 1, len_rho = 1, inv_len_rho = 1, len_T = 1, inv_len_T = 1;
+    double sqrt_M = 1;
     int octaves = 2, n_r = 500, n_z = 128;
     const double* H = nullptr;        // n_r
     const double* z_max = nullptr;    // n_r
+    const double* inv_z_max = nullptr; // 1 / z_max, n_r
     const double* rho_mid = nullptr;  // n_r
     const double* rho_prof = nullptr; // n_r*n_z
     const double* T_prof = nullptr;   // n_r*n_z

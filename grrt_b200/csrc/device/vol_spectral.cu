@@ -296,15 +296,15 @@ vol_spectral_kernel(const __grid_constant__ DevScene S0, const DevTile tile, con
                     }
                 } else {
                     been_inside = true;
-                    const double rho = v_density(V, V.perm, r, geo.z, y.ph);
-                    const double Tl = v_temperature(V, r, fabs(geo.z));
+                    double rho, Tl;
+                    v_density_temperature(V, V.perm, r, geo.z, y.ph, geo.H, geo.zm, rho, Tl);
                     if (rho > 0.0 && Tl > 0.0) {
                         ++cnt.physics;
                         double g, pue;
-                        v_redshift(V, pt, y.pr, pph, r, y.th, g, pue);
+                        v_redshift(V, pt, y.pr, pph, r, geo.ct, g, pue);
                         ph_dsp = fabs(pue) * fabs(dl);
-                        log_locate(log10(rho), V.log_rho_min, V.log_rho_max, V.n_rho, ph_ir, ph_fr);
-                        log_locate(log10(Tl), V.log_T_min, V.log_T_max, V.n_T, ph_iT, ph_fT);
+                        log_locate(log10(rho), V.log_rho_min, V.len_rho, V.inv_len_rho, V.n_rho, ph_ir, ph_fr);
+                        log_locate(log10(Tl), V.log_T_min, V.len_T, V.inv_len_T, V.n_T, ph_iT, ph_fT);
                         ph_ke = v_kappa_es(V, ph_ir, ph_fr, ph_iT, ph_fT);
                         ph_ag = fabs(g);
                         ph_rho = rho;
@@ -343,21 +343,15 @@ vol_spectral_kernel(const __grid_constant__ DevScene S0, const DevTile tile, con
                     double ka = 0.0;
                     bool thk = false;
                     if (b < snb) {
-                        const double nu = ag * __ldg(sfreqs + b);
-                        ka = v_kappa_abs(Vs, nu, ir, fr, iT, fT);
-                        const double kt = ka + ke;
-                        const double eps = (kt > 0.0) ? ka / kt : 1.0;
-                        const double dtau = kt * rho * dsp;
-                        const double B_nu = planck_nu(nu, Tl);
-                        const double Sv = eps * B_nu / (nu * nu * nu);
-                        const double e = exp(-dtau);
-                        double tau = row[2 * seg + b];
-                        tau += dtau;
+                        const BinStep st =
+                            v_bin_step(Vs, ag * __ldg(sfreqs + b), Tl, rho, dsp, ke, ir, fr, iT, fT);
+                        ka = st.ka;
+                        const double tau = __dadd_rn(row[2 * seg + b], st.dtau);
                         row[2 * seg + b] = tau;
                         thk = !(tau <= 10.0);
                         const double Tb = row[seg + b];
-                        row[b] += Tb * Sv * (1.0 - e);
-                        row[seg + b] = Tb * e;
+                        row[b] = __fma_rn(__dmul_rn(Tb, st.src), __dadd_rn(1.0, -st.e), row[b]);
+                        row[seg + b] = __dmul_rn(Tb, st.e);
                     }
                     thick += __popc(__ballot_sync(kWarp, thk));
                     if (smed >= b0 && smed < b0 + 32) kam = __shfl_sync(kWarp, ka, smed - b0);
@@ -371,7 +365,7 @@ vol_spectral_kernel(const __grid_constant__ DevScene S0, const DevTile tile, con
         if (phys) {
             cnt.bins += static_cast<unsigned>(nb);
             const double at = (ph_kamed + ph_ke) * ph_rho;
-            const double ds_tau = (at > 0.0) ? 0.05 / at : dl * 2.0;
+            const double ds_tau = (at > 0.0) ? div_f64(0.05, at) : dl * 2.0;
             const double ds_geo = 0.1 * vmax(y.r - V.r_horizon, 0.5);
             dl = vclamp(vmin(ds_tau, ds_geo), geo.H / 64.0, geo.H);
         }

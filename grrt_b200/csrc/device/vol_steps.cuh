@@ -70,9 +70,7 @@ __device__ __forceinline__ double add_intensity(double sum, double J, double f) 
 // colatitude, its height z, and the disk's scale height and photosphere height
 // at its radius. The clamp, the hand-over and the march's start need it of the
 // same two states of a step, so a trace keeps the one of its current state
-// instead of looking it up up to three times. The radial coordinate's quotient
-// is formed from the span's reciprocal and corrected by its exact residual (the
-// division's value), both tables share it, and the roundings are written out.
+// instead of looking it up up to three times.
 struct VolGeo {
     double st, ct, z, H, zm;
 };
@@ -80,20 +78,9 @@ __device__ __forceinline__ VolGeo vol_geo(const DevVolume& V, double r, double t
     VolGeo g;
     sincos(th, &g.st, &g.ct);
     g.z = __dmul_rn(r, g.ct);
-    if (r <= V.r_min || r >= V.r_outer) {
-        const int k = (r <= V.r_min) ? 0 : V.n_r - 1;
-        g.H = __ldg(V.H + k);
-        g.zm = __ldg(V.z_max + k);
-        return g;
-    }
-    const double num = __dadd_rn(r, -V.r_min);
-    const double q0 = __dmul_rn(num, V.inv_span);
-    const double q = __fma_rn(__fma_rn(-V.span, q0, num), V.inv_span, q0);
-    const double frac = __dmul_rn(q, static_cast<double>(V.n_r - 1));
-    const int idx = table_index(frac, 0, V.n_r - 2);
-    const double t = __dadd_rn(frac, -static_cast<double>(idx)), u = __dadd_rn(1.0, -t);
-    g.H = __fma_rn(__ldg(V.H + idx + 1), t, __dmul_rn(__ldg(V.H + idx), u));
-    g.zm = __fma_rn(__ldg(V.z_max + idx + 1), t, __dmul_rn(__ldg(V.z_max + idx), u));
+    const VolCell c = v_cell(V, r);
+    g.H = v_radial(V.H, c);
+    g.zm = v_radial(V.z_max, c);
     return g;
 }
 
@@ -169,7 +156,7 @@ __device__ __forceinline__ bool vol_march_rgb(const DevScene& S, double pt, doub
                                               VolCounters& cnt) {
     const DevVolume& V = S.vol;
     ++cnt.march;
-    const double r = ns.r, theta = ns.th;
+    const double r = ns.r;
     const double z = g.z, H = g.H;
     if (r < V.r_horizon || r > V.r_outer) return true;
     if (Tt[0] < 1e-6 && Tt[1] < 1e-6 && Tt[2] < 1e-6) return true;
@@ -179,36 +166,30 @@ __device__ __forceinline__ bool vol_march_rgb(const DevScene& S, double pt, doub
         return false;
     }
     been_inside = true;
-    const double rho = v_density(V, V.perm, r, z, ns.ph);
-    const double Tl = v_temperature(V, r, fabs(z));
+    double rho, Tl;
+    v_density_temperature(V, V.perm, r, z, ns.ph, H, g.zm, rho, Tl);
     if (rho > 0.0 && Tl > 0.0) {
         ++cnt.physics;
         double gs, pue;
-        v_redshift(V, pt, ns.pr, pph, r, theta, gs, pue);
+        v_redshift(V, pt, ns.pr, pph, r, g.ct, gs, pue);
         const double dsp = fabs(pue) * fabs(ds);
         int ir, iT;
         double fr, fT;
-        log_locate(log10(rho), V.log_rho_min, V.log_rho_max, V.n_rho, ir, fr);
-        log_locate(log10(Tl), V.log_T_min, V.log_T_max, V.n_T, iT, fT);
+        log_locate(log10(rho), V.log_rho_min, V.len_rho, V.inv_len_rho, V.n_rho, ir, fr);
+        log_locate(log10(Tl), V.log_T_min, V.len_T, V.inv_len_T, V.n_T, iT, fT);
         const double ke = v_kappa_es(V, ir, fr, iT, fT);
         const double ag = fabs(gs);
         double ka_med = 0.0;
+#pragma unroll
         for (int b = 0; b < 3; ++b) {
-            const double nu = ag * rgb_nu(b);
-            const double ka = v_kappa_abs(V, nu, ir, fr, iT, fT);
-            if (b == 1) ka_med = ka;
-            const double kt = ka + ke;
-            const double eps = (kt > 0.0) ? ka / kt : 1.0;
-            const double dtau = kt * rho * dsp;
-            const double B = planck_nu(nu, Tl);
-            const double Sv = eps * B / (nu * nu * nu);
-            const double e = exp(-dtau);
-            J[b] += Tt[b] * Sv * (1.0 - e);
-            Tt[b] *= e;
+            const BinStep s = v_bin_step(V, ag * rgb_nu(b), Tl, rho, dsp, ke, ir, fr, iT, fT);
+            if (b == 1) ka_med = s.ka;
+            J[b] = __fma_rn(__dmul_rn(Tt[b], s.src), __dadd_rn(1.0, -s.e), J[b]);
+            Tt[b] *= s.e;
         }
         cnt.bins += 3;
         const double at = (ka_med + ke) * rho;
-        const double ds_tau = (at > 0.0) ? 0.05 / at : ds * 2.0;
+        const double ds_tau = (at > 0.0) ? div_f64(0.05, at) : ds * 2.0;
         const double ds_geo = 0.1 * vmax(r - V.r_horizon, 0.5);
         ds = vclamp(vmin(ds_tau, ds_geo), H / 64.0, H);
     }
