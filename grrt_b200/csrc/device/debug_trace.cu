@@ -7,7 +7,7 @@
 // and an END record (termination, colour, attempts).
 //
 // The steps are the render kernels' own: dp45_attempt_k1 with the kept k1,
-// pi_control, vol_clamp, vol_enters and vol_march_rgb, so the record
+// pi_control, vol_clamp, vol_enters and the march's functions, so the record
 // list describes the ray those kernels trace for the same sample. Like the
 // reference's debug trace, the END colour is the disk's (and the volume's)
 // emission only; the sky is not added. One thread does the work: the trace is
@@ -127,7 +127,21 @@ __global__ void __launch_bounds__(32) debug_trace_kernel(const __grid_constant__
                 bool end = false;
                 while (!end) {
                     ms = rk4_step<double>(S.M, S.a, pt, pph, ms, ds);
-                    end = vol_march_rgb(S, pt, pph, ms, vol_geo(V, ms.r, ms.th), ds, been_inside, J, Tt, cnt);
+                    const VolGeo g = vol_geo(V, ms.r, ms.th);
+                    const bool thick = Tt[0] < 1e-6 && Tt[1] < 1e-6 && Tt[2] < 1e-6;
+                    const MarchState m = vol_march_state(V, ms.r, g, thick, been_inside, ds);
+                    PhysStep ps;
+                    if (m == kMarchInside && vol_physics(V, pt, pph, ms, g, ds, ps)) {
+                        double ka_med = 0.0;
+                        for (int b = 0; b < 3; ++b) {
+                            const BinStep s = v_bin_step(V, ps.ag * rgb_nu(b), ps.T, ps.rho, ps.dsp, ps.ke, ps.ir,
+                                                         ps.fr, ps.iT, ps.fT);
+                            if (b == 1) ka_med = s.ka;
+                            vol_transfer(s, J[b], Tt[b]);
+                        }
+                        ds = vol_next_ds(V, ms.r, g.H, ka_med, ps.ke, ps.rho, ds);
+                    }
+                    end = m == kMarchEnd;
                     ++mcount;
                     if (!end && mcount >= 4096) end = true;
                 }

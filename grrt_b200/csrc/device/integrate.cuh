@@ -42,10 +42,12 @@ GRRT_HD Vec5<T> axpy(const Vec5<T>& y, T h, const Vec5<T>& k) {
 struct DpConst {
     double a21, a31, a32, a41, a42, a43, a51, a52, a53, a54, a61, a62, a63, a64, a65;
     double b1, b3, b4, b5, b6, e1, e3, e4, e5, e6, e7, floor;
+    double next[2], err[2];  // a65, b6 and e5, e6
 };
 static __constant__ DpConst kDp = {dp::a21, dp::a31, dp::a32, dp::a41, dp::a42, dp::a43, dp::a51, dp::a52, dp::a53,
                                    dp::a54, dp::a61, dp::a62, dp::a63, dp::a64, dp::a65, dp::b1, dp::b3, dp::b4,
-                                   dp::b5, dp::b6, dp::e1, dp::e3, dp::e4, dp::e5, dp::e6, dp::e7, 1e-10};
+                                   dp::b5, dp::b6, dp::e1, dp::e3, dp::e4, dp::e5, dp::e6, dp::e7, 1e-10,
+                                   {dp::a65, dp::b6}, {dp::e5, dp::e6}};
 
 // n / d, correctly rounded, from inv = the rounded 1 / d: the quotient
 // corrected by its exact residual (Markstein, as recip_f64). For numbers far
@@ -57,10 +59,11 @@ __device__ __forceinline__ double div_by(double n, double d, double inv) {
 
 // n / d, correctly rounded: by the reciprocal for 2^-450 <= |n|, |d| < 2^450
 // or n = 0, by the division operator elsewhere.
+static __device__ __noinline__ double div_call(double n, double d) { return n / d; }
 __device__ __forceinline__ double div_f64(double n, double d) {
     const int hn = __double2hiint(n) & 0x7fffffff, hd = __double2hiint(d) & 0x7fffffff;
     const bool n_ok = static_cast<unsigned>(hn - 0x23d00000) < 0x38400000u || (hn | __double2loint(n)) == 0;
-    if (!n_ok || static_cast<unsigned>(hd - 0x23d00000) >= 0x38400000u) return n / d;
+    if (!n_ok || static_cast<unsigned>(hd - 0x23d00000) >= 0x38400000u) return div_call(n, d);
     return div_by(n, d, recip_f64(d));
 }
 
@@ -73,6 +76,36 @@ __device__ __forceinline__ double div_f64(double n, double d) {
 struct ErrQuotient {
     double num, den;  // error norm = num / den
 };
+
+// The error norm of dp45_attempt_k1 as the quotient it is, the largest one
+// picked by a tree: with every term finite the order of the comparisons does
+// not matter. qe: the error sum up to the sixth stage.
+__device__ __forceinline__ ErrQuotient error_quotient(const Vec5<double>& y5, double h, const Vec5<double>& k7,
+                                                      const Vec5<double>& qe) {
+    const DpConst& C = kDp;
+#define GRRT_N(f) fabs(__dmul_rn(h, __fma_rn(C.e7, k7.f, qe.f)))
+#define GRRT_D(f) __dadd_rn(fabs(y5.f), C.floor)
+    const ErrQuotient q[5] = {{GRRT_N(r), GRRT_D(r)},
+                              {GRRT_N(th), GRRT_D(th)},
+                              {GRRT_N(ph), GRRT_D(ph)},
+                              {GRRT_N(pr), GRRT_D(pr)},
+                              {GRRT_N(pth), GRRT_D(pth)}};
+#undef GRRT_N
+#undef GRRT_D
+    auto larger = [](const ErrQuotient& u, const ErrQuotient& v) {
+        const bool gt = __dmul_rn(u.num, v.den) < __dmul_rn(v.num, u.den);
+        return ErrQuotient{gt ? v.num : u.num, gt ? v.den : u.den};
+    };
+    int top = 0;
+#pragma unroll
+    for (int i = 0; i < 5; ++i) top = max(top, max(__double2hiint(q[i].num), __double2hiint(q[i].den)));
+    if (top >= 0x7ff00000) {  // an infinity or a NaN: the terms in order, a NaN skipped
+        ErrQuotient m{0.0, 1.0};
+        for (int i = 0; i < 5; ++i) m = larger(m, q[i]);
+        return m;
+    }
+    return larger(larger(larger(q[0], q[1]), larger(q[2], q[3])), q[4]);
+}
 
 #define GRRT_V4(s) {s(r), s(th), 0.0, s(pr), s(pth)}
 #define GRRT_V5(s) {s(r), s(th), s(ph), s(pr), s(pth)}
@@ -116,30 +149,47 @@ __device__ __forceinline__ ErrQuotient dp45_tail_f64(const F& f, const Vec5<doub
 #undef GRRT_QE5
 #undef GRRT_QE6
 #undef GRRT_Y5
-    // the norm of dp45_attempt_k1, the largest quotient picked by a tree: with
-    // every term finite the order of the comparisons does not matter
-#define GRRT_N(f) fabs(__dmul_rn(h, __fma_rn(C.e7, k7.f, qe.f)))
-#define GRRT_D(f) __dadd_rn(fabs(y5.f), C.floor)
-    const ErrQuotient q[5] = {{GRRT_N(r), GRRT_D(r)},
-                              {GRRT_N(th), GRRT_D(th)},
-                              {GRRT_N(ph), GRRT_D(ph)},
-                              {GRRT_N(pr), GRRT_D(pr)},
-                              {GRRT_N(pth), GRRT_D(pth)}};
-#undef GRRT_N
-#undef GRRT_D
-    auto larger = [](const ErrQuotient& u, const ErrQuotient& v) {
-        const bool gt = __dmul_rn(u.num, v.den) < __dmul_rn(v.num, u.den);
-        return ErrQuotient{gt ? v.num : u.num, gt ? v.den : u.den};
-    };
-    int top = 0;
-#pragma unroll
-    for (int i = 0; i < 5; ++i) top = max(top, max(__double2hiint(q[i].num), __double2hiint(q[i].den)));
-    if (top >= 0x7ff00000) {  // an infinity or a NaN: the terms in order, a NaN skipped
-        ErrQuotient m{0.0, 1.0};
-        for (int i = 0; i < 5; ++i) m = larger(m, q[i]);
-        return m;
+    return error_quotient(y5, h, k7, qe);
+}
+
+// dp45_tail_f64 with its last three stages as one loop body, for kernels whose
+// code must stay small: sums of no later use are formed as well.
+template <typename F>
+__device__ __forceinline__ ErrQuotient dp45_tail_rolled_f64(const F& f, const Vec5<double>& y, double h,
+                                                            const Vec5<double>& k1, const Vec5<double>& k2,
+                                                            const Vec5<double>& k3, const Vec5<double>& k4,
+                                                            Vec5<double>& y5, Vec5<double>& k7) {
+    const DpConst& C = kDp;
+#define GRRT_S5(f) \
+    __fma_rn(h, __fma_rn(C.a54, k4.f, __fma_rn(C.a53, k3.f, sum2_f64(C.a51, k1.f, C.a52, k2.f))), y.f)
+    Vec5<double> s GRRT_V4(GRRT_S5);
+#define GRRT_Q6(f) __fma_rn(C.a64, k4.f, __fma_rn(C.a63, k3.f, sum2_f64(C.a61, k1.f, C.a62, k2.f)))
+    Vec5<double> qa GRRT_V4(GRRT_Q6);
+#define GRRT_QB(f) __fma_rn(C.b4, k4.f, sum2_f64(C.b1, k1.f, C.b3, k3.f))
+    const Vec5<double> qb GRRT_V5(GRRT_QB);
+#define GRRT_QE(f) __fma_rn(C.e4, k4.f, sum2_f64(C.e1, k1.f, C.e3, k3.f))
+    Vec5<double> qe GRRT_V5(GRRT_QE);
+#undef GRRT_S5
+#undef GRRT_Q6
+#undef GRRT_QB
+#undef GRRT_QE
+#pragma unroll 1
+    for (int i = 0;; ++i) {
+        k7 = f(s);
+        if (i == 2) break;
+        const double ca = C.next[i], ce = C.err[i];
+#define GRRT_NEXT(f) __fma_rn(h, __fma_rn(ca, k7.f, qa.f), y.f)
+        s = GRRT_V5(GRRT_NEXT);
+#define GRRT_SB(f) __fma_rn(C.b5, k7.f, qb.f)
+        qa = GRRT_V5(GRRT_SB);
+#define GRRT_SE(f) __fma_rn(ce, k7.f, qe.f)
+        qe = GRRT_V5(GRRT_SE);
+#undef GRRT_NEXT
+#undef GRRT_SB
+#undef GRRT_SE
     }
-    return larger(larger(larger(q[0], q[1]), larger(q[2], q[3])), q[4]);
+    y5 = s;
+    return error_quotient(y5, h, k7, qe);
 }
 
 // f: the right-hand side of a state (its phi unused).
@@ -454,6 +504,11 @@ GRRT_HD StepDecision pi_control(double err, double tol, double dl, int retry,
 // Those cases (1 in 10^7), numbers near the range's ends and tolerances
 // where the 1e-30 rule could matter take pi_control. Positive doubles are
 // compared as integers, off the FP64 pipe.
+static __device__ __noinline__ StepDecision pi_control_call(double num, double den, double tol, double dl, int retry,
+                                                            double r5) {
+    return pi_control(num / den, tol, dl, retry, r5);
+}
+
 __device__ __forceinline__ StepDecision pi_control_q(const ErrQuotient& q, double tol, double dl, int retry,
                                                      double r5) {
     constexpr double safety = 0.9, grow_max = 5.0, shrink_max = 0.2, dl_min = 1e-6;
@@ -469,7 +524,7 @@ __device__ __forceinline__ StepDecision pi_control_q(const ErrQuotient& q, doubl
     const bool near_half = ((static_cast<unsigned>(rb) - 0x10000000u + 16u) & 0x1fffffffu) <= 32u;
     const bool near_one = static_cast<unsigned long long>(rb - 0x3ff0000000000000ll + 64) <= 128ull;
     if (!in_range || near_half || near_one || !(tol >= 1e-20 && tol <= 1e20))
-        return pi_control(div_f64(q.num, q.den), tol, dl, retry, r5);
+        return pi_control_call(q.num, q.den, tol, dl, retry, r5);
     auto less = [](double a, double b) { return __double_as_longlong(a) < __double_as_longlong(b); };
     const bool ok = rb >= 0x3ff0000000000000ll;
     double f = __dmul_rn(safety, static_cast<double>(__powf(static_cast<float>(ratio), 0.2f)));

@@ -7,11 +7,13 @@
 //
 // Same persistent execution model as the thin-disk kernel: a lane owns one
 // pixel, one loop iteration advances each live ray by one DP45 attempt (outer
-// phase) or one RK4 march step (march phase); the three channels' transfer
-// state sits in registers. As in the spectral kernel, a step keeps what the
-// next one needs and both kinds of step share their stages 2 to 4 (Kerr a=0.9,
-// 512x512, mixed form on B200: 42 -> 31 ms). The list instantiation is the FP64
-// re-trace of the mixed form (its speculation is in vol_spectral.cu).
+// phase) or one RK4 march step (march phase). The three channels' transfer of
+// the lanes' physics steps is done by the warp, ten steps at once, with the
+// rays' transfer state in shared memory (Kerr a=0.9, 512x512, mixed form on
+// B200: 23.3 -> 19.5 ms against three passes by each ray's own lane). As in the
+// spectral kernel, a step keeps what the next one needs and both kinds of step
+// share their stages 2 to 4. The list instantiation is the FP64 re-trace of the
+// mixed form (its speculation is in vol_spectral.cu).
 #include <cuda_runtime.h>
 
 #include <cstdint>
@@ -33,7 +35,7 @@ constexpr unsigned kFullMask = 0xffffffffu;
 
 }  // namespace
 
-// Three channels in registers; the march ends when all T < 1e-6.
+// The march ends when all three channels' T < 1e-6.
 // kList = false: work item = pixel of the tile, spp samples summed into the
 // outputs. kList = true (the mixed form's re-trace): work item k = sample
 // list[k] (pixel * grid^2 + s); out_d[3 q ..] receives the sample's colour and
@@ -52,7 +54,7 @@ vol_render_kernel(const __grid_constant__ DevScene S, const DevTile tile, float4
     const int grid2 = S.grid * S.grid;
 
     VolCounters cnt;
-    int pix = -1, smp = 0;
+    int pix = lane < vol_lanes_in_use(total) ? -1 : -2, smp = 0;
     double acc[3] = {0.0, 0.0, 0.0};
     bool live = false, need_start = false, marching = false;
     // the outer loop's state, or the march's (which starts from the state
@@ -60,12 +62,19 @@ vol_render_kernel(const __grid_constant__ DevScene S, const DevTile tile, float4
     Vec5<double> y{};
     Vec5<double> k1{};  // f(y) while k1_ok: the last accepted attempt's k7 or this step's first stage
     bool k1_ok = false;
-    VolGeo geo{};       // the geometry of y while geo_ok
-    bool geo_ok = false;
+    VolGeo geo{};       // the geometry of y where vol_near_radius
     double pt = 0.0, pph = 0.0, dl = 0.0, dlambda = 0.0;  // dl: trial step, or the march's step
     int retry = 0, step = 0, entries = 0;
-    // transfer state (RGB in registers)
-    double J[3] = {0.0, 0.0, 0.0}, Tt[3] = {1.0, 1.0, 1.0};
+    // transfer state of the warp's rays, and the stage of their physics steps
+    __shared__ PhysStage stage[kVolThreads / 32];
+    __shared__ double J_all[kVolThreads / 32][3][32], T_all[kVolThreads / 32][3][32];
+    PhysStage& W = stage[threadIdx.x >> 5];
+    double(&J)[3][32] = J_all[threadIdx.x >> 5];
+    double(&Tt)[3][32] = T_all[threadIdx.x >> 5];
+    bool opaque = false;  // all T < 1e-6
+    // the lane's place in a pass over physics steps: ten rays' three channels
+    const int slot_ray = lane / 3, slot_ch = lane % 3;
+    const double slot_nu = rgb_nu(slot_ch);
     int mcount = 0;
     bool been_inside = false;
     bool cancelled = false;
@@ -110,10 +119,14 @@ vol_render_kernel(const __grid_constant__ DevScene S, const DevTile tile, float4
                 step = 0;
                 entries = 0;
                 marching = false;
-                J[0] = J[1] = J[2] = 0.0;
-                Tt[0] = Tt[1] = Tt[2] = 1.0;
+#pragma unroll
+                for (int ch = 0; ch < 3; ++ch) {
+                    J[ch][lane] = 0.0;
+                    Tt[ch][lane] = 1.0;
+                }
+                opaque = false;
                 k1_ok = false;
-                geo_ok = false;
+                if (vol_near_radius(V, y.r)) geo = vol_geo(V, y.r, y.th);
                 live = true;
                 need_start = true;
             }
@@ -131,6 +144,8 @@ vol_render_kernel(const __grid_constant__ DevScene S, const DevTile tile, float4
         auto rhs = [&](const Vec5<double>& s) {
             return kerr_rhs_f64(KerrHole{S.M, S.a, S.a2, S.m2}, pt, pph, s.r, s.th, s.pr, s.pth);
         };
+        // a march step was taken; it ends inside the volume; the march ends
+        bool stepped = false, inside = false, mend = false;
         if (live && term < 0) {
             // ---- first stage, where the last step did not leave it (a march's first step
             //      takes the outer step's) ----
@@ -140,23 +155,21 @@ vol_render_kernel(const __grid_constant__ DevScene S, const DevTile tile, float4
             }
             // ---- near-disk clamp of a new outer step ----
             if (need_start) {
-                if (vol_near_radius(V, y.r)) {
-                    if (!geo_ok) geo = vol_geo(V, y.r, y.th);
-                    geo_ok = true;
-                    if (vol_clamp(k1, y.r, geo, dlambda)) ++cnt.clamp;
-                }
+                if (vol_near_radius(V, y.r) && vol_clamp(k1, y.r, geo, dlambda)) ++cnt.clamp;
                 dl = dlambda;
                 retry = 0;
                 need_start = false;
             }
             Vec5<double> k2, k3, k4;
             shared_stages_f64(rhs, marching, y, dl, k1, k2, k3, k4);
+            Vec5<double> y_new, k7;  // the step's end
+            bool moved = true;       // not a rejected attempt
             if (!marching) {
                 // ---- the rest of the DP45 attempt ----
-                Vec5<double> y5, k7;
-                const ErrQuotient err = dp45_tail_f64(rhs, y, dl, k1, k2, k3, k4, y5, k7);
+                const ErrQuotient err = dp45_tail_rolled_f64(rhs, y, dl, k1, k2, k3, k4, y_new, k7);
                 ++cnt.attempts;
-                const StepDecision d = pi_control_q(err, S.tol, dl, retry, y5.r);
+                const StepDecision d = pi_control_q(err, S.tol, dl, retry, y_new.r);
+                moved = d.accept;
                 if (!d.accept) {
                     dl = d.next;
                     ++retry;
@@ -164,38 +177,80 @@ vol_render_kernel(const __grid_constant__ DevScene S, const DevTile tile, float4
                     ++cnt.accepted;
                     dlambda = d.next;
                     ++step;  // the reference's loop counter advances on every outer iteration
-                    // hand-over to the ray-march (src/geodesic_tracer.cpp:105-153)
-                    const bool opaque = (Tt[0] < 1e-6 && Tt[1] < 1e-6 && Tt[2] < 1e-6);
-                    const bool may = vol_may_enter(V, y.r, y5.r);
-                    VolGeo g5{};
-                    if (may) g5 = vol_geo(V, y5.r, y5.th);
-                    if (!opaque && may && vol_enters(V, y, geo, y5, g5)) {
-                        marching = true;  // from the pre-step state
-                        ++entries;
-                        dl = vol_march_start(V, y.r, geo, been_inside);
-                        mcount = 0;
-                    } else {
-                        // the next outer step starts now, or when the march ends
-                        y = y5;
-                        k1 = k7;
-                        geo = g5;
-                        geo_ok = may;
-                        need_start = true;
-                    }
                 }
             } else {
                 // ---- the end of the RK4 march step ----
-                y = rk4_end_f64(y, dl, k1, k2, k3, k4);
-                geo = vol_geo(V, y.r, y.th);
+                y_new = rk4_end_f64(y, dl, k1, k2, k3, k4);
                 k1_ok = false;
-                const bool end = vol_march_rgb(S, pt, pph, y, geo, dl, been_inside, J, Tt, cnt);
                 ++mcount;
-                if (end || mcount >= 4096) {
-                    marching = false;  // the outer loop continues from the march's end state
-                    geo_ok = true;
+            }
+            // ---- where the step ended: one lookup for both kinds ----
+            const bool may = moved && !marching && vol_may_enter(V, y.r, y_new.r);
+            VolGeo g{};
+            if (moved && (marching || may || vol_near_radius(V, y_new.r))) g = vol_geo(V, y_new.r, y_new.th);
+            if (!moved) {
+            } else if (!marching) {
+                // ---- hand-over to the ray-march (src/geodesic_tracer.cpp:105-153) ----
+                if (!opaque && may && vol_enters(V, y, geo, y_new, g)) {
+                    marching = true;  // from the pre-step state
+                    ++entries;
+                    dl = vol_march_start(V, y.r, geo, been_inside);
+                    mcount = 0;
+                } else {
+                    // the next outer step starts now, or when the march ends
+                    y = y_new;
+                    k1 = k7;
+                    geo = g;
                     need_start = true;
                 }
+            } else {
+                // ---- the march's end or next step length; inside, its physics first ----
+                y = y_new;
+                geo = g;
+                stepped = true;
+                ++cnt.march;
+                const MarchState m = vol_march_state(V, y.r, geo, opaque, been_inside, dl);
+                inside = m == kMarchInside;
+                mend = m == kMarchEnd;
             }
+        }
+
+        // ---- physics of the steps that end inside the volume ----
+        bool phys = false;
+        PhysStep ps;
+        if (inside) phys = vol_physics(V, pt, pph, y, geo, dl, ps);
+
+        // ---- transfer in the three channels, ten rays at once ----
+        const unsigned pm = __ballot_sync(kFullMask, phys);
+        if (pm) {
+            const int n = __popc(pm), rank = __popc(pm & lt_mask);
+            if (phys) W.put(rank, ps, lane);
+            __syncwarp();
+            double ka_med = 0.0;
+            for (int base = 0; base < n; base += 10) {
+                const int k = base + slot_ray;
+                double ka = 0.0;
+                if (slot_ray < 10 && k < n) {
+                    const BinStep st = W.bin(V, k, slot_nu);
+                    ka = st.ka;
+                    const int src = W.src[k];
+                    vol_transfer(st, J[slot_ch][src], Tt[slot_ch][src]);
+                }
+                const bool mine = rank >= base && rank - base < 10;  // with phys
+                const double kam = __shfl_sync(kFullMask, ka, mine ? 3 * (rank - base) + 1 : 0);
+                if (mine) ka_med = kam;
+            }
+            __syncwarp();
+            if (phys) {
+                ++cnt.physics;
+                cnt.bins += 3;
+                opaque = Tt[0][lane] < 1e-6 && Tt[1][lane] < 1e-6 && Tt[2][lane] < 1e-6;
+                dl = vol_next_ds(V, y.r, geo.H, ka_med, ps.ke, ps.rho, dl);
+            }
+        }
+        if (stepped && (mend || mcount >= 4096)) {
+            marching = false;  // the outer loop continues from the march's end state
+            need_start = true;
         }
 
         // ---- finish the terminated samples ----
@@ -212,7 +267,7 @@ vol_render_kernel(const __grid_constant__ DevScene S, const DevTile tile, float4
             double col[3];
             for (int ch = 0; ch < 3; ++ch) {
                 const double nu = rgb_nu(ch);
-                col[ch] = 0.0 + J[ch] * nu * nu * nu;
+                col[ch] = 0.0 + J[ch][lane] * nu * nu * nu;
             }
             if (term == kTermEscaped && S.stars_on) {
                 const double bright = star_brightness(S.stars, y.th, y.ph);
@@ -289,7 +344,7 @@ cudaError_t launch_volume_rgb(const DevScene& S, const DevTile& tile, const Thin
     const unsigned total = static_cast<unsigned>(tile.w) * static_cast<unsigned>(tile.h);
     if (total == 0) return cudaSuccess;
     int blocks = sms * per;
-    const int needed = static_cast<int>((total + kVolThreads - 1) / kVolThreads);
+    const int needed = static_cast<int>((total + kVolThreads / 32 - 1) / (kVolThreads / 32));  // a ray a warp
     if (needed < blocks) blocks = needed;
     cudaError_t e = cudaMemsetAsync(res.queue, 0, 2 * sizeof(unsigned int), stream);
     if (e != cudaSuccess) return e;

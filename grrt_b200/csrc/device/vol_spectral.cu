@@ -10,8 +10,9 @@
 // redshift and the table coordinates of rho and T). The per-bin part of a
 // physics step (opacity, Planck function, the J / T / tau update: nb bins) is
 // done by the whole warp, one bin per lane: each loop iteration, the lanes
-// that reached a physics step are served in turn, so the cost is one pass
-// over the bins instead of nb serial passes while 31 lanes wait. Ray starts
+// that reached a physics step stage it in shared memory and are served in
+// turn, several at once with 16 bins or fewer, so the cost is one pass over the
+// bins instead of nb serial passes while 31 lanes wait. Ray starts
 // and sample finishes (reset of the ray's row, the J nu^3 sum and the
 // coalesced store of a pixel's spectrum) are served the same way.
 //
@@ -21,7 +22,11 @@
 // the geometry of its state), both kinds of step share the right-hand sides of
 // stages 2 to 4 (a warp holds both), and an iteration takes two votes unless a
 // sample ended (Kerr a=0.9, 512x512, 32 bins on B200: 62 -> 37 ms for the FP64
-// form; 101x75, 16 bins, mixed: 28 -> 14.4 ms).
+// form; 101x75, 16 bins, mixed: 28 -> 14.4 ms). What stalls the full phase is
+// instruction fetch (3.0 of 6.8 cycles an instruction), so the last stages are
+// a loop, both kinds of step share one geometry lookup, and the physics calls
+// one body of each library function; and where a frame has fewer rays than
+// lanes they are spread over the warps (33 -> 29 ms; 13.6 -> 11.7 ms).
 //
 // A ray's transfer state is a row of 4 x nb doubles per lane slot
 // [J | T | tau | pixel sum], so the warp's accesses to one row are
@@ -97,20 +102,27 @@ vol_spectral_kernel(const __grid_constant__ DevScene S0, const DevTile tile, con
     const double* freqs = freqs0;
 
     VolCounters cnt;
-    int pix = -1, smp = 0;  // kList: pix = the listed sample
+    int pix = lane < vol_lanes_in_use(total) ? -1 : -2, smp = 0;  // kList: pix = the listed sample
     bool live = false, need_start = false, marching = false;
     // the outer loop's state, or the march's (which starts from the state
     // before the step that handed over)
     Vec5<double> y{};
     Vec5<double> k1{};  // f(y) while k1_ok: the last accepted attempt's k7 or this step's first stage
     bool k1_ok = false;
-    VolGeo geo{};       // the geometry of y while geo_ok
-    bool geo_ok = false;
+    VolGeo geo{};       // the geometry of y where vol_near_radius
     double pt = 0.0, pph = 0.0, dl = 0.0, dlambda = 0.0;  // dl: trial step, or the march's step
     int retry = 0, step = 0, entries = 0, n_thick = 0, mcount = 0;
     bool been_inside = false, cancelled = false;
     unsigned iter = 0;
     bool refill = true;  // warp-uniform: some lane has no ray
+    // the lane's place in a pass over physics steps: which of the pass's rays,
+    // which bin (the first, of a ray with more bins than lanes)
+    __shared__ PhysStage stage[kSpecThreads / 32];
+    PhysStage& W = stage[threadIdx.x >> 5];
+    const int slot_bins = (kBatch || nb0 > 16) ? 32 : nb0;
+    const int rays_at_once = 32 / slot_bins;
+    const int slot_ray = lane / slot_bins, slot_bin = lane % slot_bins;
+    const unsigned slot_mask = slot_bins == 32 ? kWarp : (1u << slot_bins) - 1u;
 
     while (true) {
         if (refill) {
@@ -181,7 +193,7 @@ vol_spectral_kernel(const __grid_constant__ DevScene S0, const DevTile tile, con
                 marching = false;
                 n_thick = 0;
                 k1_ok = false;
-                geo_ok = false;
+                if (vol_near_radius(V, y.r)) geo = vol_geo(V, y.r, y.th);
                 live = true;
                 need_start = true;
                 fresh_ray = true;
@@ -216,13 +228,8 @@ vol_spectral_kernel(const __grid_constant__ DevScene S0, const DevTile tile, con
             return kerr_rhs_f64(KerrHole{S.M, S.a, S.a2, S.m2}, pt, pph, s.r, s.th, s.pr, s.pth);
         };
 
-        // physics step inputs handed to the warp (bin-independent)
-        bool phys = false;
-        double ph_ag = 0.0, ph_rho = 0.0, ph_T = 0.0, ph_dsp = 0.0, ph_ke = 0.0, ph_fr = 0.0, ph_fT = 0.0;
-        double ph_kamed = 0.0;
-        int ph_ir = 0, ph_iT = 0;
-        bool mend = false;
-        const bool marched = marching;  // this iteration's step is a march step
+        // a march step was taken; it ends inside the volume; the march ends
+        bool stepped = false, inside = false, mend = false;
         if (live && term < 0) {
             // ---- first stage, where the last step did not leave it (a march's first step
             //      takes the outer step's) ----
@@ -232,23 +239,21 @@ vol_spectral_kernel(const __grid_constant__ DevScene S0, const DevTile tile, con
             }
             // ---- near-disk clamp of a new outer step ----
             if (need_start) {
-                if (vol_near_radius(V, y.r)) {
-                    if (!geo_ok) geo = vol_geo(V, y.r, y.th);
-                    geo_ok = true;
-                    if (vol_clamp(k1, y.r, geo, dlambda)) ++cnt.clamp;
-                }
+                if (vol_near_radius(V, y.r) && vol_clamp(k1, y.r, geo, dlambda)) ++cnt.clamp;
                 dl = dlambda;
                 retry = 0;
                 need_start = false;
             }
             Vec5<double> k2, k3, k4;
             shared_stages_f64(rhs, marching, y, dl, k1, k2, k3, k4);
+            Vec5<double> y_new, k7;  // the step's end
+            bool moved = true;       // not a rejected attempt
             if (!marching) {
                 // ---- the rest of the DP45 attempt ----
-                Vec5<double> y5, k7;
-                const ErrQuotient err = dp45_tail_f64(rhs, y, dl, k1, k2, k3, k4, y5, k7);
+                const ErrQuotient err = dp45_tail_rolled_f64(rhs, y, dl, k1, k2, k3, k4, y_new, k7);
                 ++cnt.attempts;
-                const StepDecision d = pi_control_q(err, S.tol, dl, retry, y5.r);
+                const StepDecision d = pi_control_q(err, S.tol, dl, retry, y_new.r);
+                moved = d.accept;
                 if (!d.accept) {
                     dl = d.next;
                     ++retry;
@@ -256,79 +261,60 @@ vol_spectral_kernel(const __grid_constant__ DevScene S0, const DevTile tile, con
                     ++cnt.accepted;
                     dlambda = d.next;
                     ++step;  // the reference's loop counter advances on every outer iteration
-                    // hand-over to the ray-march (src/geodesic_tracer.cpp:105-153)
-                    const bool may = vol_may_enter(V, y.r, y5.r);
-                    VolGeo g5{};
-                    if (may) g5 = vol_geo(V, y5.r, y5.th);
-                    if (may && vol_enters(V, y, geo, y5, g5)) {
-                        marching = true;  // from the pre-step state
-                        ++entries;
-                        dl = vol_march_start(V, y.r, geo, been_inside);
-                        mcount = 0;
-                    } else {
-                        y = y5;
-                        k1 = k7;
-                        geo = g5;
-                        geo_ok = may;
-                        need_start = true;
-                    }
                 }
             } else {
-                // ---- the end of the RK4 march step (geometry; the bins follow below) ----
-                y = rk4_end_f64(y, dl, k1, k2, k3, k4);
-                geo = vol_geo(V, y.r, y.th);
+                // ---- the end of the RK4 march step ----
+                y_new = rk4_end_f64(y, dl, k1, k2, k3, k4);
                 k1_ok = false;
                 ++mcount;
                 ++cnt.march;
-                const double r = y.r;
-                if (r < V.r_horizon || r > V.r_outer) {
-                    mend = true;
-                } else if (n_thick == nb) {
-                    mend = true;
-                } else if (!geo_inside(V, r, geo)) {
-                    const double H = geo.H;
-                    if (been_inside && fabs(geo.z) > __fma_rn(3.0, H, geo.zm)) {
-                        mend = true;
-                    } else if (!been_inside) {
-                        dl = vmax(vmin(fabs(geo.z) / 8.0, H * 2.0), H / 64.0);
-                    } else {
-                        dl = vclamp(H / 4.0, H / 64.0, H);
-                    }
+            }
+            // ---- where the step ended: one lookup for both kinds ----
+            const bool may = moved && !marching && vol_may_enter(V, y.r, y_new.r);
+            VolGeo g{};
+            if (moved && (marching || may || vol_near_radius(V, y_new.r))) g = vol_geo(V, y_new.r, y_new.th);
+            if (!moved) {
+            } else if (!marching) {
+                // ---- hand-over to the ray-march (src/geodesic_tracer.cpp:105-153) ----
+                if (may && vol_enters(V, y, geo, y_new, g)) {
+                    marching = true;  // from the pre-step state
+                    ++entries;
+                    dl = vol_march_start(V, y.r, geo, been_inside);
+                    mcount = 0;
                 } else {
-                    been_inside = true;
-                    double rho, Tl;
-                    v_density_temperature(V, V.perm, r, geo.z, y.ph, geo.H, geo.zm, rho, Tl);
-                    if (rho > 0.0 && Tl > 0.0) {
-                        ++cnt.physics;
-                        double g, pue;
-                        v_redshift(V, pt, y.pr, pph, r, geo.ct, g, pue);
-                        ph_dsp = fabs(pue) * fabs(dl);
-                        log_locate(log10(rho), V.log_rho_min, V.len_rho, V.inv_len_rho, V.n_rho, ph_ir, ph_fr);
-                        log_locate(log10(Tl), V.log_T_min, V.len_T, V.inv_len_T, V.n_T, ph_iT, ph_fT);
-                        ph_ke = v_kappa_es(V, ph_ir, ph_fr, ph_iT, ph_fT);
-                        ph_ag = fabs(g);
-                        ph_rho = rho;
-                        ph_T = Tl;
-                        phys = true;
-                    }
+                    y = y_new;
+                    k1 = k7;
+                    geo = g;
+                    need_start = true;
                 }
+            } else {
+                // ---- the march's end or next step length; inside, its physics first ----
+                y = y_new;
+                geo = g;
+                stepped = true;
+                const MarchState m = vol_march_state(V, y.r, geo, n_thick == nb, been_inside, dl);
+                inside = m == kMarchInside;
+                mend = m == kMarchEnd;
             }
         }
 
-        // ---- per-bin transfer of this iteration's physics steps, one bin per lane ----
-        {
-            const unsigned pm = __ballot_sync(kWarp, phys);
-            for (unsigned m = pm; m; m &= m - 1) {
-                const int src = __ffs(m) - 1;
-                const double ag = __shfl_sync(kWarp, ph_ag, src);
-                const double rho = __shfl_sync(kWarp, ph_rho, src);
-                const double Tl = __shfl_sync(kWarp, ph_T, src);
-                const double dsp = __shfl_sync(kWarp, ph_dsp, src);
-                const double ke = __shfl_sync(kWarp, ph_ke, src);
-                const double fr = __shfl_sync(kWarp, ph_fr, src);
-                const double fT = __shfl_sync(kWarp, ph_fT, src);
-                const int ir = __shfl_sync(kWarp, ph_ir, src);
-                const int iT = __shfl_sync(kWarp, ph_iT, src);
+        // ---- physics of the steps that end inside the volume ----
+        bool phys = false;
+        PhysStep ps;
+        if (inside) phys = vol_physics(V, pt, pph, y, geo, dl, ps);
+
+        // ---- per-bin transfer of this iteration's physics steps, as many rays at once
+        //      as have their bins in 32 lanes ----
+        const unsigned pm = __ballot_sync(kWarp, phys);
+        if (pm) {
+            const int n = __popc(pm), rank = __popc(pm & lt_mask);
+            if (phys) W.put(rank, ps, lane);
+            __syncwarp();
+            double ka_med = 0.0;
+            for (int base = 0; base < n; base += rays_at_once) {
+                const int k = base + slot_ray;
+                const bool slot = slot_ray < rays_at_once && k < n;
+                const int src = W.src[slot ? k : base];
                 // the served lane's camera: its opacity tables and bins
                 const int sitem = kBatch ? __shfl_sync(kWarp, item, src) : 0;
                 const DevVolume& Vs = kBatch ? B.scenes[B.items[sitem].scene].vol : S0.vol;
@@ -336,42 +322,37 @@ vol_spectral_kernel(const __grid_constant__ DevScene S0, const DevTile tile, con
                 const int snb = kBatch ? B.items[sitem].nb : nb0;
                 const int smed = snb / 2;
                 double* row = row_of(src);
-                double kam = 0.0;
+                const bool mine = rank >= base && rank - base < rays_at_once;  // with phys
                 int thick = 0;
                 for (int b0 = 0; b0 < snb; b0 += 32) {
-                    const int b = b0 + lane;
+                    const int b = b0 + slot_bin;
                     double ka = 0.0;
                     bool thk = false;
-                    if (b < snb) {
-                        const BinStep st =
-                            v_bin_step(Vs, ag * __ldg(sfreqs + b), Tl, rho, dsp, ke, ir, fr, iT, fT);
+                    if (slot && b < snb) {
+                        const BinStep st = W.bin(Vs, k, __ldg(sfreqs + b));
                         ka = st.ka;
                         const double tau = __dadd_rn(row[2 * seg + b], st.dtau);
                         row[2 * seg + b] = tau;
                         thk = !(tau <= 10.0);
-                        const double Tb = row[seg + b];
-                        row[b] = __fma_rn(__dmul_rn(Tb, st.src), __dadd_rn(1.0, -st.e), row[b]);
-                        row[seg + b] = __dmul_rn(Tb, st.e);
+                        vol_transfer(st, row[b], row[seg + b]);
                     }
-                    thick += __popc(__ballot_sync(kWarp, thk));
-                    if (smed >= b0 && smed < b0 + 32) kam = __shfl_sync(kWarp, ka, smed - b0);
+                    // the ray's lanes of this chunk, and its median bin's lane
+                    const int first = mine ? (rank - base) * slot_bins : 0;
+                    thick += __popc((__ballot_sync(kWarp, thk) >> first) & slot_mask);
+                    const double kam = __shfl_sync(kWarp, ka, (first + smed - b0) & 31);
+                    if (smed >= b0 && smed < b0 + 32) ka_med = mine ? kam : ka_med;
                 }
-                if (lane == src) {
-                    ph_kamed = kam;
-                    n_thick = thick;  // bins with tau > 10 (tau only grows)
-                }
+                if (phys && mine) n_thick = thick;  // bins with tau > 10 (tau only grows)
+            }
+            __syncwarp();
+            if (phys) {
+                ++cnt.physics;
+                cnt.bins += static_cast<unsigned>(nb);
+                dl = vol_next_ds(V, y.r, geo.H, ka_med, ps.ke, ps.rho, dl);
             }
         }
-        if (phys) {
-            cnt.bins += static_cast<unsigned>(nb);
-            const double at = (ph_kamed + ph_ke) * ph_rho;
-            const double ds_tau = (at > 0.0) ? div_f64(0.05, at) : dl * 2.0;
-            const double ds_geo = 0.1 * vmax(y.r - V.r_horizon, 0.5);
-            dl = vclamp(vmin(ds_tau, ds_geo), geo.H / 64.0, geo.H);
-        }
-        if (marched && (mend || mcount >= 4096)) {
+        if (stepped && (mend || mcount >= 4096)) {
             marching = false;  // the outer loop continues from the march's end state
-            geo_ok = true;
             need_start = true;
         }
 
@@ -720,7 +701,7 @@ cudaError_t launch_volume_spectral(const DevScene& S, const DevTile& tile, const
     const unsigned total = static_cast<unsigned>(tile.w) * static_cast<unsigned>(tile.h);
     if (total == 0) return cudaSuccess;
     int blocks = sh.sms * sh.per_fp64;
-    const int needed = static_cast<int>((total + kSpecThreads - 1) / kSpecThreads);
+    const int needed = static_cast<int>((total + kSpecThreads / 32 - 1) / (kSpecThreads / 32));  // a ray a warp
     if (needed < blocks) blocks = needed;
     if (!res.spectral_scratch || res.spectral_scratch_elems < static_cast<size_t>(4) * nb * blocks * kSpecThreads)
         return cudaErrorInvalidValue;

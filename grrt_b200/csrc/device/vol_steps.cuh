@@ -35,6 +35,16 @@ __host__ __device__ __forceinline__ unsigned vol_spread_order(unsigned k, unsign
     return base + (j % kVolSpread) * kVolSpread + j / kVolSpread;
 }
 
+// Lanes of a warp that take work items: all 32 of them where the items keep the
+// grid's lanes busy; where there are fewer items than lanes, their number
+// spread over the warps, since a warp runs its lanes' different phases one
+// after another and a ray alone in its warp runs fastest.
+__device__ __forceinline__ int vol_lanes_in_use(unsigned total) {
+    const unsigned warps = gridDim.x * (blockDim.x >> 5);
+    const unsigned per = (total + warps - 1) / warps;
+    return per < 32u ? static_cast<int>(per) : 32;
+}
+
 // Warp sum of the counters, one atomic per counter per warp.
 __device__ __forceinline__ void flush_vol(DevStats* st, const VolCounters& c, bool cancelled) {
     unsigned long long v[11] = {c.attempts, c.accepted, c.rays, c.horizon, c.escaped, c.maxsteps,
@@ -144,56 +154,83 @@ __device__ __forceinline__ double rgb_nu(int ch) {
     return ch == 0 ? c / 450e-7 : (ch == 1 ? c / 550e-7 : c / 650e-7);
 }
 
-// The RGB ray-march's work at a new state ns of geometry g, reached by a step
-// of length ds (src/geodesic_tracer.cpp:183-337): inside the volume the three
-// channels' emission and absorption update J and Tt and the next ds follows
-// the optical depth and the radius; outside it ds approaches the volume (never
-// inside yet) or holds at H/4 (after being inside). Returns whether the march
-// ends here: outside [r_h, r_outer], all channels opaque, or beyond z_max + 3H
-// after being inside. The 4096-step cap is the caller's.
-__device__ __forceinline__ bool vol_march_rgb(const DevScene& S, double pt, double pph, const Vec5<double>& ns,
-                                              const VolGeo& g, double& ds, bool& been_inside, double* J, double* Tt,
-                                              VolCounters& cnt) {
-    const DevVolume& V = S.vol;
-    ++cnt.march;
-    const double r = ns.r;
-    const double z = g.z, H = g.H;
-    if (r < V.r_horizon || r > V.r_outer) return true;
-    if (Tt[0] < 1e-6 && Tt[1] < 1e-6 && Tt[2] < 1e-6) return true;
-    if (!geo_inside(V, r, g)) {
-        if (been_inside && fabs(z) > __fma_rn(3.0, H, g.zm)) return true;
-        ds = been_inside ? vclamp(H / 4.0, H / 64.0, H) : vmax(vmin(fabs(z) / 8.0, H * 2.0), H / 64.0);
-        return false;
+// The ray-march at a new state of radius r and geometry g
+// (src/geodesic_tracer.cpp:183-337): it ends outside [r_h, r_outer], when
+// opaque, or beyond z_max + 3H after being inside; inside the volume the step's
+// physics comes next; elsewhere the next step length ds approaches the volume
+// (never inside yet) or holds at H/4 (after being inside). The 4096-step cap is
+// the caller's.
+enum MarchState { kMarchOn, kMarchEnd, kMarchInside };
+__device__ __forceinline__ MarchState vol_march_state(const DevVolume& V, double r, const VolGeo& g, bool opaque,
+                                                      bool& been_inside, double& ds) {
+    if (r < V.r_horizon || r > V.r_outer || opaque) return kMarchEnd;
+    if (geo_inside(V, r, g)) {
+        been_inside = true;
+        return kMarchInside;
     }
-    been_inside = true;
-    double rho, Tl;
-    v_density_temperature(V, V.perm, r, z, ns.ph, H, g.zm, rho, Tl);
-    if (rho > 0.0 && Tl > 0.0) {
-        ++cnt.physics;
-        double gs, pue;
-        v_redshift(V, pt, ns.pr, pph, r, g.ct, gs, pue);
-        const double dsp = fabs(pue) * fabs(ds);
-        int ir, iT;
-        double fr, fT;
-        log_locate(log10(rho), V.log_rho_min, V.len_rho, V.inv_len_rho, V.n_rho, ir, fr);
-        log_locate(log10(Tl), V.log_T_min, V.len_T, V.inv_len_T, V.n_T, iT, fT);
-        const double ke = v_kappa_es(V, ir, fr, iT, fT);
-        const double ag = fabs(gs);
-        double ka_med = 0.0;
-#pragma unroll
-        for (int b = 0; b < 3; ++b) {
-            const BinStep s = v_bin_step(V, ag * rgb_nu(b), Tl, rho, dsp, ke, ir, fr, iT, fT);
-            if (b == 1) ka_med = s.ka;
-            J[b] = __fma_rn(__dmul_rn(Tt[b], s.src), __dadd_rn(1.0, -s.e), J[b]);
-            Tt[b] *= s.e;
-        }
-        cnt.bins += 3;
-        const double at = (ka_med + ke) * rho;
-        const double ds_tau = (at > 0.0) ? div_f64(0.05, at) : ds * 2.0;
-        const double ds_geo = 0.1 * vmax(r - V.r_horizon, 0.5);
-        ds = vclamp(vmin(ds_tau, ds_geo), H / 64.0, H);
-    }
-    return false;
+    if (been_inside && fabs(g.z) > __fma_rn(3.0, g.H, g.zm)) return kMarchEnd;
+    ds = been_inside ? vclamp(g.H / 4.0, g.H / 64.0, g.H) : vmax(vmin(fabs(g.z) / 8.0, g.H * 2.0), g.H / 64.0);
+    return kMarchOn;
 }
+
+// The frequency-independent part of a physics step.
+struct PhysStep {
+    double ag, rho, T, dsp, ke, fr, fT;  // |g|, density, temperature, path, kappa_es, table fractions
+    int ir, iT;                          // table cell
+};
+// At the march's state y of geometry g inside the volume, reached by a step of
+// length ds; false where there is no matter.
+__device__ __forceinline__ bool vol_physics(const DevVolume& V, double pt, double pph, const Vec5<double>& y,
+                                            const VolGeo& g, double ds, PhysStep& p) {
+    v_density_temperature(V, V.perm, y.r, g.z, y.ph, g.H, g.zm, p.rho, p.T);
+    if (!(p.rho > 0.0 && p.T > 0.0)) return false;
+    double gs, pue;
+    v_redshift(V, pt, y.pr, pph, y.r, g.ct, gs, pue);
+    p.ag = fabs(gs);
+    p.dsp = fabs(pue) * fabs(ds);
+    log_locate(log10_call(p.rho), V.log_rho_min, V.len_rho, V.inv_len_rho, V.n_rho, p.ir, p.fr);
+    log_locate(log10_call(p.T), V.log_T_min, V.len_T, V.inv_len_T, V.n_T, p.iT, p.fT);
+    p.ke = v_kappa_es(V, p.ir, p.fr, p.iT, p.fT);
+    return true;
+}
+
+// The next march step length after a physics step: an optical depth of 0.05 at
+// the median frequency (opacity ka + ke), a tenth of the distance to the
+// horizon, between H/64 and H.
+__device__ __forceinline__ double vol_next_ds(const DevVolume& V, double r, double H, double ka, double ke,
+                                              double rho, double ds) {
+    const double at = (ka + ke) * rho;
+    const double ds_tau = (at > 0.0) ? div_f64(0.05, at) : ds * 2.0;
+    const double ds_geo = 0.1 * vmax(r - V.r_horizon, 0.5);
+    return vclamp(vmin(ds_tau, ds_geo), H / 64.0, H);
+}
+
+// One frequency's transfer: J += T S (1 - e), T *= e.
+__device__ __forceinline__ void vol_transfer(const BinStep& s, double& J, double& T) {
+    J = __fma_rn(__dmul_rn(T, s.src), __dadd_rn(1.0, -s.e), J);
+    T = __dmul_rn(T, s.e);
+}
+
+// Physics steps of a warp's lanes staged in shared memory by rank, for the
+// per-frequency part that the whole warp does.
+struct PhysStage {
+    double ag[32], rho[32], T[32], dsp[32], ke[32], fr[32], fT[32];
+    int ir[32], iT[32], src[32];  // table cell, the lane
+    __device__ __forceinline__ void put(int k, const PhysStep& p, int lane) {
+        ag[k] = p.ag;
+        rho[k] = p.rho;
+        T[k] = p.T;
+        dsp[k] = p.dsp;
+        ke[k] = p.ke;
+        fr[k] = p.fr;
+        fT[k] = p.fT;
+        ir[k] = p.ir;
+        iT[k] = p.iT;
+        src[k] = lane;
+    }
+    __device__ __forceinline__ BinStep bin(const DevVolume& V, int k, double freq) const {
+        return v_bin_step(V, __dmul_rn(ag[k], freq), T[k], rho[k], dsp[k], ke[k], ir[k], fr[k], iT[k], fT[k]);
+    }
+};
 
 }  // namespace grrt_b200

@@ -37,6 +37,19 @@ __device__ __forceinline__ int table_index(double t, int lo, int hi) {
     return static_cast<int>(t);
 }
 
+// One body of each library function that a physics step calls at several
+// places: what stalls the volumetric kernels' full phase is instruction fetch
+// (44% of a warp's cycles on the 512x512 spectral frame), and a physics step's
+// code is cold each time. (Out of line as well, the geometry's sincos cost the
+// frames' long rays more than it saved.)
+static __device__ __noinline__ double exp_call(double x) { return exp(x); }
+static __device__ __noinline__ double log10_call(double x) { return log10(x); }
+static __device__ __noinline__ double2 sincos_call(double x) {
+    double2 r;
+    sincos(x, &r.x, &r.y);
+    return r;
+}
+
 // lo (1 - t) + hi t
 __device__ __forceinline__ double v_lerp(double lo, double hi, double t) {
     return __fma_rn(hi, t, __dmul_rn(lo, __dadd_rn(1.0, -t)));
@@ -162,7 +175,7 @@ __device__ __forceinline__ void v_density_temperature(const DevVolume& V, const 
         const double dz = __dadd_rn(z_abs, -zm);
         dense = !(dz >= __dmul_rn(1.5, H));
         const double d = div_f64(dz, H);
-        edge = exp(__dmul_rn(__dmul_rn(-2.0, d), d));
+        edge = exp_call(__dmul_rn(__dmul_rn(-2.0, d), d));
         z_look = z_top;
     }
     const VolCell c = v_cell(V, r);
@@ -174,12 +187,12 @@ __device__ __forceinline__ void v_density_temperature(const DevVolume& V, const 
     double taper = 1.0;
     if (r < V.r_isco) {
         const double dr = __dadd_rn(V.r_isco, -r);
-        taper = exp(div_by(-__dmul_rn(dr, dr), V.taper_w2, V.inv_taper_w2));
+        taper = exp_call(div_by(-__dmul_rn(dr, dr), V.taper_w2, V.inv_taper_w2));
     }
     const double base = __dmul_rn(
         __dmul_rn(__dmul_rn(__dmul_rn(rho_mid, rho_norm), V.rho_scale), taper), edge);
-    double sp, cp;
-    sincos(phi, &sp, &cp);
+    const double2 sc = sincos_call(phi);
+    const double sp = sc.x, cp = sc.y;
     const double nx = div_by(__dmul_rn(r, cp), V.noise_scale, V.inv_noise);
     const double ny = div_by(__dmul_rn(r, sp), V.noise_scale, V.inv_noise);
     const double nz = div_by(z, V.noise_scale, V.inv_noise);
@@ -251,7 +264,7 @@ __device__ __forceinline__ double v_kappa_es(const DevVolume& V, int ir, double 
 __device__ __forceinline__ double v_kappa_abs(const DevVolume& V, double nu, int ir, double fr, int iT, double fT) {
     int inu;
     double fnu;
-    log_locate(log10(nu), V.log_nu_min, V.len_nu, V.inv_len_nu, V.n_nu, inu, fnu);
+    log_locate(log10_call(nu), V.log_nu_min, V.len_nu, V.inv_len_nu, V.n_nu, inu, fnu);
     const size_t s0 = static_cast<size_t>(V.n_rho) * V.n_T;
     const double* L0 = V.ln_kabs + inu * s0 + ir * V.n_T + iT;
     const double* L1 = L0 + s0;
@@ -260,14 +273,14 @@ __device__ __forceinline__ double v_kappa_abs(const DevVolume& V, double nu, int
     const double l01 = v_mix(__ldg(L0 + nt), __ldg(L0 + nt + 1), fT);
     const double l10 = v_mix(__ldg(L1), __ldg(L1 + 1), fT);
     const double l11 = v_mix(__ldg(L1 + nt), __ldg(L1 + nt + 1), fT);
-    return exp(v_mix(v_mix(l00, l01, fr), v_mix(l10, l11, fr), fnu));
+    return exp_call(v_mix(v_mix(l00, l01, fr), v_mix(l10, l11, fr), fnu));
 }
 
 // One frequency's transfer over a physics step (src/geodesic_tracer.cpp:300-325):
 // opacity, optical depth and Planck emission (CGS, src/opacity.cpp:209-214) at
 // emitter frequency nu.
 struct BinStep {
-    double ka, dtau, src, e;  // kappa_abs, optical depth, source B eps / nu^3, exp(-dtau)
+    double ka, dtau, src, e;  // kappa_abs, optical depth, source B eps / nu^3, exp_call(-dtau)
 };
 __device__ __forceinline__ BinStep v_bin_step(const DevVolume& V, double nu, double T, double rho, double dsp,
                                               double ke, int ir, double fr, int iT, double fT) {
@@ -282,11 +295,11 @@ __device__ __forceinline__ BinStep v_bin_step(const DevVolume& V, double nu, dou
         const double x = div_f64(__dmul_rn(h, nu), __dmul_rn(k, T));
         if (!(x > 500.0)) {
             const double n3 = __dmul_rn(__dmul_rn(__dmul_rn(2.0 * h, nu), nu), nu);
-            B = div_f64(div_by(n3, c * c, 1.0 / (c * c)), __dadd_rn(exp(x), -1.0));
+            B = div_f64(div_by(n3, c * c, 1.0 / (c * c)), __dadd_rn(exp_call(x), -1.0));
         }
     }
     s.src = div_f64(__dmul_rn(eps, B), __dmul_rn(__dmul_rn(nu, nu), nu));
-    s.e = exp(-s.dtau);
+    s.e = exp_call(-s.dtau);
     return s;
 }
 
