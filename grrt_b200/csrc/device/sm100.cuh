@@ -150,10 +150,25 @@ __device__ __forceinline__ uint64_t desc_kmajor_sw128(uint32_t smem_addr) {
     return d;
 }
 
-// kind::f16 instruction descriptor: BF16 x BF16 -> F32, both K-major.
-__host__ __device__ constexpr uint32_t idesc_bf16_f32(int m, int n) {
-    return (1u << 4) | (1u << 7) | (1u << 10) | (static_cast<uint32_t>(n >> 3) << 17) |
-           (static_cast<uint32_t>(m >> 4) << 24);
+// The same of an MN-major operand (its M or N extent contiguous in memory),
+// stored as TMA SWIZZLE_128B boxes of 64 MN elements (128 B) x 64 K rows: 8 K
+// rows are an atom of 1024 B (the stride), the next 64 MN elements are the
+// next box (the leading offset, box_bytes).
+__device__ __forceinline__ uint64_t desc_mnmajor_sw128(uint32_t smem_addr, uint32_t box_bytes) {
+    uint64_t d = 0;
+    d |= static_cast<uint64_t>((smem_addr >> 4) & 0x3FFFu);
+    d |= static_cast<uint64_t>(box_bytes >> 4) << 16;
+    d |= static_cast<uint64_t>(1024 >> 4) << 32;
+    d |= static_cast<uint64_t>(1) << 46;
+    d |= static_cast<uint64_t>(2) << 61;
+    return d;
+}
+
+// kind::f16 instruction descriptor: BF16 x BF16 -> F32, both operands K-major
+// or (mn) both MN-major.
+__host__ __device__ constexpr uint32_t idesc_bf16_f32(int m, int n, bool mn = false) {
+    return (1u << 4) | (1u << 7) | (1u << 10) | (mn ? (1u << 15) | (1u << 16) : 0u) |
+           (static_cast<uint32_t>(n >> 3) << 17) | (static_cast<uint32_t>(m >> 4) << 24);
 }
 
 // SiLU through the hardware tanh (one special-function op):

@@ -329,54 +329,71 @@ cudaError_t launch_loss(const float* O, const float* Yb, int rows, LossWeights w
     return cudaGetLastError();
 }
 
-// 32x32 tiles through shared memory; out[c][r] = in[r][c]
-__global__ void transpose_kernel(const __nv_bfloat16* __restrict__ in, int rows, int cols, int ld_in,
-                                 __nv_bfloat16* __restrict__ out, int ld_out) {
-    __shared__ __nv_bfloat16 tile[32][33];
-    const int c0 = blockIdx.x * 32, r0 = blockIdx.y * 32;
-    for (int k = threadIdx.y; k < 32; k += blockDim.y) {
-        const int r = r0 + k, c = c0 + threadIdx.x;
-        tile[k][threadIdx.x] =
-            (r < rows && c < cols) ? in[static_cast<size_t>(r) * ld_in + c] : __float2bfloat16_rn(0.0f);
+// Column sums in row order are a chain of additions, so what a row costs is
+// its load's latency unless many rows are in flight: a block stages kTileRows
+// rows g, g + G, ... of a BF16 matrix (at most 256 columns, a multiple of 8) in
+// shared memory, the next ones in registers meanwhile (column sums of 16,384 x
+// 256: 117 -> 8 us on B200).
+constexpr int kTileRows = 32;
+constexpr int kRowChunks = kHidden / 8;                          // 16-byte pieces of the widest row
+constexpr int kTileLoads = kTileRows * kRowChunks / kHidden;     // per thread of kHidden
+struct RowTile {
+    __nv_bfloat16 v[kTileRows][kHidden];
+};
+struct RowTileLoader {
+    uint4 ahead[kTileLoads];
+    __device__ __forceinline__ void load(const __nv_bfloat16* A, int ld, int cols, int r0, int G, int rows) {
+#pragma unroll
+        for (int k = 0; k < kTileLoads; ++k) {
+            const int i = k * kHidden + threadIdx.x, row = r0 + (i / kRowChunks) * G, c = (i % kRowChunks) * 8;
+            if (row < rows && c < cols)
+                ahead[k] = *reinterpret_cast<const uint4*>(A + static_cast<size_t>(row) * ld + c);
+        }
     }
-    __syncthreads();
-    for (int k = threadIdx.y; k < 32; k += blockDim.y) {
-        const int c = c0 + k, r = r0 + threadIdx.x;
-        if (c < cols && r < rows) out[static_cast<size_t>(c) * ld_out + r] = tile[threadIdx.x][k];
+    __device__ __forceinline__ void store(RowTile& t) const {
+#pragma unroll
+        for (int k = 0; k < kTileLoads; ++k) {
+            const int i = k * kHidden + threadIdx.x;
+            *reinterpret_cast<uint4*>(&t.v[i / kRowChunks][(i % kRowChunks) * 8]) = ahead[k];
+        }
     }
-}
-
-cudaError_t launch_transpose(const __nv_bfloat16* in, int rows, int cols, int ld_in, __nv_bfloat16* out, int ld_out,
-                             cudaStream_t s) {
-    dim3 grid((cols + 31) / 32, (rows + 31) / 32), block(32, 8);
-    transpose_kernel<<<grid, block, 0, s>>>(in, rows, cols, ld_in, out, ld_out);
-    return cudaGetLastError();
-}
+};
 
 // partials[g][c] = sum of rows g, g + G, ... of column c
-__global__ void colsum_kernel(const __nv_bfloat16* __restrict__ A, int rows, int cols, int ld,
-                              float* __restrict__ partials) {
-    const int c = threadIdx.x;
-    if (c >= cols) return;
+__global__ void __launch_bounds__(kHidden)
+colsum_kernel(const __nv_bfloat16* __restrict__ A, int rows, int cols, int ld, float* __restrict__ partials) {
+    __shared__ RowTile tile;
+    const int c = threadIdx.x, G = static_cast<int>(gridDim.x);
+    RowTileLoader next;
+    next.load(A, ld, cols, blockIdx.x, G, rows);
     float acc = 0.0f;
-    for (int r = blockIdx.x; r < rows; r += gridDim.x) acc += __bfloat162float(A[static_cast<size_t>(r) * ld + c]);
-    partials[static_cast<size_t>(blockIdx.x) * cols + c] = acc;
+    for (int r0 = blockIdx.x; r0 < rows; r0 += kTileRows * G) {
+        next.store(tile);
+        __syncthreads();
+        next.load(A, ld, cols, r0 + kTileRows * G, G, rows);
+        const int n = min(kTileRows, (rows - r0 + G - 1) / G);
+        for (int k = 0; k < n; ++k) acc += __bfloat162float(tile.v[k][c]);
+        __syncthreads();
+    }
+    if (c < cols) partials[static_cast<size_t>(blockIdx.x) * cols + c] = acc;
 }
 
+// out[i] = sum over p of part[p][i], in order of p
 __global__ void reduce_rows_kernel(const float* __restrict__ part, int parts, size_t n, float* __restrict__ out) {
     const size_t i = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x;
     if (i >= n) return;
     float acc = 0.0f;
+#pragma unroll 16
     for (int p = 0; p < parts; ++p) acc += part[static_cast<size_t>(p) * n + i];
     out[i] = acc;
 }
 
 cudaError_t launch_colsum(const __nv_bfloat16* A, int rows, int cols, int ld, float* partials, int grid_parts,
                           float* out, cudaStream_t s) {
-    colsum_kernel<<<grid_parts, 256, 0, s>>>(A, rows, cols, ld, partials);
+    colsum_kernel<<<grid_parts, kHidden, 0, s>>>(A, rows, cols, ld, partials);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
-    reduce_rows_kernel<<<(cols + 255) / 256, 256, 0, s>>>(partials, grid_parts, static_cast<size_t>(cols), out);
+    reduce_rows_kernel<<<(cols + 127) / 128, 128, 0, s>>>(partials, grid_parts, static_cast<size_t>(cols), out);
     return cudaGetLastError();
 }
 
@@ -385,16 +402,34 @@ cudaError_t launch_colsum(const __nv_bfloat16* A, int rows, int cols, int ld, fl
 __global__ void __launch_bounds__(kHidden)
 layer1_bwd_kernel(const __nv_bfloat16* __restrict__ dZ1, const float* __restrict__ Xb, int rows,
                   float* __restrict__ partials) {
-    const int f = threadIdx.x;
+    __shared__ RowTile tile;
+    __shared__ float4 inputs[kTileRows];
+    const int f = threadIdx.x, G = static_cast<int>(gridDim.x);
+    RowTileLoader next;
+    float4 x_next = make_float4(0, 0, 0, 0);
+    auto load = [&](int r0) {
+        next.load(dZ1, kHidden, kHidden, r0, G, rows);
+        const int r = r0 + static_cast<int>(threadIdx.x) * G;
+        if (threadIdx.x < kTileRows && r < rows) x_next = *reinterpret_cast<const float4*>(Xb + static_cast<size_t>(r) * kIn);
+    };
+    load(blockIdx.x);
     float a0 = 0, a1 = 0, a2 = 0, a3 = 0, ab = 0;
-    for (int r = blockIdx.x; r < rows; r += gridDim.x) {
-        const float g = __bfloat162float(dZ1[static_cast<size_t>(r) * kHidden + f]);
-        const float* x = Xb + static_cast<size_t>(r) * kIn;
-        a0 += g * x[0];
-        a1 += g * x[1];
-        a2 += g * x[2];
-        a3 += g * x[3];
-        ab += g;
+    for (int r0 = blockIdx.x; r0 < rows; r0 += kTileRows * G) {
+        next.store(tile);
+        if (threadIdx.x < kTileRows) inputs[threadIdx.x] = x_next;
+        __syncthreads();
+        load(r0 + kTileRows * G);
+        const int n = min(kTileRows, (rows - r0 + G - 1) / G);
+        for (int k = 0; k < n; ++k) {
+            const float g = __bfloat162float(tile.v[k][f]);
+            const float4 x = inputs[k];
+            a0 += g * x.x;
+            a1 += g * x.y;
+            a2 += g * x.z;
+            a3 += g * x.w;
+            ab += g;
+        }
+        __syncthreads();
     }
     float* p = partials + static_cast<size_t>(blockIdx.x) * (kHidden * 5);
     p[f * 4 + 0] = a0;
@@ -410,7 +445,7 @@ cudaError_t launch_layer1_bwd(const __nv_bfloat16* dZ1, const float* Xb, int row
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
     static_assert(ParamLayout::b1 == ParamLayout::w1 + kHidden * kIn, "W1 and b1 are contiguous");
-    reduce_rows_kernel<<<(kHidden * 5 + 255) / 256, 256, 0, s>>>(partials, grid_parts, kHidden * 5,
+    reduce_rows_kernel<<<(kHidden * 5 + 127) / 128, 128, 0, s>>>(partials, grid_parts, kHidden * 5,
                                                                   grad + ParamLayout::w1);
     return cudaGetLastError();
 }
@@ -420,14 +455,16 @@ cudaError_t launch_reduce_splits(const float* part, int splits, size_t n, float*
     return cudaGetLastError();
 }
 
-__global__ void adam_begin_kernel(unsigned* step) { *step += 1; }
-
+// One optimiser step over parameter i: t = the number of this step (*step is
+// advanced by finish_step_kernel), the learning rate read from device memory so
+// that one captured graph serves every rate.
 __global__ void adam_kernel(float* __restrict__ p, const float* __restrict__ g, float* __restrict__ m,
-                            float* __restrict__ v, size_t n, const unsigned* step, float lr, float b1, float b2,
-                            float eps) {
+                            float* __restrict__ v, size_t n, const unsigned* step, const float* lr_ptr, float b1,
+                            float b2, float eps) {
     const size_t i = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x;
     if (i >= n) return;
-    const float t = static_cast<float>(*step);
+    const float lr = *lr_ptr;
+    const float t = static_cast<float>(*step + 1);
     const float c1 = 1.0f - powf(b1, t), c2 = 1.0f - powf(b2, t);
     const float gi = g[i];
     const float mi = b1 * m[i] + (1.0f - b1) * gi;
@@ -437,23 +474,28 @@ __global__ void adam_kernel(float* __restrict__ p, const float* __restrict__ g, 
     p[i] -= lr * (mi / c1) / (sqrtf(vi / c2) + eps);
 }
 
-cudaError_t launch_adam(float* params, const float* grad, float* m, float* v, size_t n, unsigned* step, float lr,
-                        float beta1, float beta2, float eps, cudaStream_t s) {
-    adam_begin_kernel<<<1, 1, 0, s>>>(step);
-    cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess) return e;
+cudaError_t launch_adam(float* params, const float* grad, float* m, float* v, size_t n, const unsigned* step,
+                        const float* lr, float beta1, float beta2, float eps, cudaStream_t s) {
     adam_kernel<<<static_cast<unsigned>((n + 255) / 256), 256, 0, s>>>(params, grad, m, v, n, step, lr, beta1, beta2,
                                                                        eps);
     return cudaGetLastError();
 }
 
-__global__ void record_loss_kernel(const float* loss, const unsigned* step, float* hist, int cap) {
-    const unsigned t = *step;  // already advanced by this step's optimiser update
-    if (t >= 1 && static_cast<int>(t - 1) < cap) hist[t - 1] = *loss;
+__global__ void finish_step_kernel(const float* loss, unsigned* step, float* hist, int cap) {
+    const unsigned t = *step;
+    if (static_cast<int>(t) < cap) hist[t] = *loss;
+    *step = t + 1;
 }
 
-cudaError_t launch_record_loss(const float* loss, const unsigned* step, float* hist, int cap, cudaStream_t s) {
-    record_loss_kernel<<<1, 1, 0, s>>>(loss, step, hist, cap);
+cudaError_t launch_finish_step(const float* loss, unsigned* step, float* hist, int cap, cudaStream_t s) {
+    finish_step_kernel<<<1, 1, 0, s>>>(loss, step, hist, cap);
+    return cudaGetLastError();
+}
+
+__global__ void set_float_kernel(float* p, float v) { *p = v; }
+
+cudaError_t launch_set_float(float* p, float v, cudaStream_t s) {
+    set_float_kernel<<<1, 1, 0, s>>>(p, v);
     return cudaGetLastError();
 }
 

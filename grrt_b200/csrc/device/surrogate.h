@@ -72,17 +72,17 @@ cudaError_t launch_layer1_fwd(const float* Xb, int rows, const float* params, fl
                               cudaStream_t s);
 cudaError_t launch_loss(const float* O, const float* Yb, int rows, LossWeights w, __nv_bfloat16* dO, float* loss,
                         cudaStream_t s);
-cudaError_t launch_transpose(const __nv_bfloat16* in, int rows, int cols, int ld_in, __nv_bfloat16* out, int ld_out,
-                             cudaStream_t s);
 // Column sums of a BF16 matrix into out[cols] (partials: grid_parts x cols floats).
 cudaError_t launch_colsum(const __nv_bfloat16* A, int rows, int cols, int ld, float* partials, int grid_parts,
                           float* out, cudaStream_t s);
 cudaError_t launch_layer1_bwd(const __nv_bfloat16* dZ1, const float* Xb, int rows, float* partials, int grid_parts,
                               float* grad, cudaStream_t s);
 cudaError_t launch_reduce_splits(const float* part, int splits, size_t n, float* out, cudaStream_t s);
-cudaError_t launch_adam(float* params, const float* grad, float* m, float* v, size_t n, unsigned* step, float lr,
-                        float beta1, float beta2, float eps, cudaStream_t s);
-cudaError_t launch_record_loss(const float* loss, const unsigned* step, float* hist, int cap, cudaStream_t s);
+cudaError_t launch_adam(float* params, const float* grad, float* m, float* v, size_t n, const unsigned* step,
+                        const float* lr, float beta1, float beta2, float eps, cudaStream_t s);
+// Records the step's loss at hist[*step] (below cap) and advances *step.
+cudaError_t launch_finish_step(const float* loss, unsigned* step, float* hist, int cap, cudaStream_t s);
+cudaError_t launch_set_float(float* p, float v, cudaStream_t s);
 // BF16 copies of the GEMM layers: wb[l] [out x in] and wt[l] [in x out]
 // (l = 2..4), w5b [16 x 256], w5t [256 x 64] (columns >= 16 left zero).
 cudaError_t launch_cast_weights(const float* params, __nv_bfloat16* const* wb, __nv_bfloat16* const* wt,

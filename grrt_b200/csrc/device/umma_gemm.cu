@@ -1,5 +1,7 @@
 // BF16 GEMM on the sm_100a tensor cores for the learned surrogate:
-//   C[M x N] = A[M x K] * B[N x K]^T   (A, B row-major BF16, i.e. K-major),
+//   C[M x N] = A[M x K] * B[N x K]^T   (A, B row-major BF16, i.e. K-major), or
+//   C[M x N] = A[K x M]^T * B[K x N]   (A, B row-major BF16, i.e. MN-major, the
+//   weight gradients: no transposed copies of the activations),
 // FP32 accumulation in tensor memory, with a fused epilogue (bias, SiLU,
 // SiLU-derivative gating, FP32/BF16 outputs, split-K partials).
 //
@@ -8,7 +10,9 @@
 //                  SWIZZLE_128B, completion on per-stage mbarriers);
 //   warp 1 lane 0: MMA issuer (4 x tcgen05.mma K=16 per stage, commit frees
 //                  the stage, a final commit signals the epilogue);
-//   warps 0-3:     epilogue, each warp reads its 32 TMEM lanes (= tile rows).
+//   warps 0-7:     epilogue, each warp reads the 32 TMEM lanes (= tile rows) of
+//                  its quadrant, warps 0-3 the even 16-column groups, 4-7 the odd.
+// The epilogue is most of a tile: read by rows, stored by 64-byte row pieces.
 // Every mbarrier wait is bounded; on timeout the CTA records an error code in
 // *err, waits (bounded) for its TMA copies in flight, frees its tensor memory
 // and returns.
@@ -32,7 +36,9 @@ namespace {
 constexpr int kBM = 128;
 constexpr int kBK = 64;
 constexpr int kStages = 4;
-constexpr int kThreads = 128;
+constexpr uint32_t kBoxBytes = 64 * kBK * 2;  // an MN-major TMA box
+constexpr int kThreads = 256;
+constexpr int kPieceRow = 20;  // floats a row of an epilogue piece takes in shared memory
 constexpr uint32_t kWaitLimit = 1u << 22;  // polls; a healthy wait needs a handful
 
 struct GemmSmem {
@@ -46,6 +52,8 @@ struct GemmSmem {
 __device__ __forceinline__ float silu(float z) { return sm100::silu_fast(z); }
 __device__ __forceinline__ float silu_grad(float z) { return sm100::silu_grad_fast(z); }
 
+// kMN: the operands are MN-major, a stage's tiles TMA boxes of 64 MN x kBK K.
+template <bool kMN>
 __global__ void __launch_bounds__(kThreads, 1)
 umma_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
                  const GemmEpilogue ep, int M, int N, int k_blocks_per_split, int k_blocks_total, int* err) {
@@ -87,7 +95,7 @@ umma_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
     __syncthreads();
     sm100::tc_fence_after();
     const uint32_t tmem = sh->tmem_base;
-    const uint32_t idesc = sm100::idesc_bf16_f32(kBM, N);
+    const uint32_t idesc = sm100::idesc_bf16_f32(kBM, N, kMN);
 
     int issued = 0;  // producer: stages handed to TMA
     if (warp == 0 && lane == 0 && nk > 0) {
@@ -101,8 +109,15 @@ umma_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
             unsigned char* b_dst = a_dst + a_bytes;
             sm100::mbar_arrive_expect_tx(&sh->full[s], stage_bytes);
             const int kx = (kb0 + i) * kBK;
-            sm100::tma_load_2d(a_dst, &tmap_a, &sh->full[s], kx, m0);
-            sm100::tma_load_2d(b_dst, &tmap_b, &sh->full[s], kx, 0);
+            if (kMN) {
+                for (int j = 0; j < kBM / 64; ++j)
+                    sm100::tma_load_2d(a_dst + j * kBoxBytes, &tmap_a, &sh->full[s], m0 + 64 * j, kx);
+                for (int j = 0; j < N / 64; ++j)
+                    sm100::tma_load_2d(b_dst + j * kBoxBytes, &tmap_b, &sh->full[s], 64 * j, kx);
+            } else {
+                sm100::tma_load_2d(a_dst, &tmap_a, &sh->full[s], kx, m0);
+                sm100::tma_load_2d(b_dst, &tmap_b, &sh->full[s], kx, 0);
+            }
             ++issued;
         }
     } else if (warp == 1 && lane == 0) {
@@ -116,12 +131,14 @@ umma_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
             sm100::tc_fence_after();
             const uint32_t a_addr = sm100::smem_u32(tiles + s * stage_bytes);
             const uint32_t b_addr = a_addr + a_bytes;
-            const uint64_t da = sm100::desc_kmajor_sw128(a_addr), db = sm100::desc_kmajor_sw128(b_addr);
+            const uint64_t da = kMN ? sm100::desc_mnmajor_sw128(a_addr, kBoxBytes) : sm100::desc_kmajor_sw128(a_addr);
+            const uint64_t db = kMN ? sm100::desc_mnmajor_sw128(b_addr, kBoxBytes) : sm100::desc_kmajor_sw128(b_addr);
+            // 16 along K per step: 32 bytes of a K-major row, 16 rows of 128
+            // bytes MN-major; the start-address field counts 16-byte units
+            constexpr int kStep = kMN ? 16 * 128 / 16 : 2;
 #pragma unroll
-            for (int k = 0; k < kBK / 16; ++k) {
-                // +32 bytes along K per step: start-address field counts 16-byte units
-                sm100::umma_f16(tmem, da + 2 * k, db + 2 * k, idesc, (i > 0 || k > 0) ? 1u : 0u);
-            }
+            for (int k = 0; k < kBK / 16; ++k)
+                sm100::umma_f16(tmem, da + kStep * k, db + kStep * k, idesc, (i > 0 || k > 0) ? 1u : 0u);
             sm100::umma_commit(&sh->empty[s]);
         }
         sm100::umma_commit(&sh->done);  // also completes when nothing was issued
@@ -134,47 +151,71 @@ umma_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
     sm100::tc_fence_after();
     __syncthreads();
     const bool good = (*reinterpret_cast<volatile int*>(&sh->failed) == 0);
-    const int row = m0 + warp * 32 + lane;
+    const int quad = warp & 3;  // the TMEM lanes a warp may read
     if (good) {
-        const uint32_t t_row = tmem + (static_cast<uint32_t>(warp * 32) << 16);
+        // Every stage has been consumed (the commit on `done` follows all MMAs), so
+        // each warp turns its 32 x 16 pieces round in its part of the ring: a
+        // lane reads a row of the accumulator, but 4 lanes store 64 consecutive
+        // bytes of a row (padded rows of 20 floats: no bank conflicts).
+        float* const piece = reinterpret_cast<float*>(tiles) + warp * (32 * kPieceRow);
+        const uint32_t t_row = tmem + (static_cast<uint32_t>(quad * 32) << 16);
         const size_t zoff = ep.split_stride * static_cast<size_t>(split);
-        for (int c0 = 0; c0 < N; c0 += 16) {
+        const bool wide = ((reinterpret_cast<uintptr_t>(ep.gate_z) | (static_cast<size_t>(ep.ld_gate) * 4)) & 15) == 0;
+        const int sub = lane >> 2, col4 = (lane & 3) * 4;  // of the row groups of 8: row and columns this lane moves
+        const int row0 = m0 + quad * 32 + sub;
+        for (int c0 = 16 * (warp >> 2); c0 < N; c0 += 32) {
+            float4 z[4], bias = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            if (ep.gate_z) {  // in flight while the accumulator is read
+#pragma unroll
+                for (int g = 0; g < 4; ++g) {
+                    const int r = row0 + 8 * g;
+                    if (r >= M) continue;
+                    const float* zp = ep.gate_z + static_cast<size_t>(r) * ep.ld_gate + c0 + col4;
+                    z[g] = wide ? *reinterpret_cast<const float4*>(zp) : make_float4(zp[0], zp[1], zp[2], zp[3]);
+                }
+            }
+            if (ep.bias) {
+                const float* bp = ep.bias + c0 + col4;
+                bias = make_float4(bp[0], bp[1], bp[2], bp[3]);
+            }
             float v[16];
             sm100::tmem_ld16(t_row + static_cast<uint32_t>(c0), v);
             if (nk <= 0) {
 #pragma unroll
                 for (int j = 0; j < 16; ++j) v[j] = 0.0f;
             }
-            if (row >= M) continue;
-            if (ep.bias) {
 #pragma unroll
-                for (int j = 0; j < 16; ++j) v[j] += ep.bias[c0 + j];
-            }
-            if (ep.gate_z) {  // backward through SiLU: v *= silu'(z)
-                const float* z = ep.gate_z + static_cast<size_t>(row) * ep.ld_gate + c0;
+            for (int j = 0; j < 16; j += 4)
+                *reinterpret_cast<float4*>(piece + lane * kPieceRow + j) = make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]);
+            __syncwarp();
 #pragma unroll
-                for (int j = 0; j < 16; ++j) v[j] *= silu_grad(z[j]);
-            }
-            if (ep.out_f32) {
-                float* o = ep.out_f32 + zoff + static_cast<size_t>(row) * ep.ld_f32 + c0;
-#pragma unroll
-                for (int j = 0; j < 16; j += 4) *reinterpret_cast<float4*>(o + j) = make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]);
-            }
-            if (ep.out_bf16) {
-                __nv_bfloat16* o = ep.out_bf16 + static_cast<size_t>(row) * ep.ld_bf16 + c0;
-                alignas(16) __nv_bfloat162 h[8];
-#pragma unroll
-                for (int j = 0; j < 8; ++j) {
-                    float x0 = v[2 * j], x1 = v[2 * j + 1];
-                    if (ep.act == kActSilu) {
-                        x0 = silu(x0);
-                        x1 = silu(x1);
-                    }
-                    h[j] = __floats2bfloat162_rn(x0, x1);
+            for (int g = 0; g < 4; ++g) {
+                const int r = row0 + 8 * g;
+                if (r >= M) continue;
+                float4 x = *reinterpret_cast<const float4*>(piece + (sub + 8 * g) * kPieceRow + col4);
+                if (ep.bias) {
+                    x.x += bias.x;
+                    x.y += bias.y;
+                    x.z += bias.z;
+                    x.w += bias.w;
                 }
-                *reinterpret_cast<uint4*>(o) = *reinterpret_cast<const uint4*>(&h[0]);
-                *reinterpret_cast<uint4*>(o + 8) = *reinterpret_cast<const uint4*>(&h[4]);
+                if (ep.gate_z) {  // backward through SiLU: x *= silu'(z)
+                    x.x *= silu_grad(z[g].x);
+                    x.y *= silu_grad(z[g].y);
+                    x.z *= silu_grad(z[g].z);
+                    x.w *= silu_grad(z[g].w);
+                }
+                if (ep.out_f32)
+                    *reinterpret_cast<float4*>(ep.out_f32 + zoff + static_cast<size_t>(r) * ep.ld_f32 + c0 + col4) = x;
+                if (ep.out_bf16) {
+                    if (ep.act == kActSilu) x = make_float4(silu(x.x), silu(x.y), silu(x.z), silu(x.w));
+                    alignas(8) const __nv_bfloat162 h[2] = {__floats2bfloat162_rn(x.x, x.y),
+                                                            __floats2bfloat162_rn(x.z, x.w)};
+                    *reinterpret_cast<uint2*>(ep.out_bf16 + static_cast<size_t>(r) * ep.ld_bf16 + c0 + col4) =
+                        *reinterpret_cast<const uint2*>(h);
+                }
             }
+            __syncwarp();  // the piece is free again
         }
     }
     if (!good && threadIdx.x == 0) {
@@ -222,18 +263,19 @@ size_t umma_gemm_smem_bytes(int N) {
     return 1024 + static_cast<size_t>(kStages) * (kBM * kBK * 2 + static_cast<size_t>(N) * kBK * 2) + sizeof(GemmSmem);
 }
 
-cudaError_t umma_gemm_bf16(const __nv_bfloat16* A, int lda, const __nv_bfloat16* B, int ldb, int M, int N, int K,
-                           int splits, const GemmEpilogue& ep, int* d_err, cudaStream_t stream) {
-    // shapes the kernel supports; everything else is a caller error
-    if (M <= 0 || N < 16 || N > 256 || (N % 16) != 0 || K <= 0 || (K % kBK) != 0 || splits < 1) return cudaErrorInvalidValue;
-    if ((lda % 8) != 0 || (ldb % 8) != 0 || lda < K || ldb < K) return cudaErrorInvalidValue;
-    if ((reinterpret_cast<uintptr_t>(A) & 15) || (reinterpret_cast<uintptr_t>(B) & 15)) return cudaErrorInvalidValue;
-    if (ep.out_bf16 && ((ep.ld_bf16 % 8) != 0 || (reinterpret_cast<uintptr_t>(ep.out_bf16) & 15))) return cudaErrorInvalidValue;
-    if (ep.out_f32 && ((ep.ld_f32 % 4) != 0 || (reinterpret_cast<uintptr_t>(ep.out_f32) & 15))) return cudaErrorInvalidValue;
-    if (splits > 1 && (ep.out_bf16 || ep.bias || ep.gate_z || !ep.out_f32 || ep.split_stride == 0))
-        return cudaErrorInvalidValue;  // split-K writes raw FP32 partials only
-    CUtensorMap ta, tb;
-    if (!make_tmap(&ta, A, M, K, lda, kBM) || !make_tmap(&tb, B, N, K, ldb, N)) return cudaErrorInvalidValue;
+namespace {
+
+// Outputs and gate of a GEMM of N columns: 16-byte accesses.
+bool epilogue_ok(const GemmEpilogue& ep, int splits) {
+    if (ep.out_bf16 && ((ep.ld_bf16 % 8) != 0 || (reinterpret_cast<uintptr_t>(ep.out_bf16) & 15))) return false;
+    if (ep.out_f32 && ((ep.ld_f32 % 4) != 0 || (reinterpret_cast<uintptr_t>(ep.out_f32) & 15))) return false;
+    // split-K writes raw FP32 partials only
+    return splits == 1 || !(ep.out_bf16 || ep.bias || ep.gate_z || !ep.out_f32 || ep.split_stride == 0);
+}
+
+template <bool kMN>
+cudaError_t launch(const CUtensorMap& ta, const CUtensorMap& tb, int M, int N, int K, int splits,
+                   const GemmEpilogue& ep, int* d_err, cudaStream_t stream) {
     const int kbt = K / kBK;
     const int per = (kbt + splits - 1) / splits;
     splits = (kbt + per - 1) / per;  // every split gets at least one K-block
@@ -244,14 +286,39 @@ cudaError_t umma_gemm_bf16(const __nv_bfloat16* A, int lda, const __nv_bfloat16*
     };
     const Attr& attr = per_device_shape<Attr>([](int) {
         Attr a;
-        a.err = cudaFuncSetAttribute(umma_gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        a.err = cudaFuncSetAttribute(umma_gemm_kernel<kMN>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      static_cast<int>(umma_gemm_smem_bytes(256)));
         return a;
     });
     if (attr.err != cudaSuccess) return attr.err;
     dim3 grid((M + kBM - 1) / kBM, splits);
-    umma_gemm_kernel<<<grid, kThreads, smem, stream>>>(ta, tb, ep, M, N, per, kbt, d_err);
+    umma_gemm_kernel<kMN><<<grid, kThreads, smem, stream>>>(ta, tb, ep, M, N, per, kbt, d_err);
     return cudaGetLastError();
+}
+
+}  // namespace
+
+cudaError_t umma_gemm_bf16(const __nv_bfloat16* A, int lda, const __nv_bfloat16* B, int ldb, int M, int N, int K,
+                           int splits, const GemmEpilogue& ep, int* d_err, cudaStream_t stream) {
+    // shapes the kernel supports; everything else is a caller error
+    if (M <= 0 || N < 16 || N > 256 || (N % 16) != 0 || K <= 0 || (K % kBK) != 0 || splits < 1) return cudaErrorInvalidValue;
+    if ((lda % 8) != 0 || (ldb % 8) != 0 || lda < K || ldb < K) return cudaErrorInvalidValue;
+    if ((reinterpret_cast<uintptr_t>(A) & 15) || (reinterpret_cast<uintptr_t>(B) & 15)) return cudaErrorInvalidValue;
+    if (!epilogue_ok(ep, splits)) return cudaErrorInvalidValue;
+    CUtensorMap ta, tb;
+    if (!make_tmap(&ta, A, M, K, lda, kBM) || !make_tmap(&tb, B, N, K, ldb, N)) return cudaErrorInvalidValue;
+    return launch<false>(ta, tb, M, N, K, splits, ep, d_err, stream);
+}
+
+cudaError_t umma_gemm_tn_bf16(const __nv_bfloat16* A, int lda, const __nv_bfloat16* B, int ldb, int M, int N, int K,
+                              int splits, const GemmEpilogue& ep, int* d_err, cudaStream_t stream) {
+    if (M <= 0 || N < 64 || N > 256 || (N % 64) != 0 || K <= 0 || (K % kBK) != 0 || splits < 1) return cudaErrorInvalidValue;
+    if ((lda % 8) != 0 || (ldb % 8) != 0 || lda < M || ldb < N) return cudaErrorInvalidValue;
+    if ((reinterpret_cast<uintptr_t>(A) & 15) || (reinterpret_cast<uintptr_t>(B) & 15)) return cudaErrorInvalidValue;
+    if (!epilogue_ok(ep, splits)) return cudaErrorInvalidValue;
+    CUtensorMap ta, tb;  // boxes of 64 columns x kBK rows; columns past M read as zero
+    if (!make_tmap(&ta, A, K, M, lda, kBK) || !make_tmap(&tb, B, K, N, ldb, kBK)) return cudaErrorInvalidValue;
+    return launch<true>(ta, tb, M, N, K, splits, ep, d_err, stream);
 }
 
 }  // namespace grrt_b200

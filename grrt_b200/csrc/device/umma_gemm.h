@@ -33,6 +33,10 @@ struct GemmEpilogue {
 // written). *d_err (device int) receives a non-zero code if a CTA timed out.
 cudaError_t umma_gemm_bf16(const __nv_bfloat16* A, int lda, const __nv_bfloat16* B, int ldb, int M, int N, int K,
                            int splits, const GemmEpilogue& ep, int* d_err, cudaStream_t stream);
+// C = A^T * B of A: [K x M] (pitch lda), B: [K x N] (pitch ldb), row-major; N a
+// multiple of 64, the rest as above.
+cudaError_t umma_gemm_tn_bf16(const __nv_bfloat16* A, int lda, const __nv_bfloat16* B, int ldb, int M, int N, int K,
+                              int splits, const GemmEpilogue& ep, int* d_err, cudaStream_t stream);
 size_t umma_gemm_smem_bytes(int N);
 
 }  // namespace grrt_b200

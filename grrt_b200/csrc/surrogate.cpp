@@ -4,7 +4,8 @@
 // Training: layer 1 (K = 4) runs on the CUDA cores; layers 2-5 and every
 // backward GEMM run on the tensor cores through umma_gemm_bf16 (tcgen05, FP32
 // accumulation in TMEM). A training step is captured once as a CUDA graph and
-// replayed. Inference: one fused tensor-core kernel (mlp_fused.cu).
+// replayed; the weight gradients and bias sums run on two side streams beside
+// the chain of the activations' gradients. Inference: one fused tensor-core kernel (mlp_fused.cu).
 //
 // Rendering: per sample, the camera ray's closed-form margins (capture,
 // graze) and the network's outputs decide the colour. A sample whose
@@ -63,11 +64,16 @@ thread_local std::string g_surr_error;
 struct GRRTSurrogate {
     int device = -1;
     cudaStream_t stream = nullptr;
+    // the weight gradients and the bias sums of a training step, beside the
+    // chain of the activations' gradients on `stream`
+    cudaStream_t side[2] = {};
+    cudaEvent_t ev_fork = nullptr, ev_join[2] = {};
     std::string error;
 
     // parameters (FP32 master), gradients, Adam moments, step counter
     float *d_params = nullptr, *d_grad = nullptr, *d_m = nullptr, *d_v = nullptr;
     unsigned* d_step = nullptr;
+    float* d_lr = nullptr;
     __nv_bfloat16 *d_wb[3] = {}, *d_wt[3] = {}, *d_w5b = nullptr, *d_w5t = nullptr;
     int* d_err = nullptr;
     DevStats* d_stats = nullptr;
@@ -79,10 +85,10 @@ struct GRRTSurrogate {
 
     // training workspace for one batch size
     int ws_batch = 0, splits = 1;
-    float *Xb = nullptr, *Yb = nullptr, *Z[4] = {}, *O = nullptr, *part = nullptr, *colpart = nullptr;
+    float *Xb = nullptr, *Yb = nullptr, *Z[4] = {}, *O = nullptr, *part = nullptr, *colpart = nullptr, *l1part = nullptr;
     float *loss = nullptr, *loss_hist = nullptr;
     int hist_cap = 0;
-    __nv_bfloat16 *H[4] = {}, *dO = nullptr, *dZ[4] = {}, *TA = nullptr, *TB = nullptr;
+    __nv_bfloat16 *H[4] = {}, *dO = nullptr, *dZ[4] = {};
     static constexpr int kColParts = 64;
 
     // inference workspace
@@ -104,13 +110,16 @@ struct GRRTSurrogate {
 
     ~GRRTSurrogate() {
         if (device >= 0) cudaSetDevice(device);
-        if (stream) cudaStreamSynchronize(stream);
+        for (cudaStream_t q : {stream, side[0], side[1]})
+            if (q) cudaStreamSynchronize(q);
         free_workspace();
+        dfree(loss_hist);
         free_inference();
         for (auto* p : {d_params, d_grad, d_m, d_v, d_X, d_Y}) {
             if (p) cudaFree(p);
         }
         dfree(d_step);
+        dfree(d_lr);
         for (int l = 0; l < 3; ++l) {
             dfree(d_wb[l]);
             dfree(d_wt[l]);
@@ -120,7 +129,10 @@ struct GRRTSurrogate {
         dfree(d_err);
         dfree(d_stats);
         dfree(d_queue);
-        if (stream) cudaStreamDestroy(stream);
+        for (cudaEvent_t e : {ev_fork, ev_join[0], ev_join[1]})
+            if (e) cudaEventDestroy(e);
+        for (cudaStream_t q : {stream, side[0], side[1]})
+            if (q) cudaStreamDestroy(q);
     }
 
     bool fail(cudaError_t e, const char* what) {
@@ -146,16 +158,14 @@ struct GRRTSurrogate {
         dfree(O);
         dfree(part);
         dfree(colpart);
+        dfree(l1part);
         dfree(loss);
-        dfree(loss_hist);
         for (int l = 0; l < 4; ++l) {
             dfree(Z[l]);
             dfree(H[l]);
             dfree(dZ[l]);
         }
         dfree(dO);
-        dfree(TA);
-        dfree(TB);
         ws_batch = 0;
     }
     void free_inference() {
@@ -184,7 +194,7 @@ struct GRRTSurrogate {
         if (fail(cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking), "cudaStreamCreate")) return false;
         const size_t P = ParamLayout::total;
         if (!dalloc(&d_params, P) || !dalloc(&d_grad, P) || !dalloc(&d_m, P) || !dalloc(&d_v, P) ||
-            !dalloc(&d_step, 1) || !dalloc(&d_err, 1) || !dalloc(&d_stats, 1) || !dalloc(&d_queue, 1))
+            !dalloc(&d_step, 1) || !dalloc(&d_lr, 1) || !dalloc(&d_err, 1) || !dalloc(&d_stats, 1) || !dalloc(&d_queue, 1))
             return !fail_msg("cudaMalloc(surrogate parameters) failed");
         for (int l = 0; l < 3; ++l)
             if (!dalloc(&d_wb[l], kHidden * kHidden) || !dalloc(&d_wt[l], kHidden * kHidden))
@@ -292,13 +302,18 @@ struct GRRTSurrogate {
     // ---- training ------------------------------------------------------------
     bool ensure_workspace(int B) {
         if (ws_batch == B) return true;
+        for (cudaStream_t& q : side)
+            if (!q && fail(cudaStreamCreateWithFlags(&q, cudaStreamNonBlocking), "cudaStreamCreate")) return false;
+        for (cudaEvent_t* e : {&ev_fork, &ev_join[0], &ev_join[1]})
+            if (!*e && fail(cudaEventCreateWithFlags(e, cudaEventDisableTiming), "cudaEventCreate")) return false;
         free_workspace();
         const size_t b = static_cast<size_t>(B);
         splits = std::max(1, std::min(32, B / 64 / 4));
         bool ok = dalloc(&Xb, b * kIn) && dalloc(&Yb, b * kYCols) && dalloc(&O, b * kOutPad) &&
                   dalloc(&part, static_cast<size_t>(splits) * kHidden * kHidden) &&
-                  dalloc(&colpart, static_cast<size_t>(kColParts) * kHidden * 5) && dalloc(&loss, 1) &&
-                  dalloc(&dO, b * kDOutPad) && dalloc(&TA, b * kHidden) && dalloc(&TB, b * kHidden);
+                  dalloc(&colpart, static_cast<size_t>(kColParts) * kHidden) &&
+                  dalloc(&l1part, static_cast<size_t>(kColParts) * kHidden * 5) && dalloc(&loss, 1) &&
+                  dalloc(&dO, b * kDOutPad);
         for (int l = 0; l < 4 && ok; ++l)
             ok = dalloc(&Z[l], b * kHidden) && dalloc(&H[l], b * kHidden) && dalloc(&dZ[l], b * kHidden);
         if (!ok) {
@@ -317,9 +332,31 @@ struct GRRTSurrogate {
         return (kbt + per - 1) / per;
     }
 
-    // Forward + loss + backward of the batch in Xb/Yb; gradients into d_grad.
+    // The work enqueued on `to` so far comes before what `from`'s next work is.
+    bool order(cudaStream_t from, cudaStream_t to, cudaEvent_t ev) {
+        return !fail(cudaEventRecord(ev, to), "event") && !fail(cudaStreamWaitEvent(from, ev, 0), "event");
+    }
+
+    // dW = dY^T X and db = the column sums of dY, over the batch, on the side
+    // streams: dY [B x ld_y] with `outs` columns used, X [B x 256].
+    bool enqueue_weight_gradient(const __nv_bfloat16* dY, int ld_y, int outs, const __nv_bfloat16* X, int B,
+                                 size_t w_off, size_t b_off) {
+        if (!order(side[0], stream, ev_fork) || !order(side[1], stream, ev_fork)) return false;
+        GemmEpilogue ep;
+        ep.out_f32 = part;
+        ep.ld_f32 = kHidden;
+        ep.split_stride = static_cast<size_t>(outs) * kHidden;
+        return !fail(umma_gemm_tn_bf16(dY, ld_y, X, kHidden, outs, kHidden, B, splits, ep, d_err, side[0]),
+                     "tensor-core GEMM") &&
+               !fail(launch_reduce_splits(part, effective_splits(B), static_cast<size_t>(outs) * kHidden,
+                                          d_grad + w_off, side[0]),
+                     "reduce") &&
+               !fail(launch_colsum(dY, B, outs, ld_y, colpart, kColParts, d_grad + b_off, side[1]), "colsum");
+    }
+
+    // Forward + loss + backward of the batch in Xb/Yb; gradients into d_grad
+    // (all of it). What follows on `stream` comes after the side streams' part.
     bool enqueue_fwd_bwd(int B) {
-        const size_t P = ParamLayout::total;
         if (fail(launch_layer1_fwd(Xb, B, d_params, Z[0], H[0], stream), "layer 1")) return false;
         for (int l = 2; l <= 4; ++l) {
             GemmEpilogue ep;
@@ -339,25 +376,9 @@ struct GRRTSurrogate {
             if (!gemm(H[3], kHidden, d_w5b, kHidden, B, kOutPad, kHidden, 1, ep)) return false;
         }
         if (fail(cudaMemsetAsync(loss, 0, sizeof(float), stream), "memset")) return false;
-        if (fail(cudaMemsetAsync(d_grad, 0, P * sizeof(float), stream), "memset")) return false;
         if (fail(launch_loss(O, Yb, B, weights, dO, loss, stream), "loss")) return false;
         // output layer: dW5 = dO^T H4, db5 = colsum(dO), dZ4 = (dO W5) * silu'(Z4)
-        if (fail(launch_transpose(dO, B, kOutPad, kDOutPad, TA, B, stream), "transpose")) return false;
-        if (fail(launch_transpose(H[3], B, kHidden, kHidden, TB, B, stream), "transpose")) return false;
-        {
-            GemmEpilogue ep;
-            ep.out_f32 = part;
-            ep.ld_f32 = kHidden;
-            ep.split_stride = static_cast<size_t>(kOutPad) * kHidden;
-            if (!gemm(TA, B, TB, B, kOutPad, kHidden, B, splits, ep)) return false;
-            if (fail(launch_reduce_splits(part, effective_splits(B), static_cast<size_t>(kOutPad) * kHidden,
-                                          d_grad + ParamLayout::w5, stream),
-                     "reduce"))
-                return false;
-        }
-        if (fail(launch_colsum(dO, B, kOutPad, kDOutPad, colpart, kColParts, d_grad + ParamLayout::b5, stream),
-                 "colsum"))
-            return false;
+        if (!enqueue_weight_gradient(dO, kDOutPad, kOutPad, H[3], B, ParamLayout::w5, ParamLayout::b5)) return false;
         {
             GemmEpilogue ep;
             ep.gate_z = Z[3];
@@ -368,20 +389,8 @@ struct GRRTSurrogate {
         }
         for (int l = 4; l >= 2; --l) {
             // dW_l = dZ_l^T H_{l-1}, db_l = colsum(dZ_l), dZ_{l-1} = (dZ_l W_l) * silu'(Z_{l-1})
-            if (fail(launch_transpose(dZ[l - 1], B, kHidden, kHidden, TA, B, stream), "transpose")) return false;
-            if (fail(launch_transpose(H[l - 2], B, kHidden, kHidden, TB, B, stream), "transpose")) return false;
-            GemmEpilogue ep;
-            ep.out_f32 = part;
-            ep.ld_f32 = kHidden;
-            ep.split_stride = static_cast<size_t>(kHidden) * kHidden;
-            if (!gemm(TA, B, TB, B, kHidden, kHidden, B, splits, ep)) return false;
-            if (fail(launch_reduce_splits(part, effective_splits(B), static_cast<size_t>(kHidden) * kHidden,
-                                          d_grad + ParamLayout::w(l), stream),
-                     "reduce"))
-                return false;
-            if (fail(launch_colsum(dZ[l - 1], B, kHidden, kHidden, colpart, kColParts, d_grad + ParamLayout::b(l),
-                                   stream),
-                     "colsum"))
+            if (!enqueue_weight_gradient(dZ[l - 1], kHidden, kHidden, H[l - 2], B, ParamLayout::w(l),
+                                         ParamLayout::b(l)))
                 return false;
             GemmEpilogue eb;
             eb.gate_z = Z[l - 2];
@@ -390,79 +399,78 @@ struct GRRTSurrogate {
             eb.ld_bf16 = kHidden;
             if (!gemm(dZ[l - 1], kHidden, d_wt[l - 2], kHidden, B, kHidden, kHidden, 1, eb)) return false;
         }
-        return !fail(launch_layer1_bwd(dZ[0], Xb, B, colpart, kColParts, d_grad, stream), "layer 1 backward");
+        if (fail(launch_layer1_bwd(dZ[0], Xb, B, l1part, kColParts, d_grad, stream), "layer 1 backward")) return false;
+        return order(stream, side[0], ev_join[0]) && order(stream, side[1], ev_join[1]);
     }
 
-    bool enqueue_train_step(int B, float lr) {
-        if (fail(launch_gather(d_X, d_Y, n_data, B, d_step, Xb, Yb, stream), "gather")) return false;
-        if (!enqueue_fwd_bwd(B)) return false;
-        if (fail(launch_adam(d_params, d_grad, d_m, d_v, ParamLayout::total, d_step, lr, 0.9f, 0.999f, 1e-8f, stream),
-                 "adam"))
-            return false;
-        if (fail(launch_record_loss(loss, d_step, loss_hist, hist_cap, stream), "record loss")) return false;
-        return !fail(launch_cast_weights(d_params, d_wb, d_wt, d_w5b, d_w5t, stream), "cast weights");
+    bool enqueue_train_step(int B) {
+        return !fail(launch_gather(d_X, d_Y, n_data, B, d_step, Xb, Yb, stream), "gather") && enqueue_fwd_bwd(B) &&
+               !fail(launch_adam(d_params, d_grad, d_m, d_v, ParamLayout::total, d_step, d_lr, 0.9f, 0.999f, 1e-8f,
+                                 stream),
+                     "adam") &&
+               !fail(launch_finish_step(loss, d_step, loss_hist, hist_cap, stream), "record loss") &&
+               !fail(launch_cast_weights(d_params, d_wb, d_wt, d_w5b, d_w5t, stream), "cast weights");
     }
 
     // `steps` Adam steps at batch B. Learning rate: lr for the first half, then
-    // halved every eighth of the run (piecewise constant, one graph per rate).
+    // halved every eighth of the run (piecewise constant).
     bool train(int steps, int B, double lr, float* loss_out) {
         if (n_data == 0) return !fail_msg("no training set: call grrt_surrogate_generate first");
         if (steps <= 0 || B < 128 || B % 128 != 0 || B > (1 << 20)) return !fail_msg("bad steps or batch size");
         cudaSetDevice(device);
         if (!ensure_workspace(B)) return false;
-        dfree(loss_hist);
-        hist_cap = 0;
         unsigned t0 = 0;
         if (fail(copy(&t0, d_step, sizeof(unsigned), cudaMemcpyDeviceToHost), "read step")) return false;
         // the loss history is indexed by the global step counter
-        hist_cap = static_cast<int>(t0) + steps;
-        if (!dalloc(&loss_hist, static_cast<size_t>(hist_cap))) return !fail_msg("cudaMalloc(loss history)");
-        int done = 0;
+        const int need = static_cast<int>(t0) + steps;
+        if (hist_cap < need) {
+            dfree(loss_hist);
+            hist_cap = 0;
+            if (!dalloc(&loss_hist, static_cast<size_t>(need))) return !fail_msg("cudaMalloc(loss history)");
+            hist_cap = need;
+        }
+        // one eager step (it also sets the kernels' launch attributes), then one graph for all rates
+        cudaGraphExec_t ge = nullptr;
         const int phases[] = {steps / 2, steps / 8, steps / 8, steps / 8, steps - steps / 2 - 3 * (steps / 8)};
         double rate = lr;
-        for (int ph = 0; ph < 5; ++ph, rate *= 0.5) {
+        bool ok = true, first = true;
+        for (int ph = 0; ok && ph < 5; ++ph, rate *= 0.5) {
             int n = phases[ph];
             if (n <= 0) continue;
-            // one eager step (it also sets the kernels' launch attributes), then a graph
-            if (!enqueue_train_step(B, static_cast<float>(rate))) return false;
-            --n;
-            ++done;
-            if (n > 0) {
-                cudaGraph_t g = nullptr;
-                cudaGraphExec_t ge = nullptr;
-                if (fail(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal), "begin capture"))
-                    return false;
-                const bool ok = enqueue_train_step(B, static_cast<float>(rate));
-                const cudaError_t ce = cudaStreamEndCapture(stream, &g);
-                if (!ok || fail(ce, "end capture")) {
-                    if (g) cudaGraphDestroy(g);
-                    return false;
-                }
-                const cudaError_t ie = cudaGraphInstantiate(&ge, g, 0);
-                cudaGraphDestroy(g);
-                if (fail(ie, "graph instantiate")) return false;
-                for (int i = 0; i < n; ++i) {
-                    if (fail(cudaGraphLaunch(ge, stream), "graph launch")) {
-                        cudaGraphExecDestroy(ge);
-                        return false;
-                    }
-                }
-                done += n;
-                const cudaError_t se = cudaStreamSynchronize(stream);
-                cudaGraphExecDestroy(ge);
-                if (fail(se, "training")) return false;
+            ok = !fail(launch_set_float(d_lr, static_cast<float>(rate), stream), "learning rate");
+            if (ok && first) {
+                ok = enqueue_train_step(B);
+                first = false;
+                --n;
             }
-            if (!check_gemm_errors()) return false;
+            if (ok && n > 0 && !ge) ok = capture_train_step(B, &ge);
+            for (int i = 0; ok && i < n; ++i) ok = !fail(cudaGraphLaunch(ge, stream), "graph launch");
         }
-        if (fail(cudaStreamSynchronize(stream), "training")) return false;
+        const cudaError_t se = cudaStreamSynchronize(stream);
+        if (ge) cudaGraphExecDestroy(ge);
+        if (!ok || fail(se, "training")) return false;
         std::vector<float> hist(static_cast<size_t>(steps));
         if (fail(copy(hist.data(), loss_hist + t0, sizeof(float) * steps, cudaMemcpyDeviceToHost), "read loss"))
             return false;
         if (loss_out) std::memcpy(loss_out, hist.data(), sizeof(float) * steps);
         last_loss = hist.back();
-        steps_done += done;
+        steps_done += steps;
         calibrated = false;
         return check_gemm_errors();
+    }
+
+    bool capture_train_step(int B, cudaGraphExec_t* ge) {
+        cudaGraph_t g = nullptr;
+        if (fail(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal), "begin capture")) return false;
+        const bool ok = enqueue_train_step(B);
+        const cudaError_t ce = cudaStreamEndCapture(stream, &g);
+        if (!ok || fail(ce, "end capture")) {
+            if (g) cudaGraphDestroy(g);
+            return false;
+        }
+        const cudaError_t ie = cudaGraphInstantiate(ge, g, 0);
+        cudaGraphDestroy(g);
+        return !fail(ie, "graph instantiate");
     }
 
     // ---- inference -----------------------------------------------------------
