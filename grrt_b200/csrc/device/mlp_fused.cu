@@ -2,7 +2,8 @@
 // persistent kernel computes out[n x 16] = network(X[n x 4]) with the hidden
 // activations kept in shared memory between layers.
 //
-// Per 128-row tile:
+// Per 128-row tile (what bounds it: the epilogue, special-function pipe 45%,
+// issue 60%, shared memory 57%; tensor pipe 34%):
 //   layer 1 (K = 4): the epilogue warps on the CUDA cores, written as BF16
 //     straight into the tile's A operand buffer (K-major, 128-byte swizzle:
 //     the layout a TMA SWIZZLE_128B load produces);
@@ -32,6 +33,7 @@
 
 #include <cstddef>
 #include <cstdint>
+#include <cstring>
 #include <mutex>
 
 #include "launch_cache.h"
@@ -72,9 +74,8 @@ struct FusedSmem {
     int failed;
 };
 
-struct FusedMaps {
-    CUtensorMap w[4];  // W2, W3, W4 (256 x 256), W5 (16 x 256)
-};
+static_assert(sizeof(MlpMaps) == 4 * sizeof(CUtensorMap), "W2, W3, W4 (256 x 256), W5 (16 x 256)");
+__device__ __forceinline__ const unsigned char* map_of(const MlpMaps& m, int l) { return m.w[l]; }
 
 // the same SiLU as the training kernels
 __device__ __forceinline__ float silu_f(float z) { return sm100::silu_fast(z); }
@@ -117,7 +118,7 @@ __device__ __forceinline__ long long slot_tile(int u, long long j) {
 }
 
 __global__ void __launch_bounds__(kThreads, 1)
-mlp_fused_kernel(const __grid_constant__ FusedMaps maps, const float* __restrict__ X, long long n_cap,
+mlp_fused_kernel(const __grid_constant__ MlpMaps maps, const float* __restrict__ X, long long n_cap,
                  const unsigned* __restrict__ n_dev, const float* __restrict__ params, float* __restrict__ out,
                  int* err) {
     // the row count: n_cap, or the device count a previous kernel wrote (at most n_cap)
@@ -148,7 +149,7 @@ mlp_fused_kernel(const __grid_constant__ FusedMaps maps, const float* __restrict
     }
     if (warp == kEpiWarps) {
         if (lane == 0)
-            for (int l = 0; l < 4; ++l) sm100::tma_prefetch_desc(&maps.w[l]);
+            for (int l = 0; l < 4; ++l) sm100::tma_prefetch_desc(map_of(maps, l));
         sm100::tmem_alloc(&sh->tmem_base, 512);
         sm100::tmem_relinquish();
     }
@@ -175,7 +176,7 @@ mlp_fused_kernel(const __grid_constant__ FusedMaps maps, const float* __restrict
                             break;
                         }
                         sm100::mbar_arrive_expect_tx(&sh->full[s], bytes);
-                        sm100::tma_load_2d(ring + s * kStageBytes, &maps.w[l], &sh->full[s], kb * 64, 0);
+                        sm100::tma_load_2d(ring + s * kStageBytes, map_of(maps, l), &sh->full[s], kb * 64, 0);
                     }
                 }
             }
@@ -230,6 +231,19 @@ mlp_fused_kernel(const __grid_constant__ FusedMaps maps, const float* __restrict
         const int r_in_tile = quad * 32 + lane;
         const int c0 = group * kColsPerThread;
         uint32_t n_acc[kSlots] = {0, 0};
+        // Layer 1's split: a warp takes 64 units (a K-block) of 32 rows, a lane
+        // two units, whose weights stay in registers; the rows' inputs go
+        // round the warp by shuffles (1,048,653 rows: 630 -> 576 us on B200).
+        // With a lane per row every weight was an L1 load, 6,650 of a tile's
+        // 19,400 cycles; with a load a row instead of the shuffles, 603 us.
+        const int kb1 = warp & 3, rows1 = (warp >> 2) * 32, unit = kb1 * 64 + 2 * lane;
+        const float4 wa = __ldg(reinterpret_cast<const float4*>(params + ParamLayout::w1) + unit);
+        const float4 wb = __ldg(reinterpret_cast<const float4*>(params + ParamLayout::w1) + unit + 1);
+        const float2 bias1 = __ldg(reinterpret_cast<const float2*>(params + ParamLayout::b1) + unit / 2);
+        auto load_x = [&](long long tile) {
+            const long long r = tile * kRows + rows1 + lane;
+            return r < n ? __ldg(reinterpret_cast<const float4*>(X + r * kIn)) : make_float4(0.f, 0.f, 0.f, 0.f);
+        };
         for (long long rr = 0; rr < rounds_epi && !*failed; ++rr) {
             for (int u = 0; u < kSlots && !*failed; ++u) {
                 if (rr >= 5 * tiles_of[u]) continue;
@@ -237,28 +251,17 @@ mlp_fused_kernel(const __grid_constant__ FusedMaps maps, const float* __restrict
                 const long long row = slot_tile(u, rr / 5) * kRows + r_in_tile;
                 unsigned char* act = act0 + u * kActBytes;
                 if (stage == 0) {
-                    // layer 1 on the CUDA cores
-                    float x0 = 0.f, x1 = 0.f, x2 = 0.f, x3 = 0.f;
-                    if (row < n) {
-                        const float4 xv = *reinterpret_cast<const float4*>(X + row * kIn);
-                        x0 = xv.x;
-                        x1 = xv.y;
-                        x2 = xv.z;
-                        x3 = xv.w;
-                    }
-                    const float4* w1 = reinterpret_cast<const float4*>(params + ParamLayout::w1);
-                    const float4* b1 = reinterpret_cast<const float4*>(params + ParamLayout::b1);
-                    for (int k = c0; k < c0 + kColsPerThread; k += 8) {
-                        float v[8];
-                        const float4 ba = __ldg(b1 + k / 4), bb = __ldg(b1 + k / 4 + 1);
-                        const float bv[8] = {ba.x, ba.y, ba.z, ba.w, bb.x, bb.y, bb.z, bb.w};
-#pragma unroll
-                        for (int j = 0; j < 8; ++j) {
-                            const float4 w = __ldg(w1 + k + j);
-                            const float z = bv[j] + w.x * x0 + w.y * x1 + w.z * x2 + w.w * x3;
-                            v[j] = silu_f(z);
-                        }
-                        *reinterpret_cast<uint4*>(act + act_offset(r_in_tile, k)) = pack8(v);
+                    // layer 1 on the CUDA cores: the lane's two units for the warp's 32 rows
+                    const float4 xv = load_x(slot_tile(u, rr / 5));
+                    unsigned char* dst = act + (kb1 * kRows + rows1) * 128 + (lane & 3) * 4;
+#pragma unroll 4
+                    for (int i = 0; i < 32; ++i) {
+                        const float x0 = __shfl_sync(0xffffffffu, xv.x, i), x1 = __shfl_sync(0xffffffffu, xv.y, i);
+                        const float x2 = __shfl_sync(0xffffffffu, xv.z, i), x3 = __shfl_sync(0xffffffffu, xv.w, i);
+                        const float za = bias1.x + wa.x * x0 + wa.y * x1 + wa.z * x2 + wa.w * x3;
+                        const float zb = bias1.y + wb.x * x0 + wb.y * x1 + wb.z * x2 + wb.w * x3;
+                        *reinterpret_cast<__nv_bfloat162*>(dst + i * 128 + (((lane >> 2) ^ (i & 7)) << 4)) =
+                            __floats2bfloat162_rn(silu_f(za), silu_f(zb));
                     }
                     fence_proxy_async();
                     mbar_arrive(&sh->act_ready[u]);
@@ -346,15 +349,20 @@ bool weight_map(CUtensorMap* m, const __nv_bfloat16* w, int rows) {
 
 size_t mlp_fused_smem_bytes() { return 1024 + kSlots * kActBytes + kStages * kStageBytes + sizeof(FusedSmem); }
 
-cudaError_t launch_mlp_fused(const float* X, long long n, const float* params, __nv_bfloat16* const* wb,
-                             const __nv_bfloat16* w5b, float* out, int* d_err, cudaStream_t s,
-                             const unsigned* d_n) {
+bool make_mlp_maps(__nv_bfloat16* const* wb, const __nv_bfloat16* w5b, MlpMaps* maps) {
+    bool ok = true;
+    for (int l = 0; l < 4; ++l) {
+        CUtensorMap m;
+        ok = ok && (l < 3 ? weight_map(&m, wb[l], kHidden) : weight_map(&m, w5b, kOutPad));
+        if (ok) std::memcpy(maps->w[l], &m, sizeof(m));
+    }
+    return ok;
+}
+
+cudaError_t launch_mlp_fused(const float* X, long long n, const float* params, const MlpMaps& maps, float* out,
+                             int* d_err, cudaStream_t s, const unsigned* d_n) {
     if (n <= 0) return cudaSuccess;
     if ((reinterpret_cast<uintptr_t>(X) & 15) || (reinterpret_cast<uintptr_t>(out) & 15)) return cudaErrorInvalidValue;
-    FusedMaps maps;
-    for (int l = 0; l < 3; ++l)
-        if (!weight_map(&maps.w[l], wb[l], kHidden)) return cudaErrorInvalidValue;
-    if (!weight_map(&maps.w[3], w5b, kOutPad)) return cudaErrorInvalidValue;
     struct Shape {
         cudaError_t attr = cudaSuccess;
         int sms = 0;

@@ -75,7 +75,10 @@ struct GRRTSurrogate {
     unsigned* d_step = nullptr;
     float* d_lr = nullptr;
     __nv_bfloat16 *d_wb[3] = {}, *d_wt[3] = {}, *d_w5b = nullptr, *d_w5t = nullptr;
-    int* d_err = nullptr;
+    MlpMaps mlp_maps{};  // of d_wb and d_w5b
+    // the tensor-core kernels' error flag: host memory that they write only on a
+    // timeout, read here after a synchronisation without a copy
+    int *h_err = nullptr, *d_err = nullptr;
     DevStats* d_stats = nullptr;
     unsigned* d_queue = nullptr;
 
@@ -126,7 +129,7 @@ struct GRRTSurrogate {
         }
         dfree(d_w5b);
         dfree(d_w5t);
-        dfree(d_err);
+        if (h_err) cudaFreeHost(h_err);
         dfree(d_stats);
         dfree(d_queue);
         for (cudaEvent_t e : {ev_fork, ev_join[0], ev_join[1]})
@@ -194,15 +197,19 @@ struct GRRTSurrogate {
         if (fail(cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking), "cudaStreamCreate")) return false;
         const size_t P = ParamLayout::total;
         if (!dalloc(&d_params, P) || !dalloc(&d_grad, P) || !dalloc(&d_m, P) || !dalloc(&d_v, P) ||
-            !dalloc(&d_step, 1) || !dalloc(&d_lr, 1) || !dalloc(&d_err, 1) || !dalloc(&d_stats, 1) || !dalloc(&d_queue, 1))
+            !dalloc(&d_step, 1) || !dalloc(&d_lr, 1) || !dalloc(&d_stats, 1) || !dalloc(&d_queue, 1))
             return !fail_msg("cudaMalloc(surrogate parameters) failed");
         for (int l = 0; l < 3; ++l)
             if (!dalloc(&d_wb[l], kHidden * kHidden) || !dalloc(&d_wt[l], kHidden * kHidden))
                 return !fail_msg("cudaMalloc(bf16 weights) failed");
         if (!dalloc(&d_w5b, kOutPad * kHidden) || !dalloc(&d_w5t, kHidden * kDOutPad))
             return !fail_msg("cudaMalloc(bf16 weights) failed");
+        if (!make_mlp_maps(d_wb, d_w5b, &mlp_maps)) return !fail_msg("tensor map encoding failed");
         cudaMemsetAsync(d_w5t, 0, sizeof(__nv_bfloat16) * kHidden * kDOutPad, stream);
-        cudaMemsetAsync(d_err, 0, sizeof(int), stream);
+        if (fail(cudaHostAlloc(reinterpret_cast<void**>(&h_err), sizeof(int), cudaHostAllocMapped), "cudaHostAlloc") ||
+            fail(cudaHostGetDevicePointer(reinterpret_cast<void**>(&d_err), h_err, 0), "map error flag"))
+            return false;
+        *h_err = 0;
         // uniform init with variance 1/fan_in; biases 0; unused output rows 0
         std::vector<float> h(P, 0.0f);
         std::mt19937 rng(seed);
@@ -236,12 +243,13 @@ struct GRRTSurrogate {
         return !fail(umma_gemm_bf16(A, lda, B, ldb, M, N, K, sp, ep, d_err, stream), "tensor-core GEMM");
     }
 
+    // Waits for the stream; false if a kernel failed or reported a timeout.
     bool check_gemm_errors() {
-        int h = 0;
-        if (fail(copy(&h, d_err, sizeof(int), cudaMemcpyDeviceToHost), "read error flag")) return false;
-        if (h != 0) {
-            error = "tensor-core kernel reported a timeout (code " + std::to_string(h) + ")";
-            cudaMemsetAsync(d_err, 0, sizeof(int), stream);
+        if (fail(cudaStreamSynchronize(stream), "tensor-core kernels")) return false;
+        const int code = *static_cast<volatile int*>(h_err);
+        if (code != 0) {
+            error = "tensor-core kernel reported a timeout (code " + std::to_string(code) + ")";
+            *h_err = 0;
             return false;
         }
         return true;
@@ -489,7 +497,7 @@ struct GRRTSurrogate {
     // O[n x 16] = network(X[n x 4]): the fused tensor-core kernel (rows
     // min(n, *d_n) when a device count is given)
     bool enqueue_forward(const float* X, size_t n, float* out, const unsigned* d_n = nullptr) {
-        return !fail(launch_mlp_fused(X, static_cast<long long>(n), d_params, d_wb, d_w5b, out, d_err, stream, d_n),
+        return !fail(launch_mlp_fused(X, static_cast<long long>(n), d_params, mlp_maps, out, d_err, stream, d_n),
                      "fused network");
     }
 
@@ -783,9 +791,7 @@ extern "C" GRRT_EXPORT int grrt_surrogate_forward(GRRTSurrogate* s, const float*
     if (!s || !d_in || !d_out || n <= 0) return -1;
     s->error.clear();
     cudaSetDevice(s->device);
-    if (!s->enqueue_forward(d_in, static_cast<size_t>(n), d_out)) return -1;
-    if (s->fail(cudaStreamSynchronize(s->stream), "forward")) return -1;
-    return s->check_gemm_errors() ? 0 : -1;
+    return s->enqueue_forward(d_in, static_cast<size_t>(n), d_out) && s->check_gemm_errors() ? 0 : -1;
 }
 
 extern "C" GRRT_EXPORT int grrt_surrogate_gradients(GRRTSurrogate* s, const float* h_in, const float* h_y, int n,
