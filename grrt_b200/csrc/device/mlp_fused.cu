@@ -244,6 +244,11 @@ mlp_fused_kernel(const __grid_constant__ MlpMaps maps, const float* __restrict__
             const long long r = tile * kRows + rows1 + lane;
             return r < n ? __ldg(reinterpret_cast<const float4*>(X + r * kIn)) : make_float4(0.f, 0.f, 0.f, 0.f);
         };
+        // the slot's next inputs, brought into L1 while this tile is computed
+        auto prefetch_x = [&](long long tile) {
+            const long long r = tile * kRows + rows1 + lane;
+            if (r < n) asm volatile("prefetch.global.L1 [%0];" ::"l"(X + r * kIn));
+        };
         for (long long rr = 0; rr < rounds_epi && !*failed; ++rr) {
             for (int u = 0; u < kSlots && !*failed; ++u) {
                 if (rr >= 5 * tiles_of[u]) continue;
@@ -253,6 +258,7 @@ mlp_fused_kernel(const __grid_constant__ MlpMaps maps, const float* __restrict__
                 if (stage == 0) {
                     // layer 1 on the CUDA cores: the lane's two units for the warp's 32 rows
                     const float4 xv = load_x(slot_tile(u, rr / 5));
+                    prefetch_x(slot_tile(u, rr / 5 + 1));
                     unsigned char* dst = act + (kb1 * kRows + rows1) * 128 + (lane & 3) * 4;
 #pragma unroll 4
                     for (int i = 0; i < 32; ++i) {

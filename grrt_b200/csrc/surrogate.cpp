@@ -27,6 +27,7 @@
 #include <memory>
 #include <random>
 #include <string>
+#include <type_traits>
 #include <vector>
 
 #include "../../include/grrt_surrogate.h"
@@ -70,6 +71,7 @@ struct GRRTSurrogate {
     cudaEvent_t ev_fork = nullptr, ev_join[2] = {};
     std::string error;
 
+    unsigned char* d_net = nullptr;  // holds the buffers below, up to the error flag
     // parameters (FP32 master), gradients, Adam moments, step counter
     float *d_params = nullptr, *d_grad = nullptr, *d_m = nullptr, *d_v = nullptr;
     unsigned* d_step = nullptr;
@@ -118,20 +120,10 @@ struct GRRTSurrogate {
         free_workspace();
         dfree(loss_hist);
         free_inference();
-        for (auto* p : {d_params, d_grad, d_m, d_v, d_X, d_Y}) {
-            if (p) cudaFree(p);
-        }
-        dfree(d_step);
-        dfree(d_lr);
-        for (int l = 0; l < 3; ++l) {
-            dfree(d_wb[l]);
-            dfree(d_wt[l]);
-        }
-        dfree(d_w5b);
-        dfree(d_w5t);
+        dfree(d_X);
+        dfree(d_Y);
+        dfree(d_net);
         if (h_err) cudaFreeHost(h_err);
-        dfree(d_stats);
-        dfree(d_queue);
         for (cudaEvent_t e : {ev_fork, ev_join[0], ev_join[1]})
             if (e) cudaEventDestroy(e);
         for (cudaStream_t q : {stream, side[0], side[1]})
@@ -188,22 +180,35 @@ struct GRRTSurrogate {
             return false;
         }
         if (fail(cudaGetDevice(&device), "cudaGetDevice")) return false;
-        cudaDeviceProp prop{};
-        if (fail(cudaGetDeviceProperties(&prop, device), "cudaGetDeviceProperties")) return false;
-        if (prop.major < 10) {
+        int major = 0;
+        if (fail(cudaDeviceGetAttribute(&major, cudaDevAttrComputeCapabilityMajor, device), "cudaDeviceGetAttribute"))
+            return false;
+        if (major < 10) {
             error = "the surrogate's tensor-core kernels need an sm_100 GPU";
             return false;
         }
         if (fail(cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking), "cudaStreamCreate")) return false;
         const size_t P = ParamLayout::total;
-        if (!dalloc(&d_params, P) || !dalloc(&d_grad, P) || !dalloc(&d_m, P) || !dalloc(&d_v, P) ||
-            !dalloc(&d_step, 1) || !dalloc(&d_lr, 1) || !dalloc(&d_stats, 1) || !dalloc(&d_queue, 1))
-            return !fail_msg("cudaMalloc(surrogate parameters) failed");
-        for (int l = 0; l < 3; ++l)
-            if (!dalloc(&d_wb[l], kHidden * kHidden) || !dalloc(&d_wt[l], kHidden * kHidden))
-                return !fail_msg("cudaMalloc(bf16 weights) failed");
-        if (!dalloc(&d_w5b, kOutPad * kHidden) || !dalloc(&d_w5t, kHidden * kDOutPad))
-            return !fail_msg("cudaMalloc(bf16 weights) failed");
+        // one allocation for everything a network keeps: sizes first, then places
+        for (int pass = 0; pass < 2; ++pass) {
+            size_t bytes = 0;
+            auto place = [&](auto** p, size_t count) {
+                if (pass == 1) *p = reinterpret_cast<std::remove_reference_t<decltype(*p)>>(d_net + bytes);
+                bytes += (count * sizeof(**p) + 255) / 256 * 256;
+            };
+            for (float** p : {&d_params, &d_grad, &d_m, &d_v}) place(p, P);
+            place(&d_step, 1);
+            place(&d_lr, 1);
+            place(&d_stats, 1);
+            place(&d_queue, 1);
+            for (int l = 0; l < 3; ++l) {
+                place(&d_wb[l], kHidden * kHidden);
+                place(&d_wt[l], kHidden * kHidden);
+            }
+            place(&d_w5b, kOutPad * kHidden);
+            place(&d_w5t, kHidden * kDOutPad);
+            if (pass == 0 && !dalloc(&d_net, bytes)) return !fail_msg("cudaMalloc(surrogate network) failed");
+        }
         if (!make_mlp_maps(d_wb, d_w5b, &mlp_maps)) return !fail_msg("tensor map encoding failed");
         cudaMemsetAsync(d_w5t, 0, sizeof(__nv_bfloat16) * kHidden * kDOutPad, stream);
         if (fail(cudaHostAlloc(reinterpret_cast<void**>(&h_err), sizeof(int), cudaHostAllocMapped), "cudaHostAlloc") ||
