@@ -339,6 +339,15 @@ GRRT_HD Vec5<float> mixed_k1(float M, float a, float pt, float pph, const Vec5<d
     return kerr_rhs<float>(M, a, pt, pph, yf);
 }
 
+// 1/x of the FP32 error norm (x > 0, far from the range's ends).
+GRRT_HD float recip_err(float x) {
+#ifdef GRRT_RHS_PINNED
+    return rcp_approx(x);
+#else
+    return recip(x);
+#endif
+}
+
 // Packed FP32 pairs: sm_100's two-wide FP32 fused multiply-add and multiply,
 // one instruction for two lanes, each lane rounded as fmaf / the float
 // product (elsewhere the lanes are computed one by one, with the same results).
@@ -358,21 +367,16 @@ GRRT_HD float2 pk_mul(float2 a, float2 b) {
 #endif
 }
 
-// A 5-vector as two packed pairs (r, theta), (phi, p_r) and p_theta alone.
-struct Pk5 {
+// The four components that feed the right-hand side as two packed pairs
+// (r, theta), (p_r, p_theta); phi is kept apart, its stage states are not formed.
+struct Pk4 {
     float2 a, b;
-    float c;
 };
-GRRT_HD Pk5 pack5(const Vec5<float>& v) { return Pk5{pk(v.r, v.th), pk(v.ph, v.pr), v.pth}; }
-GRRT_HD Vec5<float> unpack5(const Pk5& v) { return Vec5<float>{v.a.x, v.a.y, v.b.x, v.b.y, v.c}; }
+GRRT_HD Pk4 pack4(const Vec5<float>& v) { return Pk4{pk(v.r, v.th), pk(v.pr, v.pth)}; }
 // c * v, and c * v + w, per component
-GRRT_HD Pk5 pk5_mul(float c, const Pk5& v) {
-    const float2 cc = pk(c, c);
-    return Pk5{pk_mul(cc, v.a), pk_mul(cc, v.b), c * v.c};
-}
-GRRT_HD Pk5 pk5_fma(float c, const Pk5& v, const Pk5& w) {
-    const float2 cc = pk(c, c);
-    return Pk5{pk_fma(cc, v.a, w.a), pk_fma(cc, v.b, w.b), fmaf(c, v.c, w.c)};
+GRRT_HD Pk4 pk4_mul(float c, const Pk4& v) { return Pk4{pk_mul(pk(c, c), v.a), pk_mul(pk(c, c), v.b)}; }
+GRRT_HD Pk4 pk4_fma(float c, const Pk4& v, const Pk4& w) {
+    return Pk4{pk_fma(pk(c, c), v.a, w.a), pk_fma(pk(c, c), v.b, w.b)};
 }
 
 // Mixed-precision attempt: the seven right-hand sides and the stage sums in
@@ -380,52 +384,60 @@ GRRT_HD Pk5 pk5_fma(float c, const Pk5& v, const Pk5& w) {
 // so round-off does not accumulate along the ray. The error norm is formed in
 // FP32; its noise floor (about 1e-7 of |h k|/|y|) is why FP32 steps are
 // controlled against their own tolerance (DevScene::tol_fp32). The stage sums
-// run on packed pairs (three lanes of work for five components): each stage
-// state is y + h * (sum_j a_sj k_j), the sum accumulated in the tableau's
-// order with fused multiply-adds.
+// run on packed pairs: each stage state is y + h * (sum_j a_sj k_j), the sum
+// accumulated in the tableau's order with fused multiply-adds.
 // k1 = mixed_k1(y) is given by the caller (the previous accepted attempt's
 // k7, which is f at float(y5) = float(new y), or the rejected attempt's k1).
 GRRT_HD double mixed_attempt_k1(float M, float a, float pt, float pph, const Vec5<double>& y, double dl,
                                 const Vec5<float>& k1v, Vec5<double>& y5, Vec5<float>& k7_out) {
     using namespace dp;
-    const Pk5 Y = pack5(Vec5<float>{static_cast<float>(y.r), static_cast<float>(y.th), static_cast<float>(y.ph),
-                                    static_cast<float>(y.pr), static_cast<float>(y.pth)});
+    const Pk4 Y = Pk4{pk(static_cast<float>(y.r), static_cast<float>(y.th)),
+                      pk(static_cast<float>(y.pr), static_cast<float>(y.pth))};
     const float h = static_cast<float>(dl);
-    // y + h * s
-    auto stage = [&](const Pk5& sum) { return unpack5(pk5_fma(h, sum, Y)); };
-    const Pk5 K1 = pack5(k1v);
-    const Pk5 K2 = pack5(kerr_rhs<float>(M, a, pt, pph, stage(pk5_mul(float(a21), K1))));
-    const Pk5 K3 = pack5(kerr_rhs<float>(M, a, pt, pph, stage(pk5_fma(float(a32), K2, pk5_mul(float(a31), K1)))));
-    const Pk5 K4 = pack5(kerr_rhs<float>(
-        M, a, pt, pph, stage(pk5_fma(float(a43), K3, pk5_fma(float(a42), K2, pk5_mul(float(a41), K1))))));
-    const Pk5 K5 = pack5(kerr_rhs<float>(
-        M, a, pt, pph,
-        stage(pk5_fma(float(a54), K4, pk5_fma(float(a53), K3, pk5_fma(float(a52), K2, pk5_mul(float(a51), K1)))))));
-    const Pk5 K6 = pack5(kerr_rhs<float>(
-        M, a, pt, pph,
-        stage(pk5_fma(float(a65), K5,
-                      pk5_fma(float(a64), K4,
-                              pk5_fma(float(a63), K3, pk5_fma(float(a62), K2, pk5_mul(float(a61), K1))))))));
-    const Pk5 B = pk5_fma(float(b6), K6,
-                          pk5_fma(float(b5), K5, pk5_fma(float(b4), K4, pk5_fma(float(b3), K3, pk5_mul(float(b1), K1)))));
-    const Pk5 I = Pk5{pk_mul(pk(h, h), B.a), pk_mul(pk(h, h), B.b), h * B.c};
-    y5 = Vec5<double>{y.r + double(I.a.x), y.th + double(I.a.y), y.ph + double(I.b.x), y.pr + double(I.b.y),
-                      y.pth + double(I.c)};
-    const Pk5 E = pk5_fma(float(e6), K6,
-                          pk5_fma(float(e5), K5, pk5_fma(float(e4), K4, pk5_fma(float(e3), K3, pk5_mul(float(e1), K1)))));
+    // f(y + h * sum), packed, and the phi component
+    auto stage = [&](const Pk4& sum, float& ph) {
+        const Pk4 v = pk4_fma(h, sum, Y);
+        const Vec5<float> k = kerr_rhs<float>(M, a, pt, pph, Vec5<float>{v.a.x, v.a.y, 0.0f, v.b.x, v.b.y});
+        ph = k.ph;
+        return pack4(k);
+    };
+    float p2, p3, p4, p5, p6;
+    const float p1 = k1v.ph;
+    const Pk4 K1 = pack4(k1v);
+    const Pk4 K2 = stage(pk4_mul(float(a21), K1), p2);
+    const Pk4 K3 = stage(pk4_fma(float(a32), K2, pk4_mul(float(a31), K1)), p3);
+    const Pk4 K4 = stage(pk4_fma(float(a43), K3, pk4_fma(float(a42), K2, pk4_mul(float(a41), K1))), p4);
+    const Pk4 K5 = stage(
+        pk4_fma(float(a54), K4, pk4_fma(float(a53), K3, pk4_fma(float(a52), K2, pk4_mul(float(a51), K1)))), p5);
+    const Pk4 K6 = stage(
+        pk4_fma(float(a65), K5,
+                pk4_fma(float(a64), K4, pk4_fma(float(a63), K3, pk4_fma(float(a62), K2, pk4_mul(float(a61), K1))))),
+        p6);
+    const Pk4 B = pk4_fma(float(b6), K6,
+                          pk4_fma(float(b5), K5, pk4_fma(float(b4), K4, pk4_fma(float(b3), K3, pk4_mul(float(b1), K1)))));
+    const float Bp = fmaf(float(b6), p6, fmaf(float(b5), p5, fmaf(float(b4), p4, fmaf(float(b3), p3, float(b1) * p1))));
+    const Pk4 I = pk4_mul(h, B);
+    y5 = Vec5<double>{y.r + double(I.a.x), y.th + double(I.a.y), y.ph + double(h * Bp), y.pr + double(I.b.x),
+                      y.pth + double(I.b.y)};
+    const Pk4 E = pk4_fma(float(e6), K6,
+                          pk4_fma(float(e5), K5, pk4_fma(float(e4), K4, pk4_fma(float(e3), K3, pk4_mul(float(e1), K1)))));
+    const float Ep = fmaf(float(e6), p6, fmaf(float(e5), p5, fmaf(float(e4), p4, fmaf(float(e3), p3, float(e1) * p1))));
     const Vec5<float> y5f{static_cast<float>(y5.r), static_cast<float>(y5.th), static_cast<float>(y5.ph),
                           static_cast<float>(y5.pr), static_cast<float>(y5.pth)};
     const Vec5<float> k7 = kerr_rhs<float>(M, a, pt, pph, y5f);
     k7_out = k7;
-    const Vec5<float> ev = unpack5(pk5_fma(float(e7), pack5(k7), E));
+    const Pk4 e4v = pk4_fma(float(e7), pack4(k7), E);
+    const float ep = fmaf(float(e7), k7.ph, Ep);
     float err = 0.0f;
-#define GRRT_ERRF(f)                                                       \
-    {                                                                      \
-        const float v = fabsf(h * ev.f) * recip(fabsf(y5f.f) + 1e-10f);    \
-        err = (err < v) ? v : err;                                         \
-    }
-    GRRT_ERRF(r) GRRT_ERRF(th) GRRT_ERRF(ph) GRRT_ERRF(pr) GRRT_ERRF(pth)
-#undef GRRT_ERRF
+    auto term = [&](float e, float yv) {
+        const float v = fabsf(h * e) * recip_err(fabsf(yv) + 1e-10f);
+        err = (err < v) ? v : err;
+    };
+    term(e4v.a.x, y5f.r);
+    term(e4v.a.y, y5f.th);
+    term(ep, y5f.ph);
+    term(e4v.b.x, y5f.pr);
+    term(e4v.b.y, y5f.pth);
     return static_cast<double>(err);
 }
 
