@@ -388,11 +388,11 @@ GRRT_HD Pk4 pk4_fma(float c, const Pk4& v, const Pk4& w) {
 // accumulated in the tableau's order with fused multiply-adds.
 // k1 = mixed_k1(y) is given by the caller (the previous accepted attempt's
 // k7, which is f at float(y5) = float(new y), or the rejected attempt's k1).
-GRRT_HD double mixed_attempt_k1(float M, float a, float pt, float pph, const Vec5<double>& y, double dl,
-                                const Vec5<float>& k1v, Vec5<double>& y5, Vec5<float>& k7_out) {
+// mixed_attempt_yf also takes Y = float(y) and gives Y5 = float(y5), so a
+// caller that keeps it converts each state once.
+GRRT_HD double mixed_attempt_yf(float M, float a, float pt, float pph, const Vec5<double>& y, const Pk4& Y, double dl,
+                                const Vec5<float>& k1v, Vec5<double>& y5, Pk4& Y5, Vec5<float>& k7_out) {
     using namespace dp;
-    const Pk4 Y = Pk4{pk(static_cast<float>(y.r), static_cast<float>(y.th)),
-                      pk(static_cast<float>(y.pr), static_cast<float>(y.pth))};
     const float h = static_cast<float>(dl);
     // f(y + h * sum), packed, and the phi component
     auto stage = [&](const Pk4& sum, float& ph) {
@@ -426,6 +426,7 @@ GRRT_HD double mixed_attempt_k1(float M, float a, float pt, float pph, const Vec
                           static_cast<float>(y5.pr), static_cast<float>(y5.pth)};
     const Vec5<float> k7 = kerr_rhs<float>(M, a, pt, pph, y5f);
     k7_out = k7;
+    Y5 = pack4(y5f);
     const Pk4 e4v = pk4_fma(float(e7), pack4(k7), E);
     const float ep = fmaf(float(e7), k7.ph, Ep);
     float err = 0.0f;
@@ -439,6 +440,17 @@ GRRT_HD double mixed_attempt_k1(float M, float a, float pt, float pph, const Vec
     term(e4v.b.x, y5f.pr);
     term(e4v.b.y, y5f.pth);
     return static_cast<double>(err);
+}
+
+GRRT_HD Pk4 pack_state(const Vec5<double>& y) {
+    return Pk4{pk(static_cast<float>(y.r), static_cast<float>(y.th)),
+               pk(static_cast<float>(y.pr), static_cast<float>(y.pth))};
+}
+
+GRRT_HD double mixed_attempt_k1(float M, float a, float pt, float pph, const Vec5<double>& y, double dl,
+                                const Vec5<float>& k1v, Vec5<double>& y5, Vec5<float>& k7_out) {
+    Pk4 Y5;
+    return mixed_attempt_yf(M, a, pt, pph, y, pack_state(y), dl, k1v, y5, Y5, k7_out);
 }
 
 GRRT_HD double mixed_attempt_impl(float M, float a, float pt, float pph, const Vec5<double>& y, double dl,
@@ -565,35 +577,25 @@ GRRT_HD double step_factor_ratio(double tol, double err) {
 #endif
 }
 
+// err is a single-precision value. Selects in place of branches: a warp nearly
+// always holds both outcomes.
 GRRT_HD StepDecision pi_control_f32(double err, double tol, double dl, int retry,
                                                    double r5) {
     constexpr double safety = 0.9, grow_max = 5.0, shrink_max = 0.2, dl_min = 1e-6;
-    StepDecision d;
+    const bool ok = err <= tol;
+    const double lo = ok ? 1.0 : shrink_max, hi = ok ? grow_max : 1.0;
+    double f = safety * step_factor_ratio(tol, err);
+    f = (f < lo) ? lo : (hi < f) ? hi : f;
+    if (ok && !(err > 1e-30)) f = grow_max;
     const double ar = fabs(r5);
     const double cap = 5.0 * ((ar < 1.0) ? 1.0 : ar);
-    if (retry >= 20) {
-        d.accept = true;
-        d.next = dl;
-        return d;
-    }
-    if (err <= tol) {
-        double f = (err > 1e-30) ? safety * step_factor_ratio(tol, err) : grow_max;
-        f = (f < 1.0) ? 1.0 : (grow_max < f) ? grow_max : f;
-        const double nx = dl * f;
-        d.accept = true;
-        d.next = (cap < nx) ? cap : nx;
-        return d;
-    }
-    double f = safety * step_factor_ratio(tol, err);
-    f = (f < shrink_max) ? shrink_max : (1.0 < f) ? 1.0 : f;
-    const double ndl = dl * f;
-    if (ndl < dl_min) {
-        d.accept = true;
-        d.next = (cap < dl_min) ? cap : dl_min;
-        return d;
-    }
-    d.accept = false;
-    d.next = ndl;
+    const double nx = dl * f;
+    const bool tiny = !ok && nx < dl_min;
+    StepDecision d;
+    d.accept = ok || tiny || retry >= 20;
+    d.next = tiny ? dl_min : nx;
+    if ((ok || tiny) && cap < d.next) d.next = cap;
+    if (retry >= 20) d.next = dl;
     return d;
 }
 

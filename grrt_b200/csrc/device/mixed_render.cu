@@ -149,6 +149,9 @@ struct SpecStage {
     float k[5][32];                           // FP32 f(y) at the start
     unsigned q[32];                           // sample index
     const DevScene* sp[32];                   // batch: the sample's scene
+    // the lane's own sample: what its steps touch rarely, out of the registers
+    double a2e2[32], l2[32], swept[32];
+    unsigned lq[32];
 };
 }  // namespace
 
@@ -174,13 +177,15 @@ mixed_speculate_kernel(const __grid_constant__ DevScene S0, const DevTile tile, 
     // warp-uniform: prepared slots [ring_head, ring_n) and the queue state
     int ring_head = 0, ring_n = 0;
     bool drained = false;
-    unsigned q = ~0u;
     bool live = false;
     Vec5<double> y;
     Vec5<float> k1;  // FP32 f(y), kept from the previous attempt
-    double pt = 0, pph = 0, dl = 0;
+    Pk4 yf;          // float(y), likewise
+    float ptf = 0, pphf = 0;
+    double dl = 0;
     int retry = 0, step = 0;
-    mixed::Tracker trk;
+    mixed::TrackScene trk = mixed::track_scene(S0.disk_on, S0.r_in, S0.r_out, mb.margin, mb.r_near);
+    float sin_th = 0.0f;
     while (true) {
         const unsigned need = __ballot_sync(kMask, !live);
         // ---- the warp prepares its next starts (every lane one sample) ----
@@ -252,23 +257,27 @@ mixed_speculate_kernel(const __grid_constant__ DevScene S0, const DevTile tile, 
             const int rank = __popc(need & lt_mask);
             if (!live && rank < avail) {
                 const int slot = ring_head + rank;
-                q = W.q[slot];
+                W.lq[lane] = W.q[slot];
                 if (kBatch) {
                     sp = W.sp[slot];
                     Mf = static_cast<float>(S.M);
                     af = static_cast<float>(S.a);
                 }
                 y = Vec5<double>{S.cam_pos[1], S.cam_pos[2], S.cam_pos[3], W.pr[slot], W.pth[slot]};
-                pt = W.pt[slot];
-                pph = W.pph[slot];
+                const double pt = W.pt[slot], pph = W.pph[slot];
+                ptf = static_cast<float>(pt);
+                pphf = static_cast<float>(pph);
+                yf = pack_state(y);
                 k1 = Vec5<float>{W.k[0][slot], W.k[1][slot], W.k[2][slot], W.k[3][slot], W.k[4][slot]};
                 dl = S.dl0;
                 retry = 0;
                 step = 0;
-                if (kBatch)
-                    trk.reset(S.disk_on, S.r_in, S.r_out, S.mixed_margin, S.r_near_mixed, S.a, pt, pph, y.th);
-                else
-                    trk.reset(S.disk_on, S.r_in, S.r_out, mb.margin, mb.r_near, S.a, pt, pph, y.th);
+                if (kBatch) trk = mixed::track_scene(S.disk_on, S.r_in, S.r_out, S.mixed_margin, S.r_near_mixed);
+                const mixed::TrackRay ray = mixed::track_ray(S.a, pt, pph);
+                W.a2e2[lane] = ray.a2e2;
+                W.l2[lane] = ray.l2;
+                W.swept[lane] = 0.0;
+                sin_th = mixed::track_start_sin(y.th);
                 live = true;
             }
             ring_head += min(__popc(need), avail);
@@ -278,17 +287,19 @@ mixed_speculate_kernel(const __grid_constant__ DevScene S0, const DevTile tile, 
         int term = -1;
         bool retrace = false;
         Vec5<float> k7;
-        if (live && retry == 0) term = start_test(S, step, y.r);
+        if (live && (step | retry) == 0) term = start_test(S, 0, y.r);
         if (live && term < 0) {
             Vec5<double> y5;
-            const double err =
-                mixed_attempt_k1(Mf, af, static_cast<float>(pt), static_cast<float>(pph), y, dl, k1, y5, k7);
+            Pk4 y5f;
+            const double err = mixed_attempt_yf(Mf, af, ptf, pphf, y, yf, dl, k1, y5, y5f, k7);
             ++n_att;
             const StepDecision d = pi_control_f32(err, S.tol_fp32, dl, retry, y5.r);
             if (d.accept) {
                 ++n_acc;
-                retrace = trk.step(y, y5, dl);
+                retrace = mixed::track_step(
+                    trk, [&] { return mixed::TrackRay{W.a2e2[lane], W.l2[lane]}; }, W.swept[lane], sin_th, y, y5, dl);
                 y = y5;
+                yf = y5f;
                 k1 = k7;
                 dl = d.next;
                 retry = 0;
@@ -308,8 +319,10 @@ mixed_speculate_kernel(const __grid_constant__ DevScene S0, const DevTile tile, 
             }
         }
         bool queue = false;
+        unsigned q = ~0u;
         if (live && term >= 0) {
             live = false;
+            q = W.lq[lane];
             if (kBatch || !mb.spec_list) ++n_rays;  // a list's samples are counted by its producer
             const size_t o = 3 * static_cast<size_t>(q);
             if (retrace || term == kTermMaxSteps) {
