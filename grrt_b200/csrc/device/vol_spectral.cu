@@ -26,7 +26,11 @@
 // instruction fetch (3.0 of 6.8 cycles an instruction), so the last stages are
 // a loop, both kinds of step share one geometry lookup, and the physics calls
 // one body of each library function; and where a frame has fewer rays than
-// lanes they are spread over the warps (33 -> 29 ms; 13.6 -> 11.7 ms).
+// lanes they are spread over the warps (33 -> 29 ms; 13.6 -> 11.7 ms). The
+// first thousand steps of the longest ray take 11 ms among busy lanes, the
+// other 8000 then 18 ms alone in its warp, so the lanes' order keeps long rays
+// apart (vol_take_order) and a warp out of work alternates the kinds of step
+// (29 -> 27.5 ms; 11.8 -> 9.3 ms).
 //
 // A ray's transfer state is a row of 4 x nb doubles per lane slot
 // [J | T | tau | pixel sum], so the warp's accesses to one row are
@@ -115,6 +119,8 @@ vol_spectral_kernel(const __grid_constant__ DevScene S0, const DevTile tile, con
     bool been_inside = false, cancelled = false;
     unsigned iter = 0;
     bool refill = true;  // warp-uniform: some lane has no ray
+    bool turns = false;  // warp-uniform: outer and march steps take turns
+    bool turn = false;   // warp-uniform: whether it is the march steps' turn
     // the lane's place in a pass over physics steps: which of the pass's rays,
     // which bin (the first, of a ray with more bins than lanes)
     __shared__ PhysStage stage[kSpecThreads / 32];
@@ -153,8 +159,8 @@ vol_spectral_kernel(const __grid_constant__ DevScene S0, const DevTile tile, con
                             }  // else: padding slot of a short chunk, fetch again
                         } else {
                             // list: the listed samples (kList), or the pixel order;
-                            // taken in the spread order (vol_spread_order)
-                            const unsigned ks = vol_spread_order(k, total);
+                            // in vol_take_order's order
+                            const unsigned ks = vol_take_order(k, total);
                             pix = static_cast<int>(list ? list[ks] : ks);
                             smp = 0;
                             fresh_pixel = true;
@@ -215,6 +221,7 @@ vol_spectral_kernel(const __grid_constant__ DevScene S0, const DevTile tile, con
             }
             if (!__any_sync(kWarp, live || pix >= -1)) break;
             refill = __any_sync(kWarp, pix == -1);
+            turns = __any_sync(kWarp, pix == -2);
         }
 
         // ---- start of an outer step: termination tests ----
@@ -230,7 +237,16 @@ vol_spectral_kernel(const __grid_constant__ DevScene S0, const DevTile tile, con
 
         // a march step was taken; it ends inside the volume; the march ends
         bool stepped = false, inside = false, mend = false;
-        if (live && term < 0) {
+        // Once the warp finds no more work, outer steps and march steps take turns:
+        // rays that alternate between the two fall into step, and each iteration
+        // costs one kind instead of both. While every lane is busy both run, sharing
+        // stages 2 to 4.
+        const bool go = live && term < 0;
+        if (turns) {
+            turn = !turn;
+            if (!__any_sync(kWarp, go && marching == turn)) turn = !turn;
+        }
+        if (go && (!turns || marching == turn)) {
             // ---- first stage, where the last step did not leave it (a march's first step
             //      takes the outer step's) ----
             if (!k1_ok) {
