@@ -55,6 +55,8 @@ struct GRRTBatch {
     int order = GRRT_BATCH_ORDER_ROUND_ROBIN;
     int blocks_per_sm = 0;  // 0 = as many as fit
     int block = 128;        // threads per block of the FP64 thin-disk batch kernel (64, 128, 256)
+    bool schedule_set = false;     // a schedule or block size was chosen (by the caller or the autotuner)
+    bool no_sample_room = false;   // the default's sample scratch could not be had
     bool tuned = false;
     // device
     int device = -1;
@@ -157,8 +159,23 @@ struct GRRTBatch {
         return B;
     }
 
-    // FP64 thin-disk batch traced by samples (GRRT_BATCH_ORDER_SAMPLES)
-    bool by_samples() const { return !spectral && form != GRRT_FORM_MIXED && order == GRRT_BATCH_ORDER_SAMPLES; }
+    // Sample scratch up to this size is taken for a batch whose schedule nobody
+    // chose (4.2 M samples: 0.25 GB).
+    static constexpr size_t kDefaultSampleScratch = size_t(1) << 30;
+
+    // FP64 thin-disk batch traced by samples: GRRT_BATCH_ORDER_SAMPLES, and the
+    // default where its scratch fits. The kernel that takes samples prepares
+    // their starts with the whole warp and inlines the right-hand side, so it
+    // was the faster one at every size tried (B200, against 256-pixel chunks
+    // round robin: 4 cameras of 60x50 1.40 -> 0.91 ms, 12 of 256x250 7.3 ->
+    // 5.7, 64 of 256x256 37.0 -> 26.2). Without its scratch the pixels are
+    // traced lane by lane.
+    bool by_samples() const {
+        if (spectral || form == GRRT_FORM_MIXED) return false;
+        if (order == GRRT_BATCH_ORDER_SAMPLES) return true;
+        return !schedule_set && !no_sample_room && total_samples > 0 && total_samples <= 0x7f000000ull &&
+               mixed_scratch_bytes_for(total_samples) <= kDefaultSampleScratch;
+    }
 
     int max_blocks_per_sm() const {
         if (spectral) return vol_spectral_batch_max_blocks_per_sm();
@@ -189,13 +206,34 @@ struct GRRTBatch {
         return sms * per;
     }
 
+    // The scratch of the sample-based passes, grown as needed.
+    cudaError_t sample_scratch_error() {
+        const size_t need = mixed_scratch_bytes_for(total_samples);
+        if (need <= mixed_bytes) return cudaSuccess;
+        if (graph) cudaGraphExecDestroy(graph);
+        graph = nullptr;
+        cudaFree(d_mixed);
+        d_mixed = nullptr;
+        mixed_bytes = 0;
+        const cudaError_t e = cudaMalloc(&d_mixed, need);
+        if (e == cudaSuccess) mixed_bytes = need;
+        return e;
+    }
+    bool sample_scratch() { return sample_scratch_error() == cudaSuccess; }
+
     // Enqueue one batched render (as a CUDA graph replay) on stream s: RGBA
     // (float4 per pixel) or, for a spectral batch, the cubes (doubles).
     int launch(void* out, cudaStream_t s) {
         if (!upload_schedule()) return -1;
-        const int nb = blocks();
         const bool mixed = !spectral && form == GRRT_FORM_MIXED;
-        const bool samples = by_samples();
+        bool samples = by_samples();
+        if (samples && order != GRRT_BATCH_ORDER_SAMPLES && !sample_scratch()) {
+            // the default's scratch is not to be had: pixel by pixel needs none
+            cudaGetLastError();
+            no_sample_room = true;
+            samples = false;
+        }
+        const int nb = blocks();
         if (spectral) {
             const size_t need = static_cast<size_t>(4) * nb_max * nb * vol_spectral_batch_threads();
             if (need > spec_scratch_elems) {
@@ -214,16 +252,7 @@ struct GRRTBatch {
                         std::to_string(total_samples);
                 return -1;
             }
-            const size_t need = mixed_scratch_bytes_for(total_samples);
-            if (need > mixed_bytes) {
-                if (graph) cudaGraphExecDestroy(graph);
-                graph = nullptr;
-                cudaFree(d_mixed);
-                d_mixed = nullptr;
-                mixed_bytes = 0;
-                if (fail(cudaMalloc(&d_mixed, need), "cudaMalloc(mixed scratch)")) return -1;
-                mixed_bytes = need;
-            }
+            if (fail(sample_scratch_error(), "cudaMalloc(mixed scratch)")) return -1;
         }
         if (!graph || graph_out != out || graph_form != form || graph_blocks != nb || graph_block != block ||
             graph_samples != samples) {
@@ -438,6 +467,7 @@ extern "C" GRRT_EXPORT int grrt_batch_set_tuning(GRRTBatch* b, int block, double
                           "r_factor in [1, 100]";
         return -1;
     }
+    if (block != b->block) b->schedule_set = true;
     b->block = block;
     for (auto& c : b->cams) {
         c->tol_fp32 = tol_fp32;
@@ -466,6 +496,7 @@ extern "C" GRRT_EXPORT int grrt_batch_set_schedule(GRRTBatch* b, int chunk_size,
     b->chunk_size = chunk_size;
     b->order = order;
     b->blocks_per_sm = blocks_per_sm;
+    b->schedule_set = true;
     b->schedule_dirty = true;
     return 0;
 }
@@ -695,6 +726,7 @@ extern "C" GRRT_EXPORT int grrt_batch_autotune(GRRTBatch* b, const char* cache_p
         tune_out = b->d_out;
     }
     const bool mixed = !b->spectral && b->form == GRRT_FORM_MIXED;
+    b->schedule_set = true;
     Tuning cur{b->chunk_size, b->order, b->blocks_per_sm, b->block, b->cams[0]->tol_fp32, b->cams[0]->mixed_r_factor};
     Tuning best_t = cur;
     double best = 1e30;

@@ -167,7 +167,9 @@ typedef struct GRRTBatch GRRTBatch;
  * thin-disk batches): every camera's samples in camera order, traced by
  * samples with the warp staging of the single FP64 render, then resolved into
  * pixels; the chunk size and the threads per block do not apply (other
- * batches take it as camera-major). */
+ * batches take it as camera-major). An FP64 thin-disk batch whose schedule was
+ * never set is traced that way too while its scratch stays below 1 GB; setting
+ * a schedule or a block size, or the autotuner, decides otherwise. */
 #define GRRT_BATCH_ORDER_CAMERA_MAJOR 0
 #define GRRT_BATCH_ORDER_ROUND_ROBIN 1
 #define GRRT_BATCH_ORDER_SAMPLES 2
