@@ -73,11 +73,11 @@ F_ATTEMPT_EXEC = 6 * F_EVAL + 480
 # Operations the kernels execute per attempt (all of a kernel's floating-point
 # operations divided by its attempts; a fused multiply-add counts 2), from the
 # ncu instruction counters of a 512x512 4-spp frame
-# (profiles/executed_flops_thin_mixed_kernels_kerr_512x512_4spp.md): the FP64
+# (profiles/thin_kernels_inlined_kerr_512x512_4spp.md): the FP64
 # kernels (fp64_trace_kernel in both forms) and the FP32 speculation
 # (packed two-wide instructions count once there: a lower bound).
-F_EXEC_FP64_ATTEMPT = 1022.8
-F_EXEC_FP32_ATTEMPT = 479.4
+F_EXEC_FP64_ATTEMPT = 953.4
+F_EXEC_FP32_ATTEMPT = 402.3
 # DRAM bytes (read + write) of one mixed_speculate_kernel launch on the
 # 1024x1024 4-spp frame, from ncu (single-pass dram__bytes_read.sum +
 # dram__bytes_write.sum, the warp-staged kernel): 0.52 MB read + 55.17 MB

@@ -22,10 +22,10 @@
 #include <cmath>
 
 #define GRRT_HD __host__ __device__ __forceinline__
-// The right-hand side is inlined at its call sites (seven per attempt) unless
-// the translation unit sets GRRT_RHS_CALL_F64, which makes the FP64 one a
-// call to one shared body (less code to fetch, a call per evaluation). The
-// FP32 one stays inlined: its kernels are issue-bound and lose to the calls.
+// The right-hand side is inlined at its call sites unless the translation unit
+// sets GRRT_RHS_CALL_F64, which makes the FP64 one a call to one shared body.
+// The device's FP64 body has its roundings written out, so calls and inlined
+// copies give the same bits.
 
 namespace grrt_b200 {
 
@@ -257,8 +257,8 @@ __device__ __forceinline__ Vec5<double> kerr_rhs_f64(const KerrHole& K, double p
 // range's ends. The FP32 passes are bound by issue (77% of the cycles), so an
 // instruction less here counts six times an attempt. With the attempt's packed
 // sums over four components (mixed_attempt_k1): a 1024^2 4-sample speculative
-// pass 5.89 -> 5.39 ms, the components' errors against FP64 unchanged to the
-// printed digits (median 6e-8 to 5e-7 over 2^20 states).
+// pass 5.89 -> 5.43 ms. Values are those of the generic body, its order of
+// products kept (the same bits on 2^20 states).
 __device__ __forceinline__ float rcp_approx(float x) {
     float y;
     asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));

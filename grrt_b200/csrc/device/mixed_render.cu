@@ -22,8 +22,8 @@
 // The FP64 trace inlines the right-hand side into its attempt: with the
 // roundings written out (kerr.cuh) every copy has the same bits, and without
 // the calls an attempt is 1,060 instructions instead of 1,600 (Kerr a=0.998,
-// 1024x1024, 4 spp on B200: FP64 form 31.7 -> 24.0 ms, the mixed form's
-// re-trace 6.7 -> 5.3 ms; one lone ray 2.53 -> 1.71 us an attempt).
+// 1024x1024, 4 spp on B200: FP64 form 31.9 -> 24.4 ms, the mixed form's
+// re-trace 6.7 -> 5.3 ms; one lone ray 2.53 -> 1.83 us an attempt).
 #include <cuda_runtime.h>
 
 #include <cstdint>
@@ -155,10 +155,12 @@ struct SpecStage {
 };
 }  // namespace
 
-// Five resident blocks per SM (at most 96 registers): the issue-bound FP32
-// pass gains more from the fifth block's warps than it loses to the few
-// spilled registers (four blocks: 8.8 ms, five: 8.2 ms on the 1024x1024 4-spp
-// frame on B200; six, with more spills, no better).
+// Five resident blocks per SM (at most 96 registers): the pass is bound by
+// issue (78% of the cycles), and six, with spills, are no better (1024x1024, 4
+// spp on B200: 4.98 ms, six 5.01). What a step needs beside the ray is kept
+// small: FP32 state and first stage in registers, the Carter constants, swept
+// angle and sample index in shared memory, the controller without branches
+// (5.43 -> 4.98 ms).
 template <bool kBatch>
 __global__ void __launch_bounds__(kMixThreads, 5)
 mixed_speculate_kernel(const __grid_constant__ DevScene S0, const DevTile tile, const __grid_constant__ DevBatch B,

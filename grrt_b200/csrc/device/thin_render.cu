@@ -4,7 +4,7 @@
 // GeodesicTracer::trace (src/geodesic_tracer.cpp:23-181) inside the loop of
 // Renderer::render (src/renderer.cpp:30-82), in the FP64 form, one lane per
 // pixel. This kernel serves the Hamiltonian diagnostic (GRRT_DIAG_HAMILTONIAN)
-// and the batched form's pixel schedules; the FP64 form's renders otherwise
+// and the batched form's pixel schedules where one was chosen; the FP64 form's renders otherwise
 // trace by samples with the per-sample work staged per warp
 // (fp64_trace_kernel in mixed_render.cu, the same arithmetic).
 //
@@ -14,10 +14,10 @@
 // converged in the expensive part. A lane whose pixel is done takes the next
 // pixel from a global counter with one warp-aggregated atomic, which keeps
 // warps full while ray lengths range from tens to thousands of steps.
-// One shared body of the FP64 right-hand side instead of seven inlined copies
-// per attempt: less code to fetch (Kerr a=0.998, 1024x1024, 4 spp: 46.4 ->
-// 43.4 ms for the FP64 form on B200). The FP64 form and the mixed form's
-// re-trace must use the same setting, so that their arithmetic is identical.
+// One shared body of the FP64 right-hand side: inlined copies were 20% faster on
+// small batches and 2-4% slower on large ones (64 cameras of 256x256: 37.0
+// against 37.8 ms on B200), since the lanes' scenes lie in global memory and
+// the inlined copies read them again. The bits are the same either way.
 #define GRRT_RHS_CALL_F64 1
 #include <cuda_runtime.h>
 
