@@ -740,6 +740,18 @@ const MixLaunchShape& mix_shape() {
 }
 }  // namespace
 
+// Resident blocks per SM of one camera's FP64 trace of n samples. With few
+// samples a lane the launch waits for its longest rays, whose steps are quicker
+// with fewer warps beside them: up to three samples a lane of the full grid
+// (227 k), three blocks are 0-8% faster than four (B200, Kerr a=0.998: 256x256
+// 1.22 -> 1.16 ms, 320x320 1.45 -> 1.34, 384x384 1.67 -> 1.59; two blocks 1.07,
+// 1.39, 1.68); above it the fourth block's warps win (512x512 2.39 against 2.46
+// ms, 1024x1024 with 4 spp 24.4 against 28.6).
+static int fp64_trace_blocks(int per_sm, int sms, size_t n) {
+    const size_t lanes = static_cast<size_t>(sms) * per_sm * kMixThreads;
+    return (per_sm > 3 && n <= 3 * lanes) ? 3 : per_sm;
+}
+
 DevMixedBuffers mixed_buffers(void* scratch, size_t n, unsigned* queue) {
     auto* base = static_cast<unsigned char*>(scratch);
     DevMixedBuffers mb;
@@ -873,7 +885,7 @@ cudaError_t launch_thin_fp64(const DevScene& S, const DevTile& tile, const ThinO
     if (e != cudaSuccess) return e;
     const MixLaunchShape& sh = mix_shape();
     const int need = static_cast<int>((n + kMixThreads - 1) / kMixThreads);
-    int blocks = sh.sms * sh.per_fp64;
+    int blocks = sh.sms * fp64_trace_blocks(sh.per_fp64, sh.sms, n);
     if (need < blocks) blocks = need;
     mark(0);
     fp64_trace_kernel<false, false><<<blocks, kMixThreads, 0, stream>>>(S, tile, DevBatch{}, mb, res.queue,
