@@ -55,7 +55,7 @@ struct GRRTBatch {
     int order = GRRT_BATCH_ORDER_ROUND_ROBIN;
     int blocks_per_sm = 0;  // 0 = as many as fit
     int block = 128;        // threads per block of the FP64 thin-disk batch kernel (64, 128, 256)
-    bool schedule_set = false;     // a schedule or block size was chosen (by the caller or the autotuner)
+    bool schedule_set = false;  // an FP64 schedule or block size was chosen (by the caller or the FP64 autotuner)
     bool no_sample_room = false;   // the default's sample scratch could not be had
     bool tuned = false;
     // device
@@ -632,7 +632,8 @@ extern "C" GRRT_EXPORT int grrt_batch_get_stats(GRRTBatch* b, GRRTStats* out) {
     return 0;
 }
 
-// Times candidate schedules on the batch itself and keeps the fastest.
+// Times candidate schedules on the batch itself and keeps the fastest; on an
+// error the batch keeps the schedule and knobs that it had.
 //   FP64 thin-disk batches: chunk size (64..4096) x chunk order x resident
 //     blocks per SM at 128 threads per block, then threads per block (64,
 //     128, 256) x resident blocks per SM at the best chunk and order; and the
@@ -653,10 +654,27 @@ struct Tuning {
     double tol_fp32, r_factor;
 };
 
+// Sets the schedule and knobs without making them the caller's choice.
 void apply(GRRTBatch* b, const Tuning& t) {
+    const bool chosen = b->schedule_set;
     grrt_batch_set_schedule(b, t.chunk, t.order, t.bps);
     grrt_batch_set_tuning(b, t.block, t.tol_fp32, t.r_factor);
+    b->schedule_set = chosen;
 }
+
+// What a batch had before the autotuner, put back unless it came to an end.
+struct Restore {
+    GRRTBatch* b;
+    Tuning t;
+    bool chosen, keep = false;
+    ~Restore() {
+        if (keep) return;
+        const std::string why = b->error;
+        apply(b, t);
+        b->schedule_set = chosen;
+        b->error = why;
+    }
+};
 
 // best of two timed runs; < 0 on error
 double time_batch(GRRTBatch* b, void* out) {
@@ -695,6 +713,8 @@ extern "C" GRRT_EXPORT int grrt_batch_autotune(GRRTBatch* b, const char* cache_p
     if (!b) return -1;
     if (!batch_ensure_device(b)) return -1;
     const std::string key = batch_key(*b);
+    const bool mixed = !b->spectral && b->form == GRRT_FORM_MIXED;
+    const bool fp64 = !b->spectral && !mixed;
     if (cache_path && cache_path[0]) {
         std::ifstream in(cache_path);
         std::string line;
@@ -708,6 +728,7 @@ extern "C" GRRT_EXPORT int grrt_batch_autotune(GRRTBatch* b, const char* cache_p
                                         kbuf, &t.chunk, &t.order, &t.bps, &ms, &t.block, &t.tol_fp32, &t.r_factor);
             if (got == 8 && key == kbuf) {
                 apply(b, t);
+                if (fp64) b->schedule_set = true;
                 b->tuned = true;
                 if (best_ms) *best_ms = ms;
                 return 0;
@@ -725,9 +746,11 @@ extern "C" GRRT_EXPORT int grrt_batch_autotune(GRRTBatch* b, const char* cache_p
             return -1;
         tune_out = b->d_out;
     }
-    const bool mixed = !b->spectral && b->form == GRRT_FORM_MIXED;
-    b->schedule_set = true;
     Tuning cur{b->chunk_size, b->order, b->blocks_per_sm, b->block, b->cams[0]->tol_fp32, b->cams[0]->mixed_r_factor};
+    Restore restore{b, cur, b->schedule_set};
+    // what is timed is the candidate, and the FP64 form's result a choice; the
+    // mixed form's says nothing about the FP64 one
+    if (fp64) b->schedule_set = true;
     Tuning best_t = cur;
     double best = 1e30;
     auto consider = [&](const Tuning& t) -> int {
@@ -823,6 +846,7 @@ extern "C" GRRT_EXPORT int grrt_batch_autotune(GRRTBatch* b, const char* cache_p
         }
     }
     apply(b, best_t);
+    restore.keep = true;
     b->tuned = true;
     if (best_ms) *best_ms = best;
     if (cache_path && cache_path[0]) {

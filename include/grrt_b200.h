@@ -168,8 +168,11 @@ typedef struct GRRTBatch GRRTBatch;
  * samples with the warp staging of the single FP64 render, then resolved into
  * pixels; the chunk size and the threads per block do not apply (other
  * batches take it as camera-major). An FP64 thin-disk batch whose schedule was
- * never set is traced that way too while its scratch stays below 1 GB; setting
- * a schedule or a block size, or the autotuner, decides otherwise. */
+ * never chosen is traced that way too while its scratch stays below 1 GB
+ * (grrt_batch_get_schedule then reports the pixel schedule that it would have).
+ * Chosen: by grrt_batch_set_schedule, with any values; by another block size
+ * than the present one in grrt_batch_set_tuning (its tolerances alone choose
+ * nothing); by the autotuner in the FP64 form (not in the mixed form). */
 #define GRRT_BATCH_ORDER_CAMERA_MAJOR 0
 #define GRRT_BATCH_ORDER_ROUND_ROBIN 1
 #define GRRT_BATCH_ORDER_SAMPLES 2
@@ -195,7 +198,8 @@ GRRT_EXPORT int grrt_batch_get_tuning(const GRRTBatch* batch, int* block, double
  * {3, 4}, each candidate held to the mixed form's bar against the batch's
  * FP64 render (every pixel within 1e-4 relative) and dropped if it misses it.
  * cache_path (may be NULL) stores and reuses the choice for an identical
- * batch. best_ms may be NULL. */
+ * batch. best_ms may be NULL. After an error the batch has the settings that it
+ * had before. */
 GRRT_EXPORT int grrt_batch_autotune(GRRTBatch* batch, const char* cache_path, double* best_ms);
 /* framebuffers[i]: float[W_i*H_i*4] host buffer of camera i (NULL skips it). */
 GRRT_EXPORT int grrt_batch_render(GRRTBatch* batch, float* const* framebuffers);
