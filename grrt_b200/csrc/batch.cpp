@@ -56,7 +56,6 @@ struct GRRTBatch {
     int blocks_per_sm = 0;  // 0 = as many as fit
     int block = 128;        // threads per block of the FP64 thin-disk batch kernel (64, 128, 256)
     bool schedule_set = false;  // an FP64 schedule or block size was chosen (by the caller or the FP64 autotuner)
-    bool no_sample_room = false;   // the default's sample scratch could not be had
     bool tuned = false;
     // device
     int device = -1;
@@ -173,13 +172,14 @@ struct GRRTBatch {
     bool by_samples() const {
         if (spectral || form == GRRT_FORM_MIXED) return false;
         if (order == GRRT_BATCH_ORDER_SAMPLES) return true;
-        return !schedule_set && !no_sample_room && total_samples > 0 && total_samples <= 0x7f000000ull &&
+        return !schedule_set && total_samples > 0 && total_samples <= 0x7f000000ull &&
                mixed_scratch_bytes_for(total_samples) <= kDefaultSampleScratch;
     }
 
-    int max_blocks_per_sm() const {
+    int max_blocks_per_sm() const { return max_blocks_per_sm(by_samples()); }
+    int max_blocks_per_sm(bool samples) const {
         if (spectral) return vol_spectral_batch_max_blocks_per_sm();
-        if (by_samples()) return fp64_batch_max_blocks_per_sm();
+        if (samples) return fp64_batch_max_blocks_per_sm();
         return form == GRRT_FORM_MIXED ? mixed_batch_max_blocks_per_sm() : thin_batch_max_blocks_per_sm(block);
     }
 
@@ -197,11 +197,11 @@ struct GRRTBatch {
         return true;
     }
 
-    int blocks() const {
+    int blocks(bool samples) const {
         int dev = 0, sms = 0;
         cudaGetDevice(&dev);
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        const int maxb = max_blocks_per_sm();
+        const int maxb = max_blocks_per_sm(samples);
         const int per = (blocks_per_sm > 0 && blocks_per_sm < maxb) ? blocks_per_sm : maxb;
         return sms * per;
     }
@@ -219,21 +219,27 @@ struct GRRTBatch {
         if (e == cudaSuccess) mixed_bytes = need;
         return e;
     }
-    bool sample_scratch() { return sample_scratch_error() == cudaSuccess; }
+    // The same for the default trace by samples: only a small part of the free
+    // memory is taken without being asked for, and a refusal is no error (asked
+    // again at the next render).
+    bool default_sample_scratch() {
+        const size_t need = mixed_scratch_bytes_for(total_samples);
+        if (need <= mixed_bytes) return true;
+        size_t room = 0, total = 0;
+        const bool ok = cudaMemGetInfo(&room, &total) == cudaSuccess && need <= room / 8 &&
+                        sample_scratch_error() == cudaSuccess;
+        if (!ok) cudaGetLastError();
+        return ok;
+    }
 
     // Enqueue one batched render (as a CUDA graph replay) on stream s: RGBA
     // (float4 per pixel) or, for a spectral batch, the cubes (doubles).
     int launch(void* out, cudaStream_t s) {
         if (!upload_schedule()) return -1;
         const bool mixed = !spectral && form == GRRT_FORM_MIXED;
-        bool samples = by_samples();
-        if (samples && order != GRRT_BATCH_ORDER_SAMPLES && !sample_scratch()) {
-            // the default's scratch is not to be had: pixel by pixel needs none
-            cudaGetLastError();
-            no_sample_room = true;
-            samples = false;
-        }
-        const int nb = blocks();
+        // where the default's scratch is not to be had: pixel by pixel needs none
+        const bool samples = by_samples() && (order == GRRT_BATCH_ORDER_SAMPLES || default_sample_scratch());
+        const int nb = blocks(samples);
         if (spectral) {
             const size_t need = static_cast<size_t>(4) * nb_max * nb * vol_spectral_batch_threads();
             if (need > spec_scratch_elems) {

@@ -168,8 +168,9 @@ typedef struct GRRTBatch GRRTBatch;
  * samples with the warp staging of the single FP64 render, then resolved into
  * pixels; the chunk size and the threads per block do not apply (other
  * batches take it as camera-major). An FP64 thin-disk batch whose schedule was
- * never chosen is traced that way too while its scratch stays below 1 GB
- * (grrt_batch_get_schedule then reports the pixel schedule that it would have).
+ * never chosen is traced that way too while its scratch stays below 1 GB and
+ * an eighth of the free device memory (grrt_batch_get_schedule then reports the
+ * pixel schedule that it would have).
  * Chosen: by grrt_batch_set_schedule, with any values; by another block size
  * than the present one in grrt_batch_set_tuning (its tolerances alone choose
  * nothing); by the autotuner in the FP64 form (not in the mixed form). */

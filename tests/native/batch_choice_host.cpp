@@ -112,6 +112,22 @@ int main(int argc, char** argv) {
         fail_at = 0;
         grrt_batch_set_precision(b, GRRT_FORM_FP64);
         render(b, "after");
+    } else if (what == "no_room") {
+        // two cameras of 2048 x 2048: 0.5 GB of sample scratch
+        grrt_batch_destroy(b);
+        b = make(2, 2048, 2048);
+        fake::room = size_t(300) << 20;
+        render(b, "full");
+        fake::room = size_t(180) << 30;
+        render(b, "freed");
+        render(b, "replay");
+    } else if (what == "little_room") {
+        grrt_batch_destroy(b);
+        b = make(2, 2048, 2048);
+        fake::room = size_t(1) << 30;
+        render(b, "little");
+        grrt_batch_set_schedule(b, 256, GRRT_BATCH_ORDER_SAMPLES, 0);
+        render(b, "asked");
     } else if (what == "too_many") {
         // 1.05 GB of sample scratch
         grrt_batch_destroy(b);

@@ -1,7 +1,7 @@
 """Which kernel an FP64 thin-disk batch renders with (the trace by samples is
 the default, a chosen schedule or block size decides otherwise) and what the
-autotuner leaves behind. The library's host code on a host stand-in of the
-CUDA runtime; CPU only."""
+autotuner and scarce memory leave behind. The library's host code on a host
+stand-in of the CUDA runtime; CPU only."""
 import os
 import re
 import subprocess
@@ -73,3 +73,14 @@ def test_failed_autotune_changes_nothing(program, what):
     assert s["autotune"]["rc"] == -1
     a = s["after"]
     assert (a["rc"], a["ran"], a["schedule"], a["block"]) == (0, "samples", "256,1,0", "128")
+
+
+def test_scratch_only_while_there_is_room(program):
+    s = program("no_room")
+    assert s["full"]["rc"] == 0 and s["full"]["ran"] == "pixels"
+    assert s["freed"]["ran"] == s["replay"]["ran"] == "samples"  # asked again, not given up for good
+    assert s["freed"]["took"] == "memory" and s["replay"]["took"] == "none"
+    # half of what is free is not taken without being asked for
+    s = program("little_room")
+    assert s["little"]["ran"] == "pixels"
+    assert s["asked"]["rc"] == 0 and s["asked"]["ran"] == "samples"
