@@ -69,6 +69,7 @@ struct GRRTSurrogate {
     // chain of the activations' gradients on `stream`
     cudaStream_t side[2] = {};
     cudaEvent_t ev_fork = nullptr, ev_join[2] = {};
+    cudaEvent_t ev_piece[2] = {};  // ends of the last two pieces of a training run
     std::string error;
 
     unsigned char* d_net = nullptr;  // holds the buffers below, up to the error flag
@@ -115,8 +116,7 @@ struct GRRTSurrogate {
 
     ~GRRTSurrogate() {
         if (device >= 0) cudaSetDevice(device);
-        for (cudaStream_t q : {stream, side[0], side[1]})
-            if (q) cudaStreamSynchronize(q);
+        drain();
         free_workspace();
         dfree(loss_hist);
         free_inference();
@@ -124,7 +124,7 @@ struct GRRTSurrogate {
         dfree(d_Y);
         dfree(d_net);
         if (h_err) cudaFreeHost(h_err);
-        for (cudaEvent_t e : {ev_fork, ev_join[0], ev_join[1]})
+        for (cudaEvent_t e : {ev_fork, ev_join[0], ev_join[1], ev_piece[0], ev_piece[1]})
             if (e) cudaEventDestroy(e);
         for (cudaStream_t q : {stream, side[0], side[1]})
             if (q) cudaStreamDestroy(q);
@@ -248,10 +248,21 @@ struct GRRTSurrogate {
         return !fail(umma_gemm_bf16(A, lda, B, ldb, M, N, K, sp, ep, d_err, stream), "tensor-core GEMM");
     }
 
+    // The code that a kernel which has ended left in the error flag.
+    int gemm_error_code() const { return *static_cast<volatile int*>(h_err); }
+
+    // Waits for all of the network's streams; false if a kernel failed.
+    bool drain() {
+        bool ok = true;
+        for (cudaStream_t q : {stream, side[0], side[1]})
+            if (q) ok = !fail(cudaStreamSynchronize(q), "surrogate kernels") && ok;
+        return ok;
+    }
+
     // Waits for the stream; false if a kernel failed or reported a timeout.
     bool check_gemm_errors() {
         if (fail(cudaStreamSynchronize(stream), "tensor-core kernels")) return false;
-        const int code = *static_cast<volatile int*>(h_err);
+        const int code = gemm_error_code();
         if (code != 0) {
             error = "tensor-core kernel reported a timeout (code " + std::to_string(code) + ")";
             *h_err = 0;
@@ -317,7 +328,7 @@ struct GRRTSurrogate {
         if (ws_batch == B) return true;
         for (cudaStream_t& q : side)
             if (!q && fail(cudaStreamCreateWithFlags(&q, cudaStreamNonBlocking), "cudaStreamCreate")) return false;
-        for (cudaEvent_t* e : {&ev_fork, &ev_join[0], &ev_join[1]})
+        for (cudaEvent_t* e : {&ev_fork, &ev_join[0], &ev_join[1], &ev_piece[0], &ev_piece[1]})
             if (!*e && fail(cudaEventCreateWithFlags(e, cudaEventDisableTiming), "cudaEventCreate")) return false;
         free_workspace();
         const size_t b = static_cast<size_t>(B);
@@ -427,6 +438,7 @@ struct GRRTSurrogate {
 
     // `steps` Adam steps at batch B. Learning rate: lr for the first half, then
     // halved every eighth of the run (piecewise constant).
+    static constexpr int kPieceSteps = 256;
     bool train(int steps, int B, double lr, float* loss_out) {
         if (n_data == 0) return !fail_msg("no training set: call grrt_surrogate_generate first");
         if (steps <= 0 || B < 128 || B % 128 != 0 || B > (1 << 20)) return !fail_msg("bad steps or batch size");
@@ -442,34 +454,48 @@ struct GRRTSurrogate {
             if (!dalloc(&loss_hist, static_cast<size_t>(need))) return !fail_msg("cudaMalloc(loss history)");
             hist_cap = need;
         }
-        // one eager step (it also sets the kernels' launch attributes), then one graph for all rates
+        // The steps are enqueued in pieces (a rate's steps, at most kPieceSteps),
+        // one piece ahead of the GPU: after a kernel's timeout no more than the
+        // next piece still runs, each of its waits to the limit, and the GPU
+        // never waits for the check.
         cudaGraphExec_t ge = nullptr;
         const int phases[] = {steps / 2, steps / 8, steps / 8, steps / 8, steps - steps / 2 - 3 * (steps / 8)};
         double rate = lr;
-        bool ok = true, first = true;
+        bool ok = true;
+        int pieces = 0;
         for (int ph = 0; ok && ph < 5; ++ph, rate *= 0.5) {
-            int n = phases[ph];
-            if (n <= 0) continue;
+            if (phases[ph] <= 0) continue;
             ok = !fail(launch_set_float(d_lr, static_cast<float>(rate), stream), "learning rate");
-            if (ok && first) {
-                ok = enqueue_train_step(B);
-                first = false;
-                --n;
+            for (int done = 0; ok && done < phases[ph]; done += kPieceSteps) {
+                ok = enqueue_steps(B, std::min(kPieceSteps, phases[ph] - done), pieces == 0, &ge) &&
+                     !fail(cudaEventRecord(ev_piece[pieces % 2], stream), "event");
+                ++pieces;
+                if (ok && pieces > 1)
+                    ok = !fail(cudaEventSynchronize(ev_piece[pieces % 2]), "training") && gemm_error_code() == 0;
             }
-            if (ok && n > 0 && !ge) ok = capture_train_step(B, &ge);
-            for (int i = 0; ok && i < n; ++i) ok = !fail(cudaGraphLaunch(ge, stream), "graph launch");
         }
-        const cudaError_t se = cudaStreamSynchronize(stream);
+        calibrated = false;
+        ok = drain() && ok;
         if (ge) cudaGraphExecDestroy(ge);
-        if (!ok || fail(se, "training")) return false;
+        if (!check_gemm_errors() || !ok) return false;
         std::vector<float> hist(static_cast<size_t>(steps));
         if (fail(copy(hist.data(), loss_hist + t0, sizeof(float) * steps, cudaMemcpyDeviceToHost), "read loss"))
             return false;
         if (loss_out) std::memcpy(loss_out, hist.data(), sizeof(float) * steps);
         last_loss = hist.back();
         steps_done += steps;
-        calibrated = false;
-        return check_gemm_errors();
+        return true;
+    }
+
+    // n training steps: the run's first one eager (it also sets the kernels'
+    // launch attributes), the others by one graph for all rates.
+    bool enqueue_steps(int B, int n, bool first, cudaGraphExec_t* ge) {
+        if (first && !enqueue_train_step(B)) return false;
+        if (first) --n;
+        if (n > 0 && !*ge && !capture_train_step(B, ge)) return false;
+        for (int i = 0; i < n; ++i)
+            if (fail(cudaGraphLaunch(*ge, stream), "graph launch")) return false;
+        return true;
     }
 
     bool capture_train_step(int B, cudaGraphExec_t* ge) {
@@ -808,8 +834,8 @@ extern "C" GRRT_EXPORT int grrt_surrogate_gradients(GRRTSurrogate* s, const floa
     if (s->fail(s->copy(s->Xb, h_in, sizeof(float) * kIn * n, cudaMemcpyHostToDevice), "upload") ||
         s->fail(s->copy(s->Yb, h_y, sizeof(float) * kYCols * n, cudaMemcpyHostToDevice), "upload"))
         return -1;
-    if (!s->enqueue_fwd_bwd(n)) return -1;
-    if (s->fail(cudaStreamSynchronize(s->stream), "gradients") || !s->check_gemm_errors()) return -1;
+    const bool enqueued = s->enqueue_fwd_bwd(n);
+    if (!s->drain() || !s->check_gemm_errors() || !enqueued) return -1;
     float l = 0.0f;
     if (s->fail(s->copy(h_grad, s->d_grad, sizeof(float) * ParamLayout::total, cudaMemcpyDeviceToHost), "read") ||
         s->fail(s->copy(&l, s->loss, sizeof(float), cudaMemcpyDeviceToHost), "read"))

@@ -21,6 +21,7 @@ inline unsigned long long queued = 0, done = 0;  // operations so far
 inline std::vector<Op>* capture = nullptr;
 inline size_t room = size_t(1) << 40, used = 0;  // device memory
 inline std::map<void*, size_t> sizes;
+inline std::map<cudaStream_t, unsigned long long> waited;  // operations queued at a stream's last synchronisation
 inline double now_ms = 0.0;  // device clock, advanced by the work
 
 inline void run_until(unsigned long long n) {
@@ -112,7 +113,11 @@ cudaError_t cudaMemsetAsync(void* d, int v, size_t n, cudaStream_t) {
     return cudaSuccess;
 }
 cudaError_t cudaDeviceSynchronize(void) { fake::run_all(); return cudaSuccess; }
-cudaError_t cudaStreamSynchronize(cudaStream_t) { fake::run_all(); return cudaSuccess; }
+cudaError_t cudaStreamSynchronize(cudaStream_t s) {
+    fake::waited[s] = fake::queued;
+    fake::run_all();
+    return cudaSuccess;
+}
 cudaError_t cudaStreamCreateWithFlags(cudaStream_t* s, unsigned) {
     *s = reinterpret_cast<cudaStream_t>(new int);
     return cudaSuccess;
