@@ -133,10 +133,11 @@ __device__ __forceinline__ double simplex_corner(double x, double y, double z, i
 
 __device__ __forceinline__ double simplex3(const int* __restrict__ P, double x, double y, double z) {
     constexpr double F3 = 1.0 / 3.0, G3 = 1.0 / 6.0;
-    const double s = (x + y + z) * F3;
-    const int i = static_cast<int>(floor(x + s)), j = static_cast<int>(floor(y + s)), k = static_cast<int>(floor(z + s));
-    const double t = (i + j + k) * G3;
-    const double x0 = x - (i - t), y0 = y - (j - t), z0 = z - (k - t);
+    const double sum = __dadd_rn(__dadd_rn(x, y), z);
+    const int i = static_cast<int>(floor(__fma_rn(sum, F3, x))), j = static_cast<int>(floor(__fma_rn(sum, F3, y))),
+              k = static_cast<int>(floor(__fma_rn(sum, F3, z)));
+    const double n = i + j + k;
+    const double x0 = x - __fma_rn(-n, G3, i), y0 = y - __fma_rn(-n, G3, j), z0 = z - __fma_rn(-n, G3, k);
     int i1, j1, k1, i2, j2, k2;
     if (x0 >= y0) {
         if (y0 >= z0) { i1 = 1; j1 = 0; k1 = 0; i2 = 1; j2 = 1; k2 = 0; }
@@ -225,15 +226,17 @@ __device__ __forceinline__ void v_redshift(const DevVolume& V, double pt, double
         uphi = __dmul_rn(Omg, ut);
     } else {
         const double E = V.E_isco, L = V.L_isco;
-        const double Delta = r * r - 2.0 * M * r + a * a;
-        const double c = ct;
-        const double Sigma = r * r + a * a * c * c;
-        ut = (E * (r * r + a * a + 2.0 * M * a * a / r) - 2.0 * M * a * L / r) / Delta;
-        uphi = (L * (1.0 - 2.0 * M / r) + 2.0 * M * a * E / r) / Delta;
-        const double EaL = E * (r * r + a * a) - a * L;
-        const double LaE = L - a * E;
-        const double R = EaL * EaL - Delta * (r * r + LaE * LaE);
-        ur = -sqrt(vmax(0.0, R)) / Sigma;
+        const double a2 = __dmul_rn(a, a), r2 = __dmul_rn(r, r), m2a = __dmul_rn(m2, a);
+        const double ra = __dadd_rn(r2, a2);
+        const double Delta = __dadd_rn(__fma_rn(-m2, r, r2), a2);
+        const double Sigma = __fma_rn(__dmul_rn(a2, ct), ct, r2);
+        const double sum = __dadd_rn(ra, __ddiv_rn(__dmul_rn(m2a, a), r));
+        ut = __ddiv_rn(__fma_rn(E, sum, -__ddiv_rn(__dmul_rn(m2a, L), r)), Delta);
+        uphi = __ddiv_rn(__fma_rn(L, __dadd_rn(1.0, -__ddiv_rn(m2, r)), __ddiv_rn(__dmul_rn(m2a, E), r)), Delta);
+        const double EaL = __fma_rn(E, ra, -__dmul_rn(a, L));
+        const double LaE = __fma_rn(-a, E, L);
+        const double R = __fma_rn(EaL, EaL, -__dmul_rn(Delta, __fma_rn(LaE, LaE, r2)));
+        ur = __ddiv_rn(-__dsqrt_rn(vmax(0.0, R)), Sigma);
     }
     pue = __fma_rn(pph, uphi, __fma_rn(pt, ut, __dmul_rn(pr, ur)));
     g = div_f64(pue, __dmul_rn(pt, V.ut_obs));
