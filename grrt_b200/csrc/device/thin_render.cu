@@ -14,10 +14,13 @@
 // converged in the expensive part. A lane whose pixel is done takes the next
 // pixel from a global counter with one warp-aggregated atomic, which keeps
 // warps full while ray lengths range from tens to thousands of steps.
-// One shared body of the FP64 right-hand side: inlined copies were 20% faster on
-// small batches and 2-4% slower on large ones (64 cameras of 256x256: 37.0
-// against 37.8 ms on B200), since the lanes' scenes lie in global memory and
-// the inlined copies read them again. The bits are the same either way.
+// The batch calls one shared body of the FP64 right-hand side: inlined copies
+// were 20% faster on small batches and 2-4% slower on large ones (64 cameras of
+// 256x256: 37.0 against 37.8 ms on B200), since the lanes' scenes lie in global
+// memory and the inlined copies read them again. One camera's scene is a kernel
+// parameter: inlined, with the controller that does not form the error
+// quotient (diagnostic frames of Kerr a=0.998: 256x256 1.94 -> 1.43 ms, 1024x1024
+// 9.83 -> 9.06). The bits are the same either way.
 #define GRRT_RHS_CALL_F64 1
 #include <cuda_runtime.h>
 
@@ -200,9 +203,14 @@ __device__ __forceinline__ void thin_loop(const DevScene& S0, const DevBatch& B,
                 k1_ok = true;
             }
             Vec5<double> y5, k7;
-            const double err = dp45_attempt_k1<double>(S.M, S.a, pt, pph, y, dl, k1, y5, k7);
+            auto rhs = [&](const Vec5<double>& s) {
+                if constexpr (kBatch) return kerr_rhs<double>(S.M, S.a, pt, pph, s);
+                else return kerr_rhs_f64(KerrHole{S.M, S.a, S.a2, S.m2}, pt, pph, s.r, s.th, s.pr, s.pth);
+            };
+            const ErrQuotient err = dp45_attempt_f64(rhs, y, dl, k1, y5, k7);
             ++n_attempts;
-            const StepDecision d = pi_control(err, S.tol, dl, retry, y5.r);
+            const StepDecision d = kBatch ? pi_control(div_f64(err.num, err.den), S.tol, dl, retry, y5.r)
+                                          : pi_control_q(err, S.tol, dl, retry, y5.r);
             if (d.accept) {
                 ++n_accepted;
                 // equatorial crossing (src/geodesic_tracer.cpp:156-176): every
