@@ -145,7 +145,8 @@ static __constant__ RhsConst kRhs = {
 // one add to 1.5 * 2^52 rounded down (its low word then holds floor(|x| 4/pi)
 // + 1) instead of two conversions. The signs go into the polynomials' factors
 // and the clamp into the sine's argument (sin x = x that close to 0), beside
-// the chain through z.
+// the chain through z. (x = -0 gives -1e-10 where fast_sincos gives 1e-10; no
+// ray has it: colatitudes start above 0, and a sum that cancels is +0.)
 __device__ __forceinline__ void sincos_clamped_f64(double x, double& s, double& c) {
     auto flip = [](double v, unsigned sign) {
         return __hiloint2double(__double2hiint(v) ^ static_cast<int>(sign), __double2loint(v));
@@ -190,12 +191,13 @@ __device__ __forceinline__ void sincos_clamped_f64(double x, double& s, double& 
 // the residuals exact in fused multiply-adds (P. Markstein, IBM J. Res. Dev.
 // 34, 1990). The cubic step rounds up, so that the last one starts from above
 // and also rounds an all-ones significand, its one exception, correctly.
-// x = inf gives 0; a zero or subnormal x or result is not handled (NaN or 0).
+// x = inf gives 0, NaN NaN: the approximation sees |x|, the residuals a number
+// that is finite. A zero or subnormal x or result is not handled (NaN or 0).
 __device__ __forceinline__ double recip_f64(double x) {
     const int hi = __double2hiint(x);
     const double xa = __hiloint2double(min(hi & 0x7fffffff, 0x7fe00000), __double2loint(x));
     double y;
-    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(xa));
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(fabs(x)));
     double e = __fma_rn(-xa, y, 1.0);
     y = __fma_ru(y, __fma_rn(e, e, e), y);
     e = __fma_rn(-xa, y, 1.0);

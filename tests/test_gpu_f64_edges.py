@@ -1,0 +1,49 @@
+"""FP64 building blocks at the ends of their ranges (NaN, infinities, numbers
+whose products overflow, empty and reversed tables) give the bits of the plain
+operations they stand for, and scenes that reach them give the frames they
+gave before the blocks were written. Exact but where a bound is given."""
+import ctypes as C
+import os
+import subprocess
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+SRC = os.path.join(ROOT, "tests", "native", "device_f64_edges.cu")
+OUT = os.path.join(ROOT, "_build", "test", "libf64edges.so")
+NAN, INF = np.nan, np.inf
+
+
+@pytest.fixture(scope="module")
+def edges(need_gpu):
+    os.makedirs(os.path.dirname(OUT), exist_ok=True)
+    subprocess.run(["/usr/local/cuda/bin/nvcc", "-std=c++17", "-O3", "-gencode", "arch=compute_100a,code=sm_100a",
+                    "-shared", "-cudart", "static", "-Xcompiler", "-fPIC", "-ccbin", "/usr/bin/g++", "-o", OUT, SRC],
+                   check=True)
+    lib = C.CDLL(OUT)
+
+    def run(kind, rows):
+        rows = np.ascontiguousarray(rows, dtype=np.float64)
+        fast, plain = np.empty((len(rows), 2)), np.empty((len(rows), 2))
+        p = [a.ctypes.data_as(C.c_void_p) for a in (rows, fast, plain)]
+        assert lib.f64_edges(kind, p[0], len(rows), p[1], p[2]) == 0
+        return rows, fast, plain
+
+    return run
+
+
+def assert_same(result):
+    """Equal bits, any NaN like any other."""
+    rows, fast, plain = result
+    same = (fast.view(np.uint64) == plain.view(np.uint64)) | (np.isnan(fast) & np.isnan(plain))
+    bad = np.nonzero(~same.all(axis=1))[0]
+    assert len(bad) == 0, (len(bad), rows[bad[:4]], fast[bad[:4]], plain[bad[:4]])
+
+
+def test_reciprocal_of_nan_and_infinity(edges):
+    odd = [NAN, -NAN, INF, -INF, 1.0, -3.0, 2.0 ** 1022, 2.0 ** 1023]
+    x = [v for v in odd if not 2.0 ** 1022 <= abs(v) < INF] + [2.0 ** 1021]  # results of normal range, or 0
+    assert_same(edges(0, [(a, b) for a in odd + [0.0] for b in x]))
