@@ -78,8 +78,10 @@ struct ErrQuotient {
 };
 
 // The error norm of dp45_attempt_k1 as the quotient it is, the largest one
-// picked by a tree: with every term finite the order of the comparisons does
-// not matter. qe: the error sum up to the sixth stage.
+// picked by a tree. Where the products of the comparisons cannot overflow, the
+// order of the comparisons does not matter but for quotients within a rounding
+// of each other, where either may be taken. qe: the error sum up to the sixth
+// stage.
 __device__ __forceinline__ ErrQuotient error_quotient(const Vec5<double>& y5, double h, const Vec5<double>& k7,
                                                       const Vec5<double>& qe) {
     const DpConst& C = kDp;
@@ -99,7 +101,7 @@ __device__ __forceinline__ ErrQuotient error_quotient(const Vec5<double>& y5, do
     int top = 0;
 #pragma unroll
     for (int i = 0; i < 5; ++i) top = max(top, max(__double2hiint(q[i].num), __double2hiint(q[i].den)));
-    if (top >= 0x7ff00000) {  // an infinity or a NaN: the terms in order, a NaN skipped
+    if (top >= 0x5ff00000) {  // 2^512, an infinity or a NaN: the terms in order, a NaN skipped
         ErrQuotient m{0.0, 1.0};
         for (int i = 0; i < 5; ++i) m = larger(m, q[i]);
         return m;

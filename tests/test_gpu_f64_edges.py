@@ -47,3 +47,15 @@ def test_reciprocal_of_nan_and_infinity(edges):
     odd = [NAN, -NAN, INF, -INF, 1.0, -3.0, 2.0 ** 1022, 2.0 ** 1023]
     x = [v for v in odd if not 2.0 ** 1022 <= abs(v) < INF] + [2.0 ** 1021]  # results of normal range, or 0
     assert_same(edges(0, [(a, b) for a in odd + [0.0] for b in x]))
+
+
+@pytest.mark.parametrize("top", [1e3, 1e150, 1e160, 1e300])
+def test_largest_quotient(edges, top):
+    rng = np.random.default_rng(11)
+    n = 20000
+    span = np.log10(top)
+    rows = np.concatenate([10.0 ** rng.uniform(-30, span, (n, 5)), 10.0 ** rng.uniform(-12, span, (n, 5))], axis=1)
+    odd = rng.random((n, 10)) < 0.05
+    rows[odd] = rng.choice([0.0, NAN, INF, -INF, 1e-9, top], int(odd.sum()))
+    rows *= np.where(rng.random((n, 10)) < 0.5, -1.0, 1.0)
+    assert_same(edges(1, rows))
