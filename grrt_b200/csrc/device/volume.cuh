@@ -243,10 +243,12 @@ __device__ __forceinline__ void v_redshift(const DevVolume& V, double pt, double
 }
 
 // Table coordinate of a log-spaced axis of length len (src/opacity.cpp:218-224).
+// The distance from the axis' start is clamped before the quotient, which has
+// to be finite: a frequency bin of 0 or infinity has an infinite lv.
 __device__ __forceinline__ void log_locate(double lv, double lo, double len, double inv_len, int n, int& idx,
                                            double& frac) {
-    double t = __dmul_rn(div_by(__dadd_rn(lv, -lo), len, inv_len), static_cast<double>(n - 1));
-    t = vclamp(t, 0.0, static_cast<double>(n - 2));
+    const double d = vmin(vmax(__dadd_rn(lv, -lo), 0.0), len);
+    const double t = vmin(__dmul_rn(div_by(d, len, inv_len), static_cast<double>(n - 1)), static_cast<double>(n - 2));
     idx = table_index(t, 0, n - 2);
     frac = __dadd_rn(t, -static_cast<double>(idx));
 }

@@ -59,3 +59,33 @@ def test_largest_quotient(edges, top):
     rows[odd] = rng.choice([0.0, NAN, INF, -INF, 1e-9, top], int(odd.sum()))
     rows *= np.where(rng.random((n, 10)) < 0.5, -1.0, 1.0)
     assert_same(edges(1, rows))
+
+
+def test_table_cell_of_infinite_coordinates(edges):
+    rng = np.random.default_rng(12)
+    rows = [(lv, 13.0, 19.3, 60) for lv in (INF, -INF, NAN, 13.0, 19.3, np.nextafter(19.3, 20), 12.9, -323.0, 308.2)]
+    rows += [(lv, -18.0, -6.0, 100) for lv in (INF, -INF, NAN, 0.0, -0.0, -18.0, -6.0, -320.0)]
+    rows += [(lv, 13.0, 19.3, 60) for lv in rng.uniform(12.0, 21.0, 20000)]
+    assert_same(edges(2, rows))
+
+
+def spectral(grrt, bins, **kw):
+    """A small cube at the given bins, tables laid out for ordinary ones."""
+    R = grrt.Renderer(grrt.config_params(3, width=32, height=24, **kw), freqs=grrt.log_bins(n=4))
+    R.freqs = np.array(bins, dtype=np.float64)
+    grrt.lib().grrt_set_frequency_bins(R.ctx, R.freqs.ctypes.data_as(C.POINTER(C.c_double)), len(bins))
+    return R.render_spectral(), R.stats()
+
+
+@pytest.mark.parametrize("odd,like", [(0.0, 1e-3), (INF, 1e300)])
+def test_a_bin_at_the_end_of_the_range_leaves_the_others(grrt, need_gpu, odd, like):
+    """The opacity of a frequency below (above) the table is the table's end, so
+    a bin at 0 (infinity) steers the march as any other frequency out there."""
+    f = grrt.log_bins(n=4)
+    a, sa = spectral(grrt, [f[0], f[1], odd, f[2]])  # the third of four is the one that sets the step length
+    b, sb = spectral(grrt, [f[0], f[1], like, f[2]])
+    others = [0, 1, 3]
+    assert (b[..., others] > 0).any()
+    np.testing.assert_array_equal(a[..., others], b[..., others])
+    for key in ("attempts", "march_steps", "physics_steps", "bin_updates"):
+        assert sa[key] == sb[key], key
