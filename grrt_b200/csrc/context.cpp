@@ -260,6 +260,9 @@ bool GRRTContext::ensure_device() {
         V.rho_scale = vol->rho_scale;
         V.noise_scale = vol->noise_scale;
         V.inv_noise = 1.0 / V.noise_scale;
+        // an infinite scale: quotients by any finite number with reciprocal 0 are
+        // 0, as those by infinity are (div_by needs a finite divisor)
+        if (std::isinf(V.noise_scale)) V.noise_scale = 1.0;
         V.turbulence = vol->cfg.turbulence;
         V.octaves = vol->cfg.noise_octaves;
         V.n_r = vol->n_r;

@@ -89,3 +89,14 @@ def test_a_bin_at_the_end_of_the_range_leaves_the_others(grrt, need_gpu, odd, li
     np.testing.assert_array_equal(a[..., others], b[..., others])
     for key in ("attempts", "march_steps", "physics_steps", "bin_updates"):
         assert sa[key] == sb[key], key
+
+
+def test_an_infinite_noise_scale_is_uniform_matter(grrt, need_gpu):
+    """All coordinates of the noise are 0, and the noise is continuous there: at
+    1e30 they are at most 1e-28, which moves it by less than 1e-25."""
+    f = grrt.log_bins(n=4)
+    a, sa = spectral(grrt, f, disk_noise_scale=INF)
+    b, sb = spectral(grrt, f, disk_noise_scale=1e30)
+    assert sa["physics_steps"] > 0
+    assert (b > 0).any()
+    np.testing.assert_allclose(a, b, rtol=1e-9, atol=0.0)
