@@ -60,16 +60,18 @@ __device__ __forceinline__ double v_mix(double lo, double hi, double t) {
     return __fma_rn(__dadd_rn(1.0, -t), lo, __dmul_rn(t, hi));
 }
 
-// Cell and fraction of the radial tables at r (their ends outside them); every
-// radial table and profile shares it.
+// Cell and fraction of the radial tables at r; every radial table and profile
+// shares it. Outside the tables it is their end, the start first (a disk whose
+// outer edge lies at or inside r_min has no other cells).
 struct VolCell {
     int i;
     double t;
 };
 __device__ __forceinline__ VolCell v_cell(const DevVolume& V, double r) {
-    const double rc = vmin(vmax(r, V.r_min), V.r_outer);
-    const double frac =
-        __dmul_rn(div_by(__dadd_rn(rc, -V.r_min), V.span, V.inv_span), static_cast<double>(V.n_r - 1));
+    const double last = static_cast<double>(V.n_r - 1);
+    double frac = __dmul_rn(div_by(__dadd_rn(r, -V.r_min), V.span, V.inv_span), last);
+    frac = (r >= V.r_outer) ? last : frac;
+    frac = (r <= V.r_min) ? 0.0 : frac;
     const int i = table_index(frac, 0, V.n_r - 2);
     return VolCell{i, __dadd_rn(frac, -static_cast<double>(i))};
 }

@@ -69,6 +69,16 @@ def test_table_cell_of_infinite_coordinates(edges):
     assert_same(edges(2, rows))
 
 
+def test_radial_table_at_and_beyond_its_ends(edges):
+    rng = np.random.default_rng(13)
+    rows = []
+    for lo, hi in ((1.4459, 30.0), (2.01, 2.01), (2.01, 1.5), (2.01, np.nextafter(2.01, 3))):
+        r = [lo, hi, np.nextafter(lo, 0), np.nextafter(lo, 9), np.nextafter(hi, 0), np.nextafter(hi, 99), 0.0, 1e3,
+             INF, NAN] + list(rng.uniform(0.9 * min(lo, hi), 1.2 * max(lo, hi), 2000))
+        rows += [(v, lo, hi) for v in r]
+    assert_same(edges(3, rows))
+
+
 def spectral(grrt, bins, **kw):
     """A small cube at the given bins, tables laid out for ordinary ones."""
     R = grrt.Renderer(grrt.config_params(3, width=32, height=24, **kw), freqs=grrt.log_bins(n=4))
