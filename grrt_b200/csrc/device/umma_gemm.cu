@@ -179,6 +179,7 @@ umma_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
                 bias = make_float4(bp[0], bp[1], bp[2], bp[3]);
             }
             float v[16];
+            __syncwarp();  // the load is of the whole warp; rows past M were skipped lane by lane above
             sm100::tmem_ld16(t_row + static_cast<uint32_t>(c0), v);
             if (nk <= 0) {
 #pragma unroll
@@ -265,7 +266,7 @@ size_t umma_gemm_smem_bytes(int N) {
 
 namespace {
 
-// Outputs and gate of a GEMM of N columns: 16-byte accesses.
+// Outputs of a GEMM: 16-byte accesses (the gate is read in any alignment).
 bool epilogue_ok(const GemmEpilogue& ep, int splits) {
     if (ep.out_bf16 && ((ep.ld_bf16 % 8) != 0 || (reinterpret_cast<uintptr_t>(ep.out_bf16) & 15))) return false;
     if (ep.out_f32 && ((ep.ld_f32 % 4) != 0 || (reinterpret_cast<uintptr_t>(ep.out_f32) & 15))) return false;
