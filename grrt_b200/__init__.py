@@ -150,6 +150,7 @@ def load_library(path: str = LIB_PATH) -> C.CDLL:
         "grrt_surrogate_params": (C.c_longlong, [vp, P(C.c_float), C.c_longlong]),
         "grrt_surrogate_set_params": (C.c_int, [vp, P(C.c_float), C.c_longlong]),
         "grrt_surrogate_forward": (C.c_int, [vp, vp, C.c_longlong, vp]),
+        "grrt_surrogate_forward_on": (C.c_int, [vp, vp, C.c_longlong, vp, vp]),
         "grrt_surrogate_gradients": (C.c_int, [vp, P(C.c_float), P(C.c_float), C.c_int, P(C.c_float),
                                                P(C.c_double)]),
         "grrt_surrogate_render_device": (C.c_int, [vp, vp, vp, vp, vp, vp]),
@@ -634,10 +635,18 @@ class Surrogate:
         self._check(self._L.grrt_surrogate_set_params(self.s, _fptr(p), len(p)), "grrt_surrogate_set_params")
 
     def forward(self, d_in, d_out, n: int) -> None:
-        """Device pointers (int) or torch tensors: inputs float[n][4] -> outputs float[n][16]."""
-        pi = d_in if isinstance(d_in, int) else d_in.data_ptr()
+        """Device pointers (int) or torch tensors: inputs float[n][4] -> outputs float[n][16].
+
+        With tensors the work is ordered on torch's current stream; inputs given
+        as pointers must be complete. Done when the call returns."""
         po = d_out if isinstance(d_out, int) else d_out.data_ptr()
-        self._check(self._L.grrt_surrogate_forward(self.s, pi, n, po), "grrt_surrogate_forward")
+        if isinstance(d_in, int):
+            self._check(self._L.grrt_surrogate_forward(self.s, d_in, n, po), "grrt_surrogate_forward")
+        else:
+            import torch
+            stream = torch.cuda.current_stream(d_in.get_device()).cuda_stream
+            self._check(self._L.grrt_surrogate_forward_on(self.s, d_in.data_ptr(), n, po, stream),
+                        "grrt_surrogate_forward_on")
 
     def gradients(self, X: np.ndarray, Y: np.ndarray):
         X = np.ascontiguousarray(X, dtype=np.float32)

@@ -259,9 +259,11 @@ struct GRRTSurrogate {
         return ok;
     }
 
-    // Waits for the stream; false if a kernel failed or reported a timeout.
-    bool check_gemm_errors() {
-        if (fail(cudaStreamSynchronize(stream), "tensor-core kernels")) return false;
+    // Waits for the network's stream, or another; false if a kernel failed or
+    // reported a timeout.
+    bool check_gemm_errors() { return check_gemm_errors(stream); }
+    bool check_gemm_errors(cudaStream_t q) {
+        if (fail(cudaStreamSynchronize(q), "tensor-core kernels")) return false;
         const int code = gemm_error_code();
         if (code != 0) {
             error = "tensor-core kernel reported a timeout (code " + std::to_string(code) + ")";
@@ -528,7 +530,10 @@ struct GRRTSurrogate {
     // O[n x 16] = network(X[n x 4]): the fused tensor-core kernel (rows
     // min(n, *d_n) when a device count is given)
     bool enqueue_forward(const float* X, size_t n, float* out, const unsigned* d_n = nullptr) {
-        return !fail(launch_mlp_fused(X, static_cast<long long>(n), d_params, mlp_maps, out, d_err, stream, d_n),
+        return enqueue_forward(X, n, out, d_n, stream);
+    }
+    bool enqueue_forward(const float* X, size_t n, float* out, const unsigned* d_n, cudaStream_t q) {
+        return !fail(launch_mlp_fused(X, static_cast<long long>(n), d_params, mlp_maps, out, d_err, q, d_n),
                      "fused network");
     }
 
@@ -818,11 +823,17 @@ extern "C" GRRT_EXPORT int grrt_surrogate_set_params(GRRTSurrogate* s, const flo
     return s->set_params(in, static_cast<size_t>(n)) ? 0 : -1;
 }
 
-extern "C" GRRT_EXPORT int grrt_surrogate_forward(GRRTSurrogate* s, const float* d_in, long long n, float* d_out) {
+extern "C" GRRT_EXPORT int grrt_surrogate_forward_on(GRRTSurrogate* s, const float* d_in, long long n, float* d_out,
+                                                     void* stream) {
     if (!s || !d_in || !d_out || n <= 0) return -1;
     s->error.clear();
     cudaSetDevice(s->device);
-    return s->enqueue_forward(d_in, static_cast<size_t>(n), d_out) && s->check_gemm_errors() ? 0 : -1;
+    const cudaStream_t q = static_cast<cudaStream_t>(stream);
+    return s->enqueue_forward(d_in, static_cast<size_t>(n), d_out, nullptr, q) && s->check_gemm_errors(q) ? 0 : -1;
+}
+
+extern "C" GRRT_EXPORT int grrt_surrogate_forward(GRRTSurrogate* s, const float* d_in, long long n, float* d_out) {
+    return s ? grrt_surrogate_forward_on(s, d_in, n, d_out, s->stream) : -1;
 }
 
 extern "C" GRRT_EXPORT int grrt_surrogate_gradients(GRRTSurrogate* s, const float* h_in, const float* h_y, int n,

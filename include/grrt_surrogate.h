@@ -96,8 +96,13 @@ GRRT_EXPORT int grrt_surrogate_get_bands(const GRRTSurrogate* s, double* out5);
 GRRT_EXPORT long long grrt_surrogate_params(GRRTSurrogate* s, float* out, long long capacity);
 GRRT_EXPORT int grrt_surrogate_set_params(GRRTSurrogate* s, const float* in, long long n);
 /* Network outputs float[n][16] for device inputs float[n][4] (the fused
- * tensor-core inference kernel; both pointers 16-byte aligned). */
+ * tensor-core inference kernel; both pointers 16-byte aligned). The work runs
+ * on the network's own stream, so d_in must be complete when the call is made;
+ * done when the call returns. */
 GRRT_EXPORT int grrt_surrogate_forward(GRRTSurrogate* s, const float* d_in, long long n, float* d_out);
+/* The same after the work that the caller's stream (a cudaStream_t) holds. */
+GRRT_EXPORT int grrt_surrogate_forward_on(GRRTSurrogate* s, const float* d_in, long long n, float* d_out,
+                                          void* stream);
 /* One forward + backward pass on host data (n a multiple of 128; records as
  * in grrt_surrogate_dataset; termination 2 masks a row): the loss and the
  * gradient of every parameter, without an update. */
