@@ -191,13 +191,15 @@ __device__ __forceinline__ void sincos_clamped_f64(double x, double& s, double& 
 // the residuals exact in fused multiply-adds (P. Markstein, IBM J. Res. Dev.
 // 34, 1990). The cubic step rounds up, so that the last one starts from above
 // and also rounds an all-ones significand, its one exception, correctly.
-// x = inf gives 0, NaN NaN: the approximation sees |x|, the residuals a number
-// that is finite. A zero or subnormal x or result is not handled (NaN or 0).
+// x = inf gives 0; a zero or subnormal x or result is not handled (NaN or 0).
+// kNaN: a NaN gives NaN, the approximation of |x| itself and not of the number
+// that keeps the residuals finite; without, it gives 0.
+template <bool kNaN = true>
 __device__ __forceinline__ double recip_f64(double x) {
     const int hi = __double2hiint(x);
     const double xa = __hiloint2double(min(hi & 0x7fffffff, 0x7fe00000), __double2loint(x));
     double y;
-    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(fabs(x)));
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(kNaN ? fabs(x) : xa));
     double e = __fma_rn(-xa, y, 1.0);
     y = __fma_ru(y, __fma_rn(e, e, e), y);
     e = __fma_rn(-xa, y, 1.0);
@@ -225,7 +227,10 @@ __device__ __forceinline__ Vec5<double> kerr_rhs_f64(const KerrHole& K, double p
     const double Sigma = __fma_rn(__dmul_rn(a2, c), c, r2);
     const double Delta = __dadd_rn(__fma_rn(-K.m2, r, r2), a2);
     const double SD = __dmul_rn(Sigma, Delta);
-    const double inv = recip_f64(__dmul_rn(SD, s));
+    // A NaN here comes from r or theta, so Delta or s is NaN too, and with it 1/Sigma
+    // and every component (the NaN form: 24.58 against 24.40 ms on the frame of
+    // 1024x1024 with 4 samples).
+    const double inv = recip_f64<false>(__dmul_rn(SD, s));
     const double iS = __dmul_rn(__dmul_rn(Delta, s), inv);  // 1/Sigma
     const double iD = __dmul_rn(__dmul_rn(Sigma, s), inv);  // 1/Delta
     const double is = __dmul_rn(SD, inv);                   // 1/sin(theta)

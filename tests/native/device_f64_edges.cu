@@ -62,6 +62,20 @@ __global__ void locate_kernel(const double* in, int n, double* fast, double* pla
     plain[2 * i + 1] = __dadd_rn(t, -static_cast<double>(idx));
 }
 
+// (r, theta, p_r, p_theta) with a NaN in r or theta -> how many of the five
+// derivatives are NaN
+__global__ void rhs_kernel(const double* in, int n, double* fast, double* plain) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    const double* y = in + 4 * i;
+    const double a = 0.9;
+    const Vec5<double> d =
+        kerr_rhs_f64(KerrHole{1.0, a, a * a, 2.0}, -1.0, 2.0, y[0], y[1], y[2], y[3]);
+    fast[2 * i] = isnan(d.r) + isnan(d.th) + isnan(d.ph) + isnan(d.pr) + isnan(d.pth);
+    plain[2 * i] = 5.0;
+    fast[2 * i + 1] = plain[2 * i + 1] = 0.0;
+}
+
 constexpr int kNodes = 17;
 
 // (r, r_min, r_outer) -> scale height from a table of kNodes radii
@@ -91,10 +105,10 @@ __global__ void radial_kernel(const double* in, int n, const double* lut, double
 
 }  // namespace
 
-// kind: 0 reciprocal, 1 largest quotient, 2 table cell, 3 radial table. in:
-// n rows of 2, 10, 4, 3 values; fast, plain: n rows of 2.
+// kind: 0 reciprocal, 1 largest quotient, 2 table cell, 3 radial table, 4
+// right-hand side. in: n rows of 2, 10, 4, 3, 4 values; fast, plain: n rows of 2.
 extern "C" int f64_edges(int kind, const double* in, int n, double* fast, double* plain) {
-    const int cols[4] = {2, 10, 4, 3};
+    const int cols[5] = {2, 10, 4, 3, 4};
     const size_t bytes_in = sizeof(double) * cols[kind] * n, bytes_out = sizeof(double) * 2 * n;
     std::vector<double> table(kNodes);
     for (int k = 0; k < kNodes; ++k) table[k] = 0.3 + 0.11 * k * k;
@@ -109,7 +123,8 @@ extern "C" int f64_edges(int kind, const double* in, int n, double* fast, double
         if (kind == 0) recip_kernel<<<g, 128>>>(d_in, n, d_fast, d_plain);
         else if (kind == 1) quotient_kernel<<<g, 128>>>(d_in, n, d_fast, d_plain);
         else if (kind == 2) locate_kernel<<<g, 128>>>(d_in, n, d_fast, d_plain);
-        else radial_kernel<<<g, 128>>>(d_in, n, lut, d_fast, d_plain);
+        else if (kind == 3) radial_kernel<<<g, 128>>>(d_in, n, lut, d_fast, d_plain);
+        else rhs_kernel<<<g, 128>>>(d_in, n, d_fast, d_plain);
         ok = cudaMemcpy(fast, d_fast, bytes_out, cudaMemcpyDeviceToHost) == cudaSuccess &&
              cudaMemcpy(plain, d_plain, bytes_out, cudaMemcpyDeviceToHost) == cudaSuccess;
     }

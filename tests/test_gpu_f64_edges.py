@@ -49,6 +49,11 @@ def test_reciprocal_of_nan_and_infinity(edges):
     assert_same(edges(0, [(a, b) for a in odd + [0.0] for b in x]))
 
 
+def test_right_hand_side_of_nan_is_nan(edges):
+    assert_same(edges(4, [(r, th, pr, pth) for r, th in ((NAN, 1.2), (6.0, NAN), (NAN, NAN), (-NAN, 0.0))
+                          for pr in (0.0, -0.7, INF) for pth in (0.0, 1.3, -INF)]))
+
+
 @pytest.mark.parametrize("top", [1e3, 1e150, 1e160, 1e300])
 def test_largest_quotient(edges, top):
     rng = np.random.default_rng(11)
