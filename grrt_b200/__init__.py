@@ -553,6 +553,14 @@ def _fptr(a: np.ndarray):
     return a.ctypes.data_as(C.POINTER(C.c_float))
 
 
+def _torch_stream(device: int) -> int:
+    """torch's current stream on a device, by its short way where torch has it
+    (0.2 against 1.4 us, of a small network call's 27)."""
+    import torch
+    raw = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+    return raw(device) if raw else torch.cuda.current_stream(device).cuda_stream
+
+
 class Surrogate:
     """The learned surrogate (include/grrt_surrogate.h): MLP 4 -> 256 x 4 -> 6,
     trained on the GPU by the library's tensor-core kernels."""
@@ -643,9 +651,8 @@ class Surrogate:
         if isinstance(d_in, int):
             self._check(self._L.grrt_surrogate_forward(self.s, d_in, n, po), "grrt_surrogate_forward")
         else:
-            import torch
-            stream = torch.cuda.current_stream(d_in.get_device()).cuda_stream
-            self._check(self._L.grrt_surrogate_forward_on(self.s, d_in.data_ptr(), n, po, stream),
+            self._check(self._L.grrt_surrogate_forward_on(self.s, d_in.data_ptr(), n, po,
+                                                          _torch_stream(d_in.get_device())),
                         "grrt_surrogate_forward_on")
 
     def gradients(self, X: np.ndarray, Y: np.ndarray):
