@@ -98,10 +98,12 @@ __device__ __forceinline__ ErrQuotient error_quotient(const Vec5<double>& y5, do
         const bool gt = __dmul_rn(u.num, v.den) < __dmul_rn(v.num, u.den);
         return ErrQuotient{gt ? v.num : u.num, gt ? v.den : u.den};
     };
-    int top = 0;
+    unsigned top = 0;  // unsigned: the device's NaN has its sign set, through fabs too
 #pragma unroll
-    for (int i = 0; i < 5; ++i) top = max(top, max(__double2hiint(q[i].num), __double2hiint(q[i].den)));
-    if (top >= 0x5ff00000) {  // 2^512, an infinity or a NaN: the terms in order, a NaN skipped
+    for (int i = 0; i < 5; ++i)
+        top = max(top, max(static_cast<unsigned>(__double2hiint(q[i].num)),
+                           static_cast<unsigned>(__double2hiint(q[i].den))));
+    if (top >= 0x5ff00000u) {  // 2^512, an infinity or a NaN: the terms in order, a NaN skipped
         ErrQuotient m{0.0, 1.0};
         for (int i = 0; i < 5; ++i) m = larger(m, q[i]);
         return m;
