@@ -72,10 +72,9 @@ F_EVAL = 133 + 37
 F_ATTEMPT_EXEC = 6 * F_EVAL + 480
 # Operations the kernels execute per attempt (all of a kernel's floating-point
 # operations divided by its attempts; a fused multiply-add counts 2), from the
-# ncu instruction counters of a 512x512 4-spp frame
-# (profiles/thin_kernels_inlined_kerr_512x512_4spp.md): the FP64
-# kernels (fp64_trace_kernel in both forms) and the FP32 speculation
-# (packed two-wide instructions count once there: a lower bound).
+# ncu instruction counters of a 512x512 4-spp frame: the FP64 kernels
+# (fp64_trace_kernel in both forms) and the FP32 speculation (packed two-wide
+# instructions count once there: a lower bound).
 F_EXEC_FP64_ATTEMPT = 953.4
 F_EXEC_FP32_ATTEMPT = 402.3
 # DRAM bytes (read + write) of one mixed_speculate_kernel launch on the

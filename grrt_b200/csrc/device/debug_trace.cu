@@ -12,9 +12,8 @@
 // reference's debug trace, the END colour is the disk's (and the volume's)
 // emission only; the sky is not added. One thread does the work: the trace is
 // bounded by max_steps outer steps of at most 21 attempts each and 4096 march
-// steps per ray-march. A lone ray is bound by fetching the code of its attempts,
-// so a scene without a volume has a kernel without the march (457 attempts:
-// 1.20 -> 1.16 ms on B200).
+// steps per ray-march. A scene without a volume has a kernel without the march's
+// code (a ray of 457 attempts: 1.20 -> 1.16 ms on B200).
 #include <cuda_runtime.h>
 
 #include <cmath>

@@ -268,10 +268,9 @@ GRRT_HD Vec5<T> rk4_step(T M, T a, T pt, T pph, const Vec5<T>& y, T h) {
 // f(y) afresh at every attempt; mathematically it is the previous accepted
 // attempt's k7 (same state, same constants) or the rejected attempt's k1
 // (same state), so a caller that keeps it evaluates six right-hand sides per
-// attempt instead of seven. Without FMA contraction the kept value is
-// bit-identical to a fresh one; the device compiler may contract each inlined
-// copy of the right-hand side differently, so on the GPU the two can differ
-// in the last bits (the method and its step decisions are unchanged).
+// attempt instead of seven. The kept value has the bits of a fresh one: on the
+// host without FMA contraction, on the device with the roundings written out
+// (not under GRRT_RHS_GENERIC, where each inlined copy is contracted by itself).
 template <typename T>
 GRRT_HD T dp45_attempt_k1(T M, T a, T pt, T pph, const Vec5<T>& y, T h, const Vec5<T>& k1, Vec5<T>& y5,
                           Vec5<T>& k7_out) {

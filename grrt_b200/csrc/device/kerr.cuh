@@ -265,7 +265,7 @@ __device__ __forceinline__ Vec5<double> kerr_rhs_f64(const KerrHole& K, double p
 // instruction less here counts six times an attempt. With the attempt's packed
 // sums over four components (mixed_attempt_k1): a 1024^2 4-sample speculative
 // pass 5.89 -> 5.43 ms. Values are those of the generic body, its order of
-// products kept (the same bits on 2^20 states).
+// products kept (a test compares the bits on 2^18 states).
 __device__ __forceinline__ float rcp_approx(float x) {
     float y;
     asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));

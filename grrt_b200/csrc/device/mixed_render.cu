@@ -21,7 +21,7 @@
 // camera's single render.
 // The FP64 trace inlines the right-hand side into its attempt: with the
 // roundings written out (kerr.cuh) every copy has the same bits, and without
-// the calls an attempt is 1,060 instructions instead of 1,600 (Kerr a=0.998,
+// the calls an attempt is 1,120 instructions instead of 1,600 (Kerr a=0.998,
 // 1024x1024, 4 spp on B200: FP64 form 31.9 -> 24.4 ms, the mixed form's
 // re-trace 6.7 -> 5.3 ms; one lone ray 2.53 -> 1.83 us an attempt).
 #include <cuda_runtime.h>
@@ -744,9 +744,11 @@ const MixLaunchShape& mix_shape() {
 // samples a lane the launch waits for its longest rays, whose steps are quicker
 // with fewer warps beside them: up to three samples a lane of the full grid
 // (227 k), three blocks are 0-8% faster than four (B200, Kerr a=0.998: 256x256
-// 1.22 -> 1.16 ms, 320x320 1.45 -> 1.34, 384x384 1.67 -> 1.59; two blocks 1.07,
-// 1.39, 1.68); above it the fourth block's warps win (512x512 2.39 against 2.46
-// ms, 1024x1024 with 4 spp 24.4 against 28.6).
+// 1.22 -> 1.16 ms, 320x320 1.45 -> 1.34, 384x384 1.67 -> 1.59); above it the
+// fourth block's warps win (512x512 2.39 against 2.46 ms, 1024x1024 with 4 spp
+// 24.4 against 28.6). Two blocks take 1.07, 1.39 and 1.68 ms: better than three
+// where the samples barely outnumber the lanes, worse from 320x320 on; the rule
+// does not go that far, and where their line lies was not measured.
 static int fp64_trace_blocks(int per_sm, int sms, size_t n) {
     const size_t lanes = static_cast<size_t>(sms) * per_sm * kMixThreads;
     return (per_sm > 3 && n <= 3 * lanes) ? 3 : per_sm;

@@ -2,8 +2,9 @@
 // persistent kernel computes out[n x 16] = network(X[n x 4]) with the hidden
 // activations kept in shared memory between layers.
 //
-// Per 128-row tile (what bounds it: the epilogue, special-function pipe 45%,
-// issue 60%, shared memory 57%; tensor pipe 34%):
+// Per 128-row tile (special-function pipe 45%, issue 60%, shared memory 57%,
+// tensor pipe 34%: no pipe is the bound; without the tanh or with a quarter of
+// the weight stream it is no faster, with a quarter of the MMA work 6%):
 //   layer 1 (K = 4): the epilogue warps on the CUDA cores, written as BF16
 //     straight into the tile's A operand buffer (K-major, 128-byte swizzle:
 //     the layout a TMA SWIZZLE_128B load produces);

@@ -358,9 +358,9 @@ struct GRRTSurrogate {
         return (kbt + per - 1) / per;
     }
 
-    // The work enqueued on `to` so far comes before what `from`'s next work is.
-    bool order(cudaStream_t from, cudaStream_t to, cudaEvent_t ev) {
-        return !fail(cudaEventRecord(ev, to), "event") && !fail(cudaStreamWaitEvent(from, ev, 0), "event");
+    // What `waiter` gets from now on starts after the work that `source` holds.
+    bool order(cudaStream_t waiter, cudaStream_t source, cudaEvent_t ev) {
+        return !fail(cudaEventRecord(ev, source), "event") && !fail(cudaStreamWaitEvent(waiter, ev, 0), "event");
     }
 
     // dW = dY^T X and db = the column sums of dY, over the batch, on the side
