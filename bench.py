@@ -219,6 +219,13 @@ def run_reference_arm(args):
     rank = int(os.environ.get("RANK", "0"))
     if rank != 0:
         return
+    sys.path.insert(0, os.path.join(ROOT, "tests"))
+    import oracle_bind
+    if not (oracle_bind.ref_available("fast") or oracle_bind.ref_available("strict")):
+        print(json.dumps({"impl": "reference",
+                          "unavailable": "the reference's sources are not here, so oracle/_ref could not be built"}),
+              flush=True)
+        return
     stride = 16
     for w in range(args.warmup):
         cpu_reference_sample(w % stride, stride * 4)
