@@ -828,7 +828,13 @@ extern "C" GRRT_EXPORT int grrt_surrogate_forward_on(GRRTSurrogate* s, const flo
     if (!s || !d_in || !d_out || n <= 0) return -1;
     s->error.clear();
     cudaSetDevice(s->device);
-    const cudaStream_t q = static_cast<cudaStream_t>(stream);
+    cudaStream_t q = static_cast<cudaStream_t>(stream);
+    // a stream under capture has no work to follow and cannot be waited for
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    if (q != s->stream && (cudaStreamIsCapturing(q, &capture) != cudaSuccess || capture != cudaStreamCaptureStatusNone)) {
+        cudaGetLastError();
+        q = s->stream;
+    }
     return s->enqueue_forward(d_in, static_cast<size_t>(n), d_out, nullptr, q) && s->check_gemm_errors(q) ? 0 : -1;
 }
 

@@ -100,7 +100,8 @@ GRRT_EXPORT int grrt_surrogate_set_params(GRRTSurrogate* s, const float* in, lon
  * on the network's own stream, so d_in must be complete when the call is made;
  * done when the call returns. */
 GRRT_EXPORT int grrt_surrogate_forward(GRRTSurrogate* s, const float* d_in, long long n, float* d_out);
-/* The same after the work that the caller's stream (a cudaStream_t) holds. */
+/* The same after the work that the caller's stream (a cudaStream_t) holds; with
+ * a stream under capture it runs on the network's stream, outside the graph. */
 GRRT_EXPORT int grrt_surrogate_forward_on(GRRTSurrogate* s, const float* d_in, long long n, float* d_out,
                                           void* stream);
 /* One forward + backward pass on host data (n a multiple of 128; records as

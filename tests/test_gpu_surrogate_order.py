@@ -25,3 +25,25 @@ def test_forward_waits_for_its_input(grrt, need_gpu, side_stream):
         S.forward(late, got, n)
     torch.cuda.synchronize()
     assert torch.equal(got, want)
+
+
+def test_forward_under_capture_runs_outside_the_graph(grrt, need_gpu):
+    """As with pointers: the outputs are there when the call returns, and the
+    capture of the program's other work goes on."""
+    import torch
+    S = grrt.Surrogate(3)
+    n = 300
+    x = torch.rand(n, 4, device="cuda", generator=torch.Generator(device="cuda").manual_seed(2))
+    want, got, y = torch.empty(n, 16, device="cuda"), torch.zeros(n, 16, device="cuda"), torch.zeros(8, device="cuda")
+    torch.cuda.synchronize()
+    S.forward(x, want, n)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, capture_error_mode="relaxed"):
+        y += 1
+        S.forward(x, got, n)
+        y += 1
+    torch.cuda.synchronize()
+    assert torch.equal(got, want)
+    graph.replay()
+    torch.cuda.synchronize()
+    assert bool((y == 2).all())
